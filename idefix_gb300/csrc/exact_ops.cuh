@@ -65,6 +65,38 @@ IDFX_HD T times_sign(T x, T s, uint64_t sb) {
   }
 }
 
+// x 2^K, exact: on the FP64 path an add to the exponent field (the FP64 pipe
+// is what the sweeps wait for), zeros as they are, and the product where the
+// result could leave the normal range; FP32 the product
+template <int K, typename T>
+IDFX_HD T pow2x(T x) {
+  constexpr double f = K >= 0 ? (double)(1 << (K >= 0 ? K : 0)) : 1.0 / (double)(1 << (K < 0 ? -K : 0));
+  if constexpr (sizeof(T) == 8) {
+    const uint64_t u = dbits(x);
+    if (((uint32_t)(u >> 52) & 0x7ffu) - 64u < 1920u) return dfrom(u + ((uint64_t)(int64_t)K << 52));
+    if ((u << 1) == 0ull) return x;
+    return x * f;
+  } else {
+    return x * T(f);
+  }
+}
+
+// x < y: on the FP64 path from the bit patterns (ordered as signed integers
+// once the negative ones are reversed; zeros equal, NaNs false)
+template <typename T>
+IDFX_HD bool lt(T x, T y) {
+  if constexpr (sizeof(T) == 8) {
+    const uint64_t M = 0x7FFFFFFFFFFFFFFFull, I = 0x7FF0000000000000ull;
+    const uint64_t u = dbits(x), w = dbits(y);
+    if ((u & M) > I || (w & M) > I) return false;
+    const int64_t a = (u >> 63) ? -(int64_t)(u & M) : (int64_t)u;
+    const int64_t b = (w >> 63) ? -(int64_t)(w & M) : (int64_t)w;
+    return a < b;
+  } else {
+    return x < y;
+  }
+}
+
 // One upwind term of CalcContactAverage, (1 - w) a + w b with the weight w
 // in {0, 1/2, 1} (storeFlux.hpp:40-43).  The FP64 path forms the two
 // products exactly on the integer pipe - a product by 1 is the value, by 0 a

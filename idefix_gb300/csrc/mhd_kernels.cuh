@@ -576,8 +576,8 @@ __device__ __forceinline__ void store_emf(const Geo& g, const Fields& f, long lo
     if constexpr (D == 3) Eb[c] = sb * r.F[d::BXb];
     if (g.emf == kEmfContact) {
       T s = T(0.5);
-      if (r.F[vv::RHO] > T(kEpsUctContact)) s = T(1);
-      if (r.F[vv::RHO] < T(-kEpsUctContact)) s = T(0);
+      if (lt(T(kEpsUctContact), r.F[vv::RHO])) s = T(1);
+      if (lt(r.F[vv::RHO], T(-kEpsUctContact))) s = T(0);
       SV[c] = s;
     }
     return;
@@ -712,6 +712,7 @@ __device__ __forceinline__ void d_sweep_march(const Geo& g, const Fields& f, con
   const T gam = (T)g.gamma;
   T w[NV][W];
   T vrp[NV];            // right-face state of the previous cell
+  T dl[NV];             // PLM in FP64: the next cell's difference on the left
   T Fp[v::BX1];         // flux x A of the previous face
   T cp = T(0);          // cmax of the previous face
   T nx[NV];             // prefetched stencil value of the next step
@@ -731,6 +732,7 @@ __device__ __forceinline__ void d_sweep_march(const Geo& g, const Fields& f, con
     if (n == dd::BXn) continue;
 #pragma unroll
     for (int m = 0; m < W - 1; m++) w[n][m + 1] = vcT[n * g.ncell + c0 + (m - 1 - H) * sd];
+    if constexpr (ORDER == 2 && sizeof(T) == 8) dl[n] = w[n][2] - w[n][1];
     if constexpr (PF) nx[n] = vcT[n * g.ncell + c0 + (H - 1) * sd];
   }
   if constexpr (PF) nbn = vs[f0];
@@ -799,9 +801,15 @@ __device__ __forceinline__ void d_sweep_march(const Geo& g, const Fields& f, con
       } else {
         w[n][W - 1] = vcT[n * g.ncell + cc + H * sd];
       }
-      // FP64: odd variables' limiter quotient on the integer pipe
-      Recon<ORDER>::cell(w[n], dxd, n == v::RHO || n == v::PRS, vl[n], vr[n], shk, l3,
-                         sizeof(T) == 8 && (n & 1));
+      if constexpr (ORDER == 2 && sizeof(T) == 8) {
+        // PLM in FP64: the difference on the left is the last step's on the
+        // right (the same operation on the same values)
+        const T dvp = w[n][2] - w[n][1];
+        Recon<ORDER>::plm(w[n][1], dl[n], dvp, shk, vl[n], vr[n]);
+        dl[n] = dvp;
+      } else {
+        Recon<ORDER>::cell(w[n], dxd, n == v::RHO || n == v::PRS, vl[n], vr[n], shk, l3);
+      }
     }
     if (c >= m0) {
       T vL[NV], vR[NV];
@@ -842,7 +850,7 @@ __device__ __forceinline__ void d_sweep_march(const Geo& g, const Fields& f, con
             const double prev = (invdt == 1) ? 0.0 : (PF ? curI : f.InvDt[cu]);
             double inv;
             if constexpr (sizeof(T) == 8) {
-              inv = prev + div_r(0.5 * (r.cmax + cp), Recip{g.dx[DIR], g.rdx[DIR]});
+              inv = prev + div_r(pow2x<-1>(r.cmax + cp), Recip{g.dx[DIR], g.rdx[DIR]});
             } else {
               inv = prev + to_f64(T(0.5) * (r.cmax + cp) * invdxT);
             }

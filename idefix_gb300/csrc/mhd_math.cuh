@@ -18,6 +18,7 @@
 #include "exact_ops.cuh"
 #include "intdiv.cuh"
 #include "rdiv.cuh"
+#include "seeddiv.cuh"
 
 namespace idfx {
 
@@ -64,18 +65,20 @@ __device__ __forceinline__ float fdiv_corrected(float a, float b) {
   return __fmaf_rn(e, r, q);
 }
 
-// division: FP64 IEEE correctly rounded (the bit-identical path); FP32 (the
-// mixed path, FP32-accurate rather than bit-matched) fdiv_corrected
+// division: FP64 IEEE correctly rounded (the bit-identical path; from FP32
+// seeds, three FP64-pipe operations instead of the hardware sequence's
+// seven, seeddiv.cuh); FP32 (the mixed path, FP32-accurate rather than
+// bit-matched) fdiv_corrected
 template <typename T>
 __device__ __forceinline__ T dv(T a, T b) {
   if constexpr (sizeof(T) == 4) {
     return fdiv_corrected(a, b);
   } else {
-    return a / b;
+    return quot(a, b);
   }
 }
 
-// square root: FP64 IEEE (the bit-identical path); FP32 x * rsqrt(x), within
+// square root: FP64 IEEE (the bit-identical path, seeddiv.cuh); FP32 x * rsqrt(x), within
 // 2 ulp (the tiny offset keeps sqrt(0) = 0; negative arguments stay NaN) -
 // measured not to change the mixed path's errors against FP64
 template <typename T>
@@ -83,19 +86,14 @@ __device__ __forceinline__ T sqr(T x) {
   if constexpr (sizeof(T) == 4) {
     return x * rsqrtf(x + 1.2e-38f);
   } else {
-    return sqrt(x);
+    return root(x);
   }
 }
 
-// 1 / b: FP64 the correctly rounded reciprocal (__drcp_rn, one instruction
-// sequence shorter than a general division, equal to 1 / b); FP32 as dv
+// 1 / b, as dv
 template <typename T>
 __device__ __forceinline__ T rcp(T b) {
-  if constexpr (sizeof(T) == 8) {
-    return rcp_rn(b);
-  } else {
-    return fdiv_corrected(T(1), b);
-  }
+  return dv(T(1), b);
 }
 
 // the same quotient computed on the integer pipe for FP64 (intdiv.cuh): used
@@ -168,7 +166,11 @@ __device__ __forceinline__ void prim_to_cons(T gm1, T* U, const T* V, T rgm1 = T
     (void)rgm1;
     pq = dv(V[v::PRS], gm1);
   }
-  U[v::ENG] = mad(T(0.5), mag, mad(T(0.5) * V[v::RHO], kin, pq));
+  if constexpr (sizeof(T) == 8) {  // the halves exact on the integer pipe
+    U[v::ENG] = pow2x<-1>(mag) + (pow2x<-1>(V[v::RHO]) * kin + pq);
+  } else {
+    U[v::ENG] = mad(T(0.5), mag, mad(T(0.5) * V[v::RHO], kin, pq));
+  }
 }
 
 // FUSED (mixed path, FP64 state): the same FP64 pressure recovery with the
@@ -235,9 +237,10 @@ __device__ __forceinline__ T flux_bb(const T* V) {
   return mad(V[d::Xn], V[d::BXb], -(V[d::BXn] * V[d::Xb]));
 }
 
-// physical MHD flux along DIR (flux.hpp:28-95); U is read before F is written
-template <int D, int DIR, typename T>
-__device__ __forceinline__ void phys_flux(T* F, const T* V, const T* U) {
+// physical MHD flux along DIR (flux.hpp:28-95); U is read before F is
+// written; ptot = PRS + B^2 / 2 of the state where the caller has it
+template <int D, int DIR, bool HAVE_PT = false, typename T>
+__device__ __forceinline__ void phys_flux(T* F, const T* V, const T* U, T pt = T(0)) {
   using v = Var<D>;
   using d = Dir<D, DIR>;
   const T uXn = U[d::Xn], uE = U[v::ENG];
@@ -251,15 +254,26 @@ __device__ __forceinline__ void phys_flux(T* F, const T* V, const T* U) {
   F[d::BXn] = T(0);
   F[d::BXt] = flux_bt<D, DIR>(V);
   if constexpr (D == 3) F[d::BXb] = flux_bb<D, DIR>(V);
-  T Bmag2, vB;
+  T vB;
   if constexpr (D == 3) {
-    Bmag2 = sumsq<3>(V[v::BX1], V[v::BX2], V[v::BX3]);
     vB = mad(V[v::MX3], V[v::BX3], mad(V[v::MX2], V[v::BX2], V[v::MX1] * V[v::BX1]));
   } else {
-    Bmag2 = sumsq<2>(V[v::BX1], V[v::BX2], T(0));
     vB = mad(V[v::MX2], V[v::BX2], V[v::MX1] * V[v::BX1]);
   }
-  const T ptot = mad(T(0.5), Bmag2, V[v::PRS]);
+  T ptot = pt;
+  if constexpr (!HAVE_PT) {
+    T Bmag2;
+    if constexpr (D == 3) {
+      Bmag2 = sumsq<3>(V[v::BX1], V[v::BX2], V[v::BX3]);
+    } else {
+      Bmag2 = sumsq<2>(V[v::BX1], V[v::BX2], T(0));
+    }
+    if constexpr (sizeof(T) == 8) {
+      ptot = pow2x<-1>(Bmag2) + V[v::PRS];
+    } else {
+      ptot = mad(T(0.5), Bmag2, V[v::PRS]);
+    }
+  }
   F[v::ENG] = mad(uE + ptot, V[d::Xn], -(V[d::BXn] * (vB)));
   F[d::Xn] += ptot;
 }
@@ -275,14 +289,22 @@ __device__ __forceinline__ T lim_minmod(T, T) {
 }
 
 template <typename T>
-// ipipe: the quotient on the integer pipe (dvi, the same correctly rounded
-// value).  The FP64 sweeps are bound by the narrow FP64 pipe while the
-// integer pipe idles: half of the limiter quotients go there (the FP64 cycle
-// 140.1 -> 137.7 ms at 256^3; all of them, or the right-state twins of the
-// HLLD quotients as well, gave nothing - the integer division's latency)
-__device__ __forceinline__ T lim_vanleer(T dvp, T dvm, bool ipipe = false) {  // :54-57
-  if (dvp * dvm > T(0)) return ipipe ? dvi(T(2) * dvp * dvm, dvp + dvm) : dv(T(2) * dvp * dvm, dvp + dvm);
+__device__ __forceinline__ T lim_vanleer(T dvp, T dvm) {  // :54-57
+  if (dvp * dvm > T(0)) return dv(T(2) * dvp * dvm, dvp + dvm);
   return T(0);
+}
+
+// half the van Leer slope on the FP64 path, 0.5 ((2 dvp) dvm) / (dvp + dvm):
+// scaling by 2 is exact, so inside the seeded quotient's exponent band this
+// is the correctly rounded (dvp dvm) / (dvp + dvm) - one product instead of
+// three and no product by 1/2; outside it the expression as it stands
+__device__ __forceinline__ double half_vanleer(double dvp, double dvm) {
+  const double p = dvp * dvm;
+  if (!gt0(p)) return 0.0;
+  const double s = dvp + dvm;
+  double q;
+  if (try_seed_quot(p, seed_div(s), q)) return q;
+  return 0.5 * ((2.0 * dvp * dvm) / s);
 }
 
 template <typename T>
@@ -406,21 +428,32 @@ __device__ __forceinline__ void ppm_states(T vm2, T vm1, T v0, T vp1, T vp2, T& 
 template <int ORDER>
 struct Recon {
   static constexpr int H = (ORDER == 1 ? 0 : (ORDER == 4 ? 2 : 1));  // ORDER 5: 1
+  // PLM from the centre value and the differences on its two sides
+  template <typename T>
+  __device__ __forceinline__ static void plm(T w, T dvm, T dvp, bool shock, T& vl, T& vr) {
+    if constexpr (sizeof(T) == 8) {
+      const double h = shock ? 0.0 : half_vanleer(dvp, dvm);
+      vr = w + h;
+      vl = w - h;
+    } else {
+      const T d = shock ? lim_minmod(dvp, dvm) : lim_vanleer(dvp, dvm);
+      vr = mad(T(0.5), d, w);
+      vl = mad(T(-0.5), d, w);
+    }
+  }
   // shock: the cell is flagged by shock flattening (minmod slope, PLM and
   // LimO3 only, extrapolateToFaces.hpp:96-218)
   template <typename T>
   // e2: (0.1 dx)^2 and its reciprocal (LimO3, FP64 path; Geo::l3b, l3y)
   __device__ __forceinline__ static void cell(const T* w, T dx, bool pos, T& vl, T& vr, bool shock = false,
-                                              const Recip& e2 = Recip{0.0, 0.0}, bool ipipe = false) {
+                                              const Recip& e2 = Recip{0.0, 0.0}) {
     if constexpr (ORDER == 1) {
       vl = w[0];
       vr = w[0];
     } else if constexpr (ORDER == 2) {
       const T dvm = w[1] - w[0];
       const T dvp = w[2] - w[1];
-      const T d = shock ? lim_minmod(dvp, dvm) : lim_vanleer(dvp, dvm, ipipe);
-      vr = mad(T(0.5), d, w[1]);
-      vl = mad(T(-0.5), d, w[1]);
+      plm(w[1], dvm, dvp, shock, vl, vr);
     } else if constexpr (ORDER == 3) {
       const T dm = w[1] - w[0];
       const T dp = w[2] - w[1];
@@ -463,23 +496,22 @@ struct RiemannOut {
   T cmax, sl, sr;
 };
 
-// a / b where several quotients share b: on the FP64 path with the
-// reciprocal R = recip(b) formed once (Markstein, rdiv.cuh), bit-identical to
-// a / b; the FP32 path divides
+// a / b where several quotients share b: on the FP64 path with the divisor
+// prepared once (seeddiv.cuh); the FP32 path divides
 template <typename T>
-__device__ __forceinline__ T shared_div(T a, T b, const Recip& R) {
+__device__ __forceinline__ T shared_div(T a, T b, const SeedDiv& R) {
   if constexpr (sizeof(T) == 8) {
-    return div_r(a, R);
+    return quot(a, R);
   } else {
     return dv(a, b);
   }
 }
 template <typename T>
-__device__ __forceinline__ Recip shared_recip(T b) {
+__device__ __forceinline__ SeedDiv shared_divisor(T b) {
   if constexpr (sizeof(T) == 8) {
-    return recip(b);
+    return seed_div(b);
   } else {
-    return Recip{0.0, 0.0};
+    return SeedDiv{};
   }
 }
 
@@ -496,16 +528,21 @@ __device__ __forceinline__ T fast_speed(T gamma, const T* v) {
   const T Btmag2 = mad(b3, b3, b2 * b2);
   const T Bmag2 = mad(b1, b1, Btmag2);
   T c = gpr - Bmag2;
-  c = gpr + Bmag2 + sqr(mad(T(4) * gpr, Btmag2, c * c));
-  c = sqr(dv(T(0.5) * c, v[vv::RHO]));
+  if constexpr (sizeof(T) == 8) {  // products by 4 and 1/2 exact on the integer pipe
+    c = gpr + Bmag2 + sqr(pow2x<2>(gpr) * Btmag2 + c * c);
+    c = sqr(dv(pow2x<-1>(c), v[vv::RHO]));
+  } else {
+    c = gpr + Bmag2 + sqr(mad(T(4) * gpr, Btmag2, c * c));
+    c = sqr(dv(T(0.5) * c, v[vv::RHO]));
+  }
   return c;
 }
 
 template <int D, typename T>
 __device__ __forceinline__ T half_b2(const T* v) {
   using vv = Var<D>;
-  if constexpr (D == 3) return T(0.5) * (sumsq<3>(v[vv::BX1], v[vv::BX2], v[vv::BX3]));
-  return T(0.5) * (sumsq<2>(v[vv::BX1], v[vv::BX2], T(0)));
+  if constexpr (D == 3) return pow2x<-1>(sumsq<3>(v[vv::BX1], v[vv::BX2], v[vv::BX3]));
+  return pow2x<-1>(sumsq<2>(v[vv::BX1], v[vv::BX2], T(0)));
 }
 
 // HLLD (Miyoshi & Kusano 2005) with the reference's HLLC fall-back near
@@ -554,7 +591,6 @@ __device__ __forceinline__ void riemann_hlld(T gamma, T rgm1, const T* vL, const
   bool dbl = false;
   T Bx = T(0), sBx = T(1), SM = T(0), pts = T(0), duL = T(0), duR = T(0);
   uint64_t sBxb = 0ull;
-  Recip RsL{}, RsR{};
   T rhoL = T(0), rhoR = T(0), sqrL = T(0), sqrR = T(0), S1L = T(0), S1R = T(0);
   T bn = T(0), bLt = T(0), bLb = T(0), bRt = T(0), bRb = T(0);  // star field components
   T vsL = T(0), vsR = T(0), wsL = T(0), wsR = T(0);
@@ -570,18 +606,16 @@ __device__ __forceinline__ void riemann_hlld(T gamma, T rgm1, const T* vL, const
     SM = (duR * uR[Xn] - duL * uL[Xn] - ptR + ptL) * scrh;
     pts = duR * uR[RHO] * ptL - duL * uL[RHO] * ptR + vL[RHO] * vR[RHO] * duR * duL * (vR[Xn] - vL[Xn]);
     pts *= scrh;
-    // (sl - SM) and (sr - SM) divide the star density and the star energy
-    RsL = shared_recip(sl - SM);
-    RsR = shared_recip(sr - SM);
-    rhoL = shared_div(uL[RHO] * duL, sl - SM, RsL);
-    rhoR = shared_div(uR[RHO] * duR, sr - SM, RsR);
+    rhoL = dv(uL[RHO] * duL, sl - SM);
+    rhoR = dv(uR[RHO] * duR, sr - SM);
     sqrL = sqr(rhoL);
     sqrR = sqr(rhoR);
     S1L = SM - dv(fabs(Bx), sqrL);
     S1R = SM + dv(fabs(Bx), sqrR);
     int revert_to_hllc = 0;
-    if ((S1L - sl) < T(1.e-4) * (SM - sl)) revert_to_hllc = 1;
-    if ((S1R - sr) > T(-1.e-4) * (sr - SM)) revert_to_hllc = 1;
+    // SM - sl is -(sl - SM): the difference that divides above
+    if (lt(S1L - sl, T(1.e-4) * -(sl - SM))) revert_to_hllc = 1;
+    if (lt(T(-1.e-4) * (sr - SM), S1R - sr)) revert_to_hllc = 1;
     if (revert_to_hllc) {
       // field components of the HLL state (sr uR - sl uL + FL - FR) / (sr - sl);
       // the normal component's fluxes are zero
@@ -627,13 +661,16 @@ __device__ __forceinline__ void riemann_hlld(T gamma, T rgm1, const T* vL, const
     uS[n] = sideL ? uL[n] : uR[n];
   }
   T* F = r.F;
-  phys_flux<D, DIR>(F, vS, uS);
+  const T pt = sideL ? ptL : ptR;
+  if constexpr (sizeof(T) == 8) {
+    phys_flux<D, DIR, true>(F, vS, uS, pt);  // pt: the same sum as the flux's total pressure
+  } else {
+    phys_flux<D, DIR>(F, vS, uS);
+  }
   if (!sub) return;
   // star state of the chosen side (us)
   const T s = sideL ? sl : sr;
   const T du = sideL ? duL : duR;
-  const T pt = sideL ? ptL : ptR;
-  const Recip Rs = sideL ? RsL : RsR;
   const T vs = sideL ? vsL : vsR;
   const T ws = sideL ? wsL : wsR;
   T us[NV];
@@ -652,11 +689,11 @@ __device__ __forceinline__ void riemann_hlld(T gamma, T rgm1, const T* vL, const
     T scrh = a;
     scrh -= b;
     us[ENG] = du * uS[ENG] - pt * vS[Xn] + pts * SM + Bx * scrh;
-    us[ENG] = shared_div(us[ENG], s - SM, Rs);
+    us[ENG] = dv(us[ENG], s - SM);
   }
   if (dbl) {
     // double-star state of the chosen side (uss); F += S1 (uss - us)
-    const Recip Rq = shared_recip(sqrL + sqrR);  // divides the four double-star values
+    const SeedDiv Rq = shared_divisor(sqrL + sqrR);  // divides the four double-star values
     T vss = sqrL * vsL + sqrR * vsR + times_sign(bRt - bLt, sBx, sBxb);
     vss = shared_div(vss, sqrL + sqrR, Rq);
     T wss = T(0);
@@ -690,8 +727,10 @@ __device__ __forceinline__ void riemann_hlld(T gamma, T rgm1, const T* vL, const
     const uint64_t sgnb = sideL ? (sBxb ^ (1ull << 63)) : sBxb;
     uss[ENG] = us[ENG] + times_sign(sq * scrh, sgn, sgnb);
     const T S1 = sideL ? S1L : S1R;
+    // density and normal momentum are the single star's: no contribution
 #pragma unroll
-    for (int n = 0; n < NV; n++) F[n] = mad(S1, uss[n] - us[n], F[n]);
+    for (int n = 0; n < NV; n++)
+      if (n != RHO && n != Xn) F[n] = mad(S1, uss[n] - us[n], F[n]);
   }
   // F += s (us - u) of the chosen side: single star F = Fs + s (us - u),
   // double star F = (Fs + S1 (uss - us)) + s (us - u), the reference's order

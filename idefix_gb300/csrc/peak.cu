@@ -7,6 +7,7 @@
 #include "fpconv.cuh"
 #include "intdiv.cuh"
 #include "rdiv.cuh"
+#include "seeddiv.cuh"
 
 namespace {
 
@@ -59,6 +60,16 @@ __global__ void k_check_division(long long n, unsigned long long seed, unsigned 
   // the reciprocal form of the flux sweeps (rdiv.cuh)
   const double r2 = idfx::div_r(a, idfx::recip(b));
   if (__double_as_longlong(r0) != __double_as_longlong(r2)) atomicAdd(bad, 1ull);
+  // the seeded quotient and square root (seeddiv.cuh), also at and beside equal operands and exact squares
+  auto differ = [](double x, double y) {
+    return __double_as_longlong(x) != __double_as_longlong(y) && !(x != x && y != y);
+  };
+  const double near_b = __longlong_as_double(__double_as_longlong(b) + (long long)(h3 >> 8) % 3 - 1);
+  const double sq = b * near_b;
+  if (differ(r0, idfx::quot(a, b)) || differ(near_b / b, idfx::quot(near_b, b)) ||
+      differ(sqrt(fabs(a)), idfx::root(fabs(a))) || differ(sqrt(sq), idfx::root(sq)) ||
+      differ(sqrt(a), idfx::root(a)))
+    atomicAdd(bad, 1ull);
 }
 
 // f2d_exact on a stride of all binary32 patterns, d2f_rn on random binary64
