@@ -696,6 +696,7 @@ void choose_segments(Engine& e) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  e.sms = sms;
   const long long want = (long long)sms * 512;
   for (int d = 0; d < e.g.D; d++) {
     // marching columns: the two other directions (with the CT extension)
@@ -833,7 +834,7 @@ int idfx_gpu_create(const idfx_gpu_config* cfg, void* stream, idfx_gpu** out) {
   return IDFX_OK;
 }
 
-// Autotuner of the march segment length per direction: the sweeps of each
+// Autotuner of the mixed path's sweep kernels and segment lengths: the sweeps of each
 // direction are timed alone for every candidate (min over reps launches);
 // they accumulate into Uc, InvDt and the EMF arrays, so the whole field pool
 // and the control block are saved first and put back afterwards.  Results
@@ -843,6 +844,12 @@ int idfx_gpu_autotune(idfx_gpu* h, int reps) {
   Engine& e = h->e;
   if (e.g.order == IDFX_LEARNED && !e.learned)
     return fail(e, IDFX_ERR_STATE, "the learned reconstruction needs idfx_gpu_set_learned first");
+  if (e.precision == IDFX_FP64) {
+    // nothing to choose: the FP64 sweeps take one thread per cell whatever the
+    // segments are (which stay inside the tuner's range)
+    for (int d = 0; d < e.g.D; d++) e.seg[d] = e.seg[d] < 4 ? 4 : e.seg[d];
+    return IDFX_OK;
+  }
   if (reps < 1) reps = 1;
   double* backup = nullptr;
   IDFX_CK(cudaMalloc(&backup, e.pool_len * sizeof(double)));

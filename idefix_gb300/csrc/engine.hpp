@@ -28,6 +28,7 @@ struct Engine {
   int log_period = 0, check_nan_period = 0;
   long long ncycles = 0;     // host mirror of the cycle counter
   int seg[3] = {32, 32, 32}; // marching segment per direction
+  int sms = 152;             // multiprocessors of the device
   int only_dir = -1;         // >= 0: sweeps launch that direction alone (autotuner)
   bool stage_outputs = false;  // mixed path: a stage end queued in this run wrote the next stage's inputs
   bool faces_saved = false;    // periodic block: the last face update queued wrote the next cycle's Vs0

@@ -11,6 +11,7 @@
 
 #include "../../include/idefix_gb300.h"
 #include "ensemble.hpp"
+#include "sweep_cell.cuh"
 
 using namespace idfx;
 
@@ -174,8 +175,15 @@ int upload_table(EnsEngine& e, EnsTable& t, const std::vector<int4>& items) {
   return IDFX_OK;
 }
 
-std::vector<int4> sweep_items(const EnsEngine& e, int dir, const std::vector<int>& boxes) {
+std::vector<int4> sweep_items(const EnsEngine& e, int dir, const std::vector<int>& boxes, int nt) {
   std::vector<int4> v;
+  if (e.precision == IDFX_FP64) {  // one entry per tile of nt cells
+    for (int b : boxes) {
+      const long long n = cell_tiles(e.boxes[b].g, dir, nt);
+      for (long long x = 0; x < n; x++) v.push_back(make_int4(b, (int)x, 0, 0));
+    }
+    return v;
+  }
   for (int b : boxes) {
     const Geo& g = e.boxes[b].g;
     const long long nx = (sweep_cols(g, dir) + kTM - 1) / kTM;
@@ -214,7 +222,18 @@ int build_tables(EnsEngine& e) {
   if (!rc) rc = upload_table(e, e.begin64, begin64);
   if (!rc) rc = upload_table(e, e.edges64, edges64);
   if (!rc) rc = upload_table(e, e.active64, active64);
-  for (int d = 0; d < e.D && !rc; d++) rc = upload_table(e, e.sweep[d], sweep_items(e, d, order));
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  for (int d = 0; d < e.D && !rc; d++) {
+    e.cell_nt[d] = cell_threads(sms, [&](int t) {
+      long long n = 0;
+      for (int b = 0; b < e.nbox; b++) n += cell_tiles(e.boxes[b].g, d, t);
+      return n;
+    });
+    rc = upload_table(e, e.sweep[d], sweep_items(e, d, order, e.cell_nt[d]));
+    if (!rc && e.precision == IDFX_FP64) rc = upload_table(e, e.sweep64[d], sweep_items(e, d, order, kTM));
+  }
   return rc;
 }
 
@@ -402,6 +421,7 @@ float time_sweep(EnsEngine& e, int dir, const EnsTable& t, int reps, cudaEvent_t
 // sweeps accumulate into Uc, InvDt and the EMF arrays, so the whole state is
 // saved first and put back afterwards.
 int autotune(EnsEngine& e, int reps) {
+  if (e.precision == IDFX_FP64) return IDFX_OK;  // the FP64 sweeps have no segments
   double* backup = nullptr;
   if (cudaMalloc(&backup, e.pool_len * sizeof(double)) != cudaSuccess)
     return ens_fail(e, IDFX_ERR_CUDA, "autotune: no room for the state backup");
@@ -432,7 +452,7 @@ int autotune(EnsEngine& e, int reps) {
         if (s > kv.first[d]) break;
         for (int b : members) e.boxes[b].seg[d] = s;
         rc = upload_boxes(e);
-        if (!rc) rc = upload_table(e, trial, sweep_items(e, d, members));
+        if (!rc) rc = upload_table(e, trial, sweep_items(e, d, members, e.cell_nt[d]));
         if (rc) break;
         const float ms = time_sweep(e, d, trial, reps, ea, eb);
         if (ms < best_ms) {
@@ -500,8 +520,9 @@ EnsPersist ens_persist_args(const EnsEngine& e) {
   P.active = e.active64.items;
   P.nactive = e.active64.n;
   for (int d = 0; d < 3; d++) {
-    P.sweep[d] = e.sweep[d].items;
-    P.nsweep[d] = d < e.D ? e.sweep[d].n : 0;
+    const EnsTable& t = e.precision == IDFX_FP64 ? e.sweep64[d] : e.sweep[d];
+    P.sweep[d] = t.items;
+    P.nsweep[d] = d < e.D ? t.n : 0;
   }
   P.nbox = e.nbox;
   P.nstages = e.nstages;

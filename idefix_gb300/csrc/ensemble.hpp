@@ -61,9 +61,12 @@ struct EnsEngine {
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   EnsTable fill, begin, sweep[3], edges, active;
+  EnsTable sweep64[3];                          // FP64 sweeps: tiles of 64 cells (persistent kernel)
+  int cell_nt[3] = {128, 128, 128};             // FP64 sweeps: threads of the batched launches' blocks
   EnsTable fill64, begin64, edges64, active64;  // the same phases at 64 threads per item (persistent kernel)
   std::vector<EnsTable*> tables() {
-    return {&fill, &begin, &sweep[0], &sweep[1], &sweep[2], &edges, &active, &fill64, &begin64, &edges64, &active64};
+    return {&fill, &begin, &sweep[0], &sweep[1], &sweep[2], &edges, &active, &sweep64[0], &sweep64[1],
+            &sweep64[2], &fill64, &begin64, &edges64, &active64};
   }
   GridBar* d_bar = nullptr;
   cudaGraphExec_t exec_persist = nullptr;  // one chunk of cycles as one persistent launch

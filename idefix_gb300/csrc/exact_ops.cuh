@@ -65,17 +65,32 @@ IDFX_HD T times_sign(T x, T s, uint64_t sb) {
   }
 }
 
-// x 2^K, exact: on the FP64 path an add to the exponent field (the FP64 pipe
-// is what the sweeps wait for), zeros as they are, and the product where the
-// result could leave the normal range; FP32 the product
+// 0 x and x / 2
+IDFX_HD double zero_times(double x) {  // (+0) x
+  const uint64_t u = dbits(x);
+  if (((u >> 52) & 0x7ffu) != 0x7ffu) return dfrom(u & (1ull << 63));
+  return dfrom(0x7FF8000000000000ull);
+}
+IDFX_HD double half_of(double x) {
+  const uint64_t u = dbits(x);
+  const uint32_t e = (uint32_t)(u >> 52) & 0x7ffu;
+  if (e - 2u < 2045u) return dfrom(u - (1ull << 52));
+  if ((u << 1) == 0ull) return x;
+  return rare_mul(0.5, x);
+}
+
+// x 2^K: on the FP64 path an add to the exponent field (the FP64 pipe is what
+// the sweeps wait for), zeros as they are, and the product, as a call, where
+// the result could leave the normal range; FP32 the product
 template <int K, typename T>
 IDFX_HD T pow2x(T x) {
-  constexpr double f = K >= 0 ? (double)(1 << (K >= 0 ? K : 0)) : 1.0 / (double)(1 << (K < 0 ? -K : 0));
+  static_assert(K >= -1 && K <= 2, "half, twice, four times");
+  constexpr double f = K < 0 ? 0.5 : (double)(1 << (K < 0 ? 0 : K));
   if constexpr (sizeof(T) == 8) {
     const uint64_t u = dbits(x);
     if (((uint32_t)(u >> 52) & 0x7ffu) - 64u < 1920u) return dfrom(u + ((uint64_t)(int64_t)K << 52));
     if ((u << 1) == 0ull) return x;
-    return x * f;
+    return rare_mul(x, f);
   } else {
     return x * T(f);
   }
@@ -97,6 +112,67 @@ IDFX_HD bool lt(T x, T y) {
   }
 }
 
+// x <= y, and |x| >= |y|, the same way
+template <typename T>
+IDFX_HD bool le(T x, T y) {
+  if constexpr (sizeof(T) == 8) {
+    const uint64_t I = 0x7FF0000000000000ull << 1;
+    return (dbits(x) << 1) <= I && (dbits(y) << 1) <= I && !lt(y, x);
+  } else {
+    return x <= y;
+  }
+}
+template <typename T>
+IDFX_HD bool abs_ge(T x, T y) {
+  if constexpr (sizeof(T) == 8) {
+    const uint64_t u = dbits(x) << 1, w = dbits(y) << 1, I = 0x7FF0000000000000ull << 1;
+    return u <= I && w <= u;
+  } else {
+    return fabsf(x) >= fabsf(y);
+  }
+}
+
+// the sign of x: -1, 0 (zeros, NaN) or 1; and s |x| for such a sign and
+// x >= 0, the product's value (0 x where s is 0)
+template <typename T>
+IDFX_HD int sgn_of(T x) {
+  return (int)gt0(x) - (int)lt0(x);
+}
+template <typename T>
+IDFX_HD T times_sgn(int s, T x) {
+  if constexpr (sizeof(T) == 8) {
+    if (s == 0) return zero_times(x);
+    return dfrom(dbits(x) ^ (s < 0 ? 1ull << 63 : 0ull));
+  } else {
+    return s * x;
+  }
+}
+
+// x y < 0 and x y <= 0: on the FP64 path from the signs where both exponents
+// are far enough from the ends for the product to be normal, else the product
+template <typename T>
+IDFX_HD bool prod_lt0(T x, T y) {
+  if constexpr (sizeof(T) == 8) {
+    const uint64_t u = dbits(x), w = dbits(y);
+    if (((uint32_t)(u >> 52) & 0x7ffu) - 513u < 1022u && ((uint32_t)(w >> 52) & 0x7ffu) - 513u < 1022u)
+      return ((u ^ w) >> 63) != 0ull;
+    return lt0(rare_mul(x, y));
+  } else {
+    return x * y < T(0);
+  }
+}
+template <typename T>
+IDFX_HD bool prod_le0(T x, T y) {
+  if constexpr (sizeof(T) == 8) {
+    const uint64_t u = dbits(x), w = dbits(y);
+    if (((uint32_t)(u >> 52) & 0x7ffu) - 513u < 1022u && ((uint32_t)(w >> 52) & 0x7ffu) - 513u < 1022u)
+      return ((u ^ w) >> 63) != 0ull;
+    return le0(rare_mul(x, y));
+  } else {
+    return x * y <= T(0);
+  }
+}
+
 // One upwind term of CalcContactAverage, (1 - w) a + w b with the weight w
 // in {0, 1/2, 1} (storeFlux.hpp:40-43).  The FP64 path forms the two
 // products exactly on the integer pipe - a product by 1 is the value, by 0 a
@@ -104,18 +180,6 @@ IDFX_HD bool lt(T x, T y) {
 // w's bit pattern, so only the sum issues on the FP64 pipe; any other weight,
 // and non-finite or subnormal values, take the FP64 expression.  Every case
 // is bit-identical to the reference's expression.
-IDFX_HD double zero_times(double x) {  // (+0) x
-  const uint64_t u = dbits(x);
-  if (((u >> 52) & 0x7ffu) != 0x7ffu) return dfrom(u & (1ull << 63));
-  return 0.0 * x;
-}
-IDFX_HD double half_of(double x) {  // x / 2
-  const uint64_t u = dbits(x);
-  const uint32_t e = (uint32_t)(u >> 52) & 0x7ffu;
-  if (e - 2u < 2045u) return dfrom(u - (1ull << 52));
-  if ((u << 1) == 0ull) return x;
-  return 0.5 * x;
-}
 template <typename E>
 IDFX_HD E upwind_term(E w, E a, E b) {
   if constexpr (sizeof(E) == 8) {
@@ -131,8 +195,8 @@ IDFX_HD E upwind_term(E w, E a, E b) {
       p = half_of(a);
       q = half_of(b);
     } else {
-      p = (1.0 - w) * a;
-      q = w * b;
+      p = rare_mul(rare_add(1.0, -w), a);
+      q = rare_mul(w, b);
     }
     return p + q;
   } else {

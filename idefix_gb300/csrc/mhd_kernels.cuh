@@ -277,7 +277,8 @@ __device__ __forceinline__ void stage_begin_cell(const Geo& g, const Fields& f, 
 #pragma unroll
   for (int d = 0; d < D; d++) {
     const double* vs = f.Vs + d * g.nface;
-    V[v::BX1 + d] = 0.5 * (vs[fc] + vs[fc + g.fs[d]]);
+    const double b2 = vs[fc] + vs[fc + g.fs[d]];
+    V[v::BX1 + d] = sizeof(E) == 8 ? pow2x<-1>(b2) : 0.5 * b2;  // FP64 path: the half off the FP64 pipe
   }
   if (copy) {
 #pragma unroll
@@ -654,7 +655,8 @@ __device__ __forceinline__ void store_emf(const Geo& g, const Fields& f, long lo
 }
 
 // ---------------------------------------------------------------------------
-// Flux sweeps (RiemannSolver::CalcFlux<DIR> + Fluid_CorrectFluxFunctor +
+// FP32 flux sweeps (the FP64 ones are in sweep_cell.cuh;
+// RiemannSolver::CalcFlux<DIR> + Fluid_CorrectFluxFunctor +
 // Fluid_CalcRHSFunctor, calcRightHandSide.hpp:84-195,333-550): each thread
 // owns one column (a line of cells along DIR) and marches a segment of `seg`
 // cells, keeping the reconstruction stencil, the left face state and the
@@ -668,10 +670,8 @@ __device__ __forceinline__ void store_emf(const Geo& g, const Fields& f, long lo
 // ---------------------------------------------------------------------------
 constexpr int kTM = 64;
 
-// T: arithmetic of the reconstruction and the Riemann solve (double: the
-// bit-exact path; float: the mixed-precision path).  The state is read in
-// FP64 and converted once per cell; the flux difference, the conserved
-// update and InvDt are FP64 in both.
+// T = float: reconstruction and Riemann solve of the mixed path; the
+// conserved state and InvDt accumulate in FP64.
 template <int D, int DIR, int ORDER, int SOLVER, typename T>
 __device__ __forceinline__ void d_sweep_march(const Geo& g, const Fields& f, const Ctl* ctl, int invdt,
                                               int last_dir, int seg, dim3 bid) {
@@ -683,10 +683,9 @@ __device__ __forceinline__ void d_sweep_march(const Geo& g, const Fields& f, con
   constexpr int W = 2 * H + 1;
   constexpr int A = (DIR == 0) ? 1 : 0;
   constexpr int B = (DIR == 2) ? 1 : 2;
-  // FP32 sweeps are load-latency bound: issue the next step's loads before
-  // the current step's arithmetic.  FP64 sweeps are FP64-issue bound and
-  // keep their registers for the arithmetic.
-  constexpr bool PF = (sizeof(T) == 4);
+  static_assert(sizeof(T) == 4, "marching sweep: FP32 path");
+  // load-latency bound: the next step's loads are issued before the current
+  // step's arithmetic
   // flattened column index over the (A, B) plane, CT extension included
   const int nA = g.n[A] + 2 * g.ext;
   const int nB = (D == 3) ? g.n[B] + 2 * g.ext : 1;
@@ -712,17 +711,10 @@ __device__ __forceinline__ void d_sweep_march(const Geo& g, const Fields& f, con
   const T gam = (T)g.gamma;
   T w[NV][W];
   T vrp[NV];            // right-face state of the previous cell
-  T dl[NV];             // PLM in FP64: the next cell's difference on the left
   T Fp[v::BX1];         // flux x A of the previous face
   T cp = T(0);          // cmax of the previous face
   T nx[NV];             // prefetched stencil value of the next step
-  // primitives in the arithmetic type: the FP32 copy for the mixed path
-  const T* vcT;
-  if constexpr (sizeof(T) == 4) {
-    vcT = f.Vc32;
-  } else {
-    vcT = f.Vc;
-  }
+  const T* vcT = f.Vc32;
   double nbn = 0.0;     // prefetched normal face field of the next face
   double nU[v::BX1];    // prefetched conserved state of the next cell to update
   double nI = 0.0;      // prefetched InvDt of that cell
@@ -732,36 +724,19 @@ __device__ __forceinline__ void d_sweep_march(const Geo& g, const Fields& f, con
     if (n == dd::BXn) continue;
 #pragma unroll
     for (int m = 0; m < W - 1; m++) w[n][m + 1] = vcT[n * g.ncell + c0 + (m - 1 - H) * sd];
-    if constexpr (ORDER == 2 && sizeof(T) == 8) dl[n] = w[n][2] - w[n][1];
-    if constexpr (PF) nx[n] = vcT[n * g.ncell + c0 + (H - 1) * sd];
+    nx[n] = vcT[n * g.ncell + c0 + (H - 1) * sd];
   }
-  if constexpr (PF) nbn = vs[f0];
+  nbn = vs[f0];
   const T dtdVT = (T)ctl->dtdV;
   const T areaT = (T)g.A[DIR];
-  const T invdxT = T(1) / (T)g.dx[DIR];  // FP32 path only
-  double run_max = 0.0;                  // max of InvDt over this thread's cells
+  const T invdxT = T(1) / (T)g.dx[DIR];
+  double run_max = 0.0;  // max of InvDt over this thread's cells
   for (int c = m0 - 1; c <= m1; c++) {
     const long long cc = c0 + (long long)(c - m0) * sd;
     const bool more = c < m1;
     double curU[v::BX1];
     double curI = 0.0;
-    if constexpr (!PF && DIR != 0) {
-      // FP64: the same L2 prefetch along y and z, kPrefetch steps ahead (the
-      // step's loads are otherwise issued right before their use; measured:
-      // y and z sweeps 35.15 -> 34.90 ms per 256^3 cycle, an L1 prefetch
-      // no better)
-      if (c + kPrefetch + H + 1 < g.nt[DIR]) {
-#pragma unroll
-        for (int n = 0; n < NV; n++)
-          if (n != dd::BXn) prefetch_l2(vcT + n * g.ncell + cc + (kPrefetch + H + 1) * sd);
-        prefetch_l2(vs + f0 + (long long)(c + 1 + kPrefetch - m0) * fsd);
-        if (active_col) {
-#pragma unroll
-          for (int n = 0; n < v::BX1; n++) prefetch_l2(f.Uc + n * g.ncell + cc + kPrefetch * sd);
-        }
-      }
-    }
-    if constexpr (PF) {
+    {
       // L2 prefetch kPrefetch steps ahead along y (measured: +11 % on the
       // FP32 y sweep; along x consecutive steps share cache lines and the
       // extra requests cost more than they save, along z no gain); only
@@ -795,21 +770,9 @@ __device__ __forceinline__ void d_sweep_march(const Geo& g, const Fields& f, con
       if (n == dd::BXn) continue;
 #pragma unroll
       for (int m = 0; m < W - 1; m++) w[n][m] = w[n][m + 1];
-      if constexpr (PF) {
-        w[n][W - 1] = nx[n];
-        if (more) nx[n] = vcT[n * g.ncell + cc + (H + 1) * sd];
-      } else {
-        w[n][W - 1] = vcT[n * g.ncell + cc + H * sd];
-      }
-      if constexpr (ORDER == 2 && sizeof(T) == 8) {
-        // PLM in FP64: the difference on the left is the last step's on the
-        // right (the same operation on the same values)
-        const T dvp = w[n][2] - w[n][1];
-        Recon<ORDER>::plm(w[n][1], dl[n], dvp, shk, vl[n], vr[n]);
-        dl[n] = dvp;
-      } else {
-        Recon<ORDER>::cell(w[n], dxd, n == v::RHO || n == v::PRS, vl[n], vr[n], shk, l3);
-      }
+      w[n][W - 1] = nx[n];
+      if (more) nx[n] = vcT[n * g.ncell + cc + (H + 1) * sd];
+      Recon<ORDER>::cell(w[n], dxd, n == v::RHO || n == v::PRS, vl[n], vr[n], shk, l3);
     }
     if (c >= m0) {
       T vL[NV], vR[NV];
@@ -819,22 +782,16 @@ __device__ __forceinline__ void d_sweep_march(const Geo& g, const Fields& f, con
         vL[n] = vrp[n];
         vR[n] = vl[n];
       }
-      T bn;
-      if constexpr (PF) {
-        bn = from_f64<T>(nbn);
-        if (more) nbn = vs[f0 + (long long)(c + 1 - m0) * fsd];
-      } else {
-        bn = from_f64<T>(vs[f0 + (long long)(c - m0) * fsd]);
-      }
+      const T bn = from_f64<T>(nbn);
+      if (more) nbn = vs[f0 + (long long)(c + 1 - m0) * fsd];
       vL[dd::BXn] = bn;
       vR[dd::BXn] = bn;
       RiemannOut<D, T> r;
       riemann<D, DIR, SOLVER>(gam, (T)g.rgm1, vL, vR, r);
       store_emf<D, DIR>(g, f, cc, r, vL, vR);
       if (active_col) {
-        // flux x area and the flux difference in the arithmetic type T; the
-        // conserved state accumulates in FP64 (for T = double this is the
-        // reference's expression, operation for operation)
+        // flux x area and the flux difference in FP32; the conserved state
+        // accumulates in FP64
         T FA[v::BX1];
 #pragma unroll
         for (int n = 0; n < v::BX1; n++) FA[n] = r.F[n] * areaT;
@@ -843,17 +800,11 @@ __device__ __forceinline__ void d_sweep_march(const Geo& g, const Fields& f, con
 #pragma unroll
           for (int n = 0; n < v::BX1; n++) {
             const T rhs = -dtdVT * (FA[n] - Fp[n]);
-            const double u = PF ? curU[n] : f.Uc[n * g.ncell + cu];
-            f.Uc[n * g.ncell + cu] = u + to_f64(rhs);
+            f.Uc[n * g.ncell + cu] = curU[n] + to_f64(rhs);
           }
           if (invdt) {
-            const double prev = (invdt == 1) ? 0.0 : (PF ? curI : f.InvDt[cu]);
-            double inv;
-            if constexpr (sizeof(T) == 8) {
-              inv = prev + div_r(pow2x<-1>(r.cmax + cp), Recip{g.dx[DIR], g.rdx[DIR]});
-            } else {
-              inv = prev + to_f64(T(0.5) * (r.cmax + cp) * invdxT);
-            }
+            const double prev = (invdt == 1) ? 0.0 : curI;
+            const double inv = prev + to_f64(T(0.5) * (r.cmax + cp) * invdxT);
             f.InvDt[cu] = inv;
             if (inv > run_max) run_max = inv;  // NaN never compares greater
           }
@@ -1539,6 +1490,7 @@ __device__ __forceinline__ double rk_combine(double u, double u0, double wc, dou
     // RK2's 1/2 (u + u0): the halving exact on the integer pipe
     if (wc == w0) return wc == 0.5 ? half_of(u + u0) : wc * (u + u0);
   }
+  if (wc == 0.5 && w0 == 0.5) return pow2x<-1>(u) + pow2x<-1>(u0);  // the products exact on the integer pipe
   return wc * u + w0 * u0;
 }
 
@@ -1828,7 +1780,17 @@ __device__ __forceinline__ void d_stage_end(const Geo& g, const Fields& f, const
 #pragma unroll
   for (int n = 0; n < v::BX1; n++) {
     double u = f.Uc[n * g.ncell + c];
-    if (combine) u = rk_combine<E>(u, f.Uc0[n * g.ncell + c], wc, w0);
+    if (combine) {
+      // (this pass is not bound by the FP64 pipe: rk_combine's halves on the
+      // integer pipe made it 2.09 instead of 1.99 ms per 256^3 cycle, and 2.19
+      // instead of 1.96 on the mixed path)
+      const double u0 = f.Uc0[n * g.ncell + c];
+      if (sizeof(E) == 4 && wc == w0) {
+        u = wc * (u + u0);
+      } else {
+        u = wc * u + w0 * u0;
+      }
+    }
     U[n] = u;
   }
 #pragma unroll

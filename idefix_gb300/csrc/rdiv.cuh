@@ -61,7 +61,7 @@ IDFX_HD double div_r(double a, const Recip& R) {
     }
     if ((A << 1) == 0ull) return dfrom((A ^ B) & (1ull << 63));  // +-0 / b
   }
-  return a / R.b;
+  return rare_div(a, R.b);
 }
 
 }  // namespace idfx

@@ -1,33 +1,31 @@
-// Correctly rounded FP64 quotients and square roots from FP32 seeds.
+// Correctly rounded FP64 quotients and square roots without the FP64 pipe.
 //
 // One FP64 instruction holds a scheduler's FP64 pipe for 64 cycles here (76
 // with all four busy: about 520 G thread-operations per second for the whole
 // GPU), while FP32 and integer instructions issue every cycle beside it; the
 // flux sweeps run at that pipe's rate.  A hardware-sequence division takes
 // 7.2 pipe operations, a square root 7.5, a reciprocal 4.5 (measured on
-// independent chains).  The forms below take three each:
-//   q0   the quotient to about 42 bits, in FP32 pairs: the significands of
-//        a and b as head + tail, a hardware reciprocal y of b's head, one
-//        residual correction; assembled into a double with integer
-//        operations
-//   r0 = a - b q0            (one FMA)
-//   q1 = q0 + r0 y           (one FMA; within 2^-11 ulp of a correctly
-//                             rounded step: 42 + 22 bits)
-//   r1 = a - b q1            (one FMA, exact)
-// q1 is the correctly rounded quotient exactly when |r1| < |b| ulp(q1) / 2
-// (half of that where q1 is a power of two, whose lower neighbour is nearer);
-// the test compares the leading words of the bit patterns.  Where it does
-// not hold (about one quotient in 2^11, and every quotient whose FP32 pair
-// straddles a binade), or an exponent is outside a safe band, or an operand
-// is zero, subnormal, infinite or NaN, the hardware operation gives the
-// result.  So the result is the IEEE one for every input, whatever the
-// accuracy of the seed.  The square root is the same with s1^2 in place of
-// b q1: s1 is right exactly when |x - s1^2| < s1 ulp(s1) (x - s1^2 is a
-// multiple of ulp(s1)^2, so the quarter-ulp^2 terms cannot matter).
-// Measured with the limiter, HLLD and fast speeds on these forms (and the
-// halves, fours and comparisons on the integer pipe): the three FP64 sweeps
-// of 256^3 cells (PLM, HLLD, both stages) 33.5 / 33.6 / 33.4 -> 27.5 / 27.1 /
-// 26.6 ms.
+// independent chains).  Here a quotient is formed from the significands m
+// and d (m in [d, 2 d)) with FP32 pairs and integers alone:
+//   q0  m / d to about 41 bits in FP32 pairs - head and tail of both, a
+//       hardware reciprocal f of d's head, one residual correction - as an
+//       integer in units of 2^-42, two units low so that
+//   r0 = m 2^42 - d q0      is positive (it fits 64 bits, so 64-bit wrapping
+//                           arithmetic gives it exactly)
+//   c  = the nearest integer to r0 2^10 f, twelve bits
+//   r1 = r0 2^10 - d c      exact, within (1/2 + 2^-9) d of zero
+// and q = q0 2^10 + c, one more or less where |r1| > d / 2 (equality cannot
+// be: d has 53 bits and the quotient one bit more would have to divide it).
+// The residual decides the rounding exactly, so the result is the IEEE one
+// for every input, whatever the last bits of the seed.  The square root is the same
+// with r0 = x 2^32 - s0^2 and r1 = r0 2^20 - c (s0 2^11 + c), against s: s is
+// right exactly when -s < r1 <= s.  Exponents outside a safe band, zeros,
+// subnormals, infinities and NaNs take the hardware operation.
+// Measured on the 256^3 FP64 sweeps (x / y / z, both stages): hardware
+// sequences 33.5 / 33.6 / 33.4 ms, a form with three FP64 operations per
+// quotient (and the halves, fours and comparisons on the integer pipe) 27.5 /
+// 27.1 / 26.6 ms with the marching sweep and 25.1 / 25.4 / 25.2 ms with a thread
+// per cell, this form 19.1 / 19.4 / 19.2 ms.
 // Newton's iteration with a residual test of the rounding, as in J.-M.
 // Muller et al., Handbook of Floating-Point Arithmetic, ch. on division and
 // square root.  Checked bit for bit against `/` and `sqrt` on the host and
@@ -37,9 +35,17 @@
 #include <stdint.h>
 
 #include "fpconv.cuh"  // fbits / ffrom
-#include "rdiv.cuh"    // fma_rn
+#include "rdiv.cuh"
 
 namespace idfx {
+
+// a called function on the device: some thirty quotients and roots of one
+// face inlined are half of a sweep's instructions (256^3 sweeps 3 % slower)
+#ifdef __CUDACC__
+#define IDFX_CALL static __device__ __noinline__
+#else
+#define IDFX_CALL inline
+#endif
 
 // approximate 1 / sqrt of a float in [1, 4)
 IDFX_HD float rsqrt_seed(float f) {
@@ -58,10 +64,13 @@ IDFX_HD float fma_f(float a, float b, float c) {
   return fmaf(a, b, c);
 #endif
 }
+IDFX_HD float clamp_f(float x, float lo, float hi) { return fminf(fmaxf(x, lo), hi); }
 
-// exponent field inside [200, 1800): products, residuals and ulps of such
-// operands stay normal
+// exponent field inside [200, 1800)
 IDFX_HD bool seed_band(uint32_t e) { return e - 200u < 1600u; }
+
+// the significand of u with its leading one
+IDFX_HD uint64_t significand(uint64_t u) { return (u & 0xfffffffffffffull) | (1ull << 52); }
 
 // head and tail (24 + 23 bits) of the significand of u times 2^odd, in [1, 2)
 // (odd = 0) or [2, 4)
@@ -71,91 +80,90 @@ IDFX_HD void seed_split(uint64_t u, uint32_t odd, float& h, float& l) {
   l = ffrom((((uint32_t)u >> 6) & 0x7fffffu) + 0x34000000u + o) - ffrom(0x34000000u + o);
 }
 
-// the double head + tail (|tail| < 2^-20 of head's binade), times 2^(e - 896)
-// and with the sign bit s: the tail rounded to 2^-42 of the binade
-IDFX_HD double seed_join(float h, float l, uint32_t e, uint64_t s) {
-  const uint32_t f = fbits(h);
-  const uint32_t m = (f & 0x7f800000u) - (19u << 23) + 0x400000u;  // 1.5 x 2^-19 of the binade
-  const int32_t t = (int32_t)(fbits(ffrom(m) + l) - m);
-  return dfrom((((uint64_t)f << 29) + ((uint64_t)e << 52) + ((uint64_t)(int64_t)t << 10)) | s);
+// head h in [1, 2) plus tail e f (|tail| < 2^-20) as an integer in units of
+// 2^-42, `low` units less
+IDFX_HD uint64_t seed_fixed(float h, float e, float f, uint32_t low) {
+  const uint32_t m = 0x36400000u;  // 1.5 x 2^-19: its last place is 2^-42
+  const int32_t t = (int32_t)(fbits(fma_f(e, f, ffrom(m))) - (m + low));
+  return ((uint64_t)((fbits(h) & 0x7fffffu) | 0x800000u) << 19) + (uint64_t)(int64_t)t;
 }
 
-// the leading word of |x|
-IDFX_HD uint32_t abs_hi(double x) { return (uint32_t)(dbits(x) >> 32) & 0x7fffffffu; }
+// nearest integer to x f 2^k, for 0 <= x f 2^k < 2^22
+IDFX_HD uint32_t seed_round(uint32_t x, float f) {
+  return fbits(fma_f((float)x, f, 8388608.0f)) - 0x4b000000u;
+}
 
 // a divisor prepared for several quotients
 struct SeedDiv {
   double b;
-  double y;      // about 1 / b (22 bits)
-  float h, l, f; // significand head and tail, and the head's reciprocal
-  bool ok;       // b's exponent is inside the band
+  float h, l, f;  // significand head and tail, and the head's reciprocal
 };
 
 IDFX_HD SeedDiv seed_div(double b) {
   SeedDiv d;
-  const uint64_t B = dbits(b);
-  const uint32_t eb = (uint32_t)(B >> 52) & 0x7ffu;
   d.b = b;
-  d.ok = seed_band(eb);
-  seed_split(B, 0u, d.h, d.l);
+  seed_split(dbits(b), 0u, d.h, d.l);
   d.f = rcp_seed(d.h);
-  d.y = dfrom((((uint64_t)fbits(d.f) << 29) + ((uint64_t)(1919u - eb) << 52)) ^ (B & (1ull << 63)));
   return d;
 }
 
-// a / d.b into q; false where the hardware division has to be taken
-IDFX_HD bool try_seed_quot(double a, const SeedDiv& d, double& q) {
-  const uint64_t A = dbits(a), B = dbits(d.b);
+// a / D.b into q; false where the hardware division has to be taken
+IDFX_HD bool try_quot(double a, const SeedDiv& D, double& q) {
+  const uint64_t A = dbits(a), B = dbits(D.b);
   const uint32_t ea = (uint32_t)(A >> 52) & 0x7ffu;
   const uint32_t eb = (uint32_t)(B >> 52) & 0x7ffu;
+  const uint64_t ma = significand(A), d = significand(B);
+  const uint32_t up = ma < d ? 1u : 0u;  // m in [d, 2 d)
+  const uint64_t m = ma << up;
   float ah, al;
-  seed_split(A, 0u, ah, al);
-  const float qh = ah * d.f;
-  const float e = fma_f(-d.l, qh, fma_f(-d.h, qh, ah) + al);
-  const uint64_t s = (A ^ B) & (1ull << 63);
-  const double q0 = seed_join(qh, e * d.f, 896u + ea - eb, s);
-  const double r0 = fma_rn(-q0, d.b, a);
-  const double q1 = fma_rn(r0, d.y, q0);
-  const double r1 = fma_rn(-q1, d.b, a);
-  const uint64_t Q = dbits(q1);
-  // |b| ulp(q1) / 2: the exponents added, 1023 + 53 off; one less at a power of two
-  uint32_t lim = abs_hi(d.b) + (((uint32_t)(Q >> 52) & 0x7ffu) << 20) - (1076u << 20);
-  if ((Q << 12) == 0ull) lim -= 1u << 20;
-  q = q1;
-  return d.ok && seed_band(ea) && seed_band(ea - eb + 1023u) && abs_hi(r1) < lim;
+  seed_split(A, up, ah, al);
+  const float qh = clamp_f(ah * D.f, 1.0f, 1.99999988f);
+  const float e = fma_f(-D.l, qh, fma_f(-D.h, qh, ah) + al);
+  const uint64_t q0 = seed_fixed(qh, e, D.f, 2u);
+  const uint64_t r0 = (m << 42) - d * q0;
+  const uint32_t c = seed_round((uint32_t)(r0 >> 24), D.f * ffrom((127u - 18u) << 23));
+  const int64_t r1 = (int64_t)((r0 << 10) - d * c);
+  uint64_t z = (q0 << 10) + c;
+  if (2 * r1 > (int64_t)d) z += 1ull;
+  if (2 * r1 < -(int64_t)d) z -= 1ull;
+  const uint32_t eq = ea - eb + 1022u - up;
+  q = dfrom((z + ((uint64_t)eq << 52)) | ((A ^ B) & (1ull << 63)));
+  return seed_band(ea) && seed_band(eb) && seed_band(eq);
 }
 
-// a / d.b, correctly rounded
-IDFX_HD double quot(double a, const SeedDiv& d) {
+// a / D.b, correctly rounded
+IDFX_HD double quot(double a, const SeedDiv& D) {
   double q;
-  if (try_seed_quot(a, d, q)) return q;
-  return a / d.b;
+  if (try_quot(a, D, q)) return q;
+  return rare_div(a, D.b);
 }
 // a / b, correctly rounded
-IDFX_HD double quot(double a, double b) { return quot(a, seed_div(b)); }
+IDFX_CALL double quot(double a, double b) { return quot(a, seed_div(b)); }
 
 // sqrt(x), correctly rounded
-IDFX_HD double root(double x) {
+IDFX_CALL double root(double x) {
   const uint64_t X = dbits(x);
   const uint32_t ex = (uint32_t)(X >> 52);  // with the sign bit: negative x is outside the band
   const uint32_t odd = (ex + 1u) & 1u;      // 2^(ex - 1023) = 2^odd 4^k
   const uint32_t k = (ex + 1u - odd) >> 1;  // k + 512
+  const uint64_t m = significand(X) << odd;
   float h, l;
   seed_split(X, odd, h, l);
   const float f = rsqrt_seed(h);
-  const float sh = h * f;
+  const float sh = clamp_f(h * f, 1.0f, 1.99999988f);
   const float e = fma_f(-sh, sh, h) + l;
-  const double s0 = seed_join(sh, e * (0.5f * f), 896u + k - 512u, 0ull);
-  const double y = dfrom(((uint64_t)fbits(f) << 29) + ((uint64_t)(895u + 512u - k) << 52));  // about 1 / (2 sqrt(x))
-  const double r0 = fma_rn(-s0, s0, x);
-  const double s1 = fma_rn(r0, y, s0);
-  const double r1 = fma_rn(-s1, s1, x);
-  const uint64_t S = dbits(s1);
-  // s1 ulp(s1): the exponents added, 1023 + 52 off; half at a power of two
-  uint32_t lim = (uint32_t)(S >> 32) + (((uint32_t)(S >> 52) & 0x7ffu) << 20) - (1075u << 20);
-  if ((S << 12) == 0ull) lim -= 1u << 20;
-  if (seed_band(ex) && abs_hi(r1) < lim) return s1;
-  return sqrt(x);
+  const uint64_t s0 = seed_fixed(sh, e, 0.5f * f, 2u);
+  const uint64_t r0 = (m << 32) - s0 * s0;
+  const uint32_t c = seed_round((uint32_t)(r0 >> 16), f * ffrom((127u - 17u) << 23));
+  const int64_t r1 = (int64_t)((r0 << 20) - ((s0 << 11) + c) * c);
+  uint64_t z = (s0 << 10) + c;
+  if (r1 > (int64_t)z) {
+    z += 1ull;
+  } else if (r1 <= -(int64_t)z) {
+    z -= 1ull;
+  }
+  if (seed_band(ex)) return dfrom(z + ((uint64_t)(k + 510u) << 52));
+  return rare_sqrt(x);
 }
 
 }  // namespace idfx

@@ -1,0 +1,239 @@
+// FP64 flux sweeps with one thread per cell (every direction, 2-D and 3-D).
+#pragma once
+#include "mhd_kernels.cuh"
+
+namespace idfx {
+
+// ---------------------------------------------------------------------------
+// The lines of cells along the sweep direction (the active cells and one
+// ghost cell at each end, for every column of the other two directions
+// including the CT extension) are laid end to end, `cols` neighbouring lines
+// side by side, and the sequence is cut into tiles of blockDim.x cells that
+// overlap by two positions: thread t holds column t % cols of position
+// t / cols of its tile.  A thread reconstructs its cell, hands the right-face
+// state to the thread of the next position through shared memory, solves the
+// face on the left of its cell, hands flux and wave speed to the thread of
+// the position before it, and updates its cell - one reconstruction and one
+// Riemann problem deep, where the march of one thread along a segment of s
+// cells goes through s + 2 and s + 1 of them one after the other.
+//   Why: the FP64 pipe bounds these sweeps (seeddiv.cuh), and one warp per
+// scheduler already fills it, so what a launch costs is its FP64 work shared
+// out evenly.  A march repeats two reconstructions and a face per segment: short
+// segments, which fill the GPU at small and middle sizes, repeat half of their
+// work and more; long ones leave it idle.  Here the overlap of a tile is the only
+// work done twice (2 of 128 positions along x, 2 of 128 / cols across it), at every size.
+// PPM needs one position more at the front: the limited value of a face and
+// the second difference of a cell are formed once, by the thread of the cell
+// on the left, and handed on.
+// Measured (both stages of a cycle, x / y / z sweeps): 256^3 PLM + HLLD 27.5 /
+// 27.1 / 26.6 -> 25.1 / 25.4 / 25.2 ms against the march, 64^3 0.75 / 0.75 / 0.76
+// -> 0.49 / 0.52 / 0.52 ms, 2-D 256^2 0.28 / 0.28 -> 0.14 / 0.15 ms, 2-D 64^2
+// 0.10 -> 0.045 ms, 91 x 62 x 45 PPM + HLL (RK3) 3.8 / 3.9 / 3.9 -> 1.5 / 1.7 /
+// 1.8 ms (the segments the block chose for itself); with the quotients and roots off the FP64 pipe
+// (seeddiv.cuh) 256^3 19.1 / 19.4 / 19.2 ms, at the pipe's rate (81 % busy of
+// the 84 % it reaches; 156 registers, 12 warps per multiprocessor; 16 warps at
+// 128 registers were 3 % slower).  Products emulated on the integer pipe
+// beside it (69 issue slots each) took a quarter of the pipe's work away and
+// changed the time by -6 to +10 %: the sweeps' instruction stream then waits on itself.
+// ---------------------------------------------------------------------------
+constexpr int kCellThreads = 128;  // largest block
+
+// columns side by side: lanes along x are neighbours in memory already; across
+// x, two share half a 32-byte sector and cost 2 of 64 positions (256^3 y and z
+// sweeps within 1 % of the x sweep; four columns the same there and 6 % slower
+// at 64^3, eight 4 % slower)
+__host__ __device__ constexpr int cell_cols(int dir) { return dir == 0 ? 1 : 2; }
+// block size for a launch of tiles(nt) blocks of nt threads: smaller blocks
+// where fewer than two per multiprocessor would leave schedulers without a warp
+template <typename Tiles>
+inline int cell_threads(int sms, Tiles tiles) {
+  int nt = kCellThreads;
+  while (nt > 32 && tiles(nt) < 2 * sms) nt /= 2;
+  return nt;
+}
+
+// tiles of nt cells of the lines along dir
+__host__ inline long long cell_tiles(const Geo& g, int dir, int nt) {
+  const int a = (dir == 0) ? 1 : 0, b = (dir == 2) ? 1 : 2, cols = cell_cols(dir);
+  const int lead = (g.order == 4) ? 1 : 0;  // PPM's extra position
+  const int step = nt / cols - 2 - lead;
+  const long long lines = (long long)(g.n[a] + 2 * g.ext) * (g.D == 3 ? g.n[b] + 2 * g.ext : 1);
+  const long long total = (lines + cols - 1) / cols * (g.n[dir] + 2 + lead);
+  return (total - 2 - lead + step - 1) / step;
+}
+
+// shared memory of a block of nt threads: right-face states (PPM: before
+// them, face values and second differences), flux x area and wave speed
+__host__ __device__ constexpr size_t cell_smem_bytes(int D, int nt) {
+  return sizeof(double) * (size_t)((2 * D + 1) + (D + 2) + 1) * (size_t)nt;
+}
+
+template <int D, int DIR, int ORDER, int SOLVER>
+__device__ __forceinline__ void d_sweep_cell(const Geo& g, const Fields& f, const Ctl* ctl, int invdt, int last_dir,
+                                             unsigned tile, double* sm) {
+  if (ctl->done) return;
+  using T = double;
+  using v = Var<D>;
+  using dd = Dir<D, DIR>;
+  constexpr int NV = v::NV, NU = v::BX1, NS = NV - 1;
+  constexpr int H = Recon<ORDER>::H;
+  constexpr int E = (ORDER == 4) ? 1 : 0;
+  constexpr int A = (DIR == 0) ? 1 : 0, B = (DIR == 2) ? 1 : 2;
+  constexpr int cols = cell_cols(DIR);
+  const int nt = (int)blockDim.x, tid = (int)threadIdx.x;
+  double* ss = sm;            // [NS][nt] right-face states
+  double* sf = sm + NS * nt;  // [NU + 1][nt] flux x area, wave speed
+  const int t = tid / cols, npos = nt / cols;
+  // 32-bit indices: a position stands for a cell, of which a device holds
+  // fewer than 2^31
+  const unsigned nA = (unsigned)(g.n[A] + 2 * g.ext);
+  const unsigned nB = (D == 3) ? (unsigned)(g.n[B] + 2 * g.ext) : 1u;
+  const unsigned P = (unsigned)(g.n[DIR] + 2 + E);  // positions of a line: cells beg - 1 - E .. end
+  const unsigned q = tile * (unsigned)(npos - 2 - E) + (unsigned)t;
+  const unsigned bundle = q / P;
+  const int p = (int)(q - bundle * P);
+  const unsigned line = bundle * cols + (unsigned)(tid - t * cols);
+  const bool valid = line < nA * nB;
+  int idx[3];
+  idx[DIR] = g.beg[DIR] - 1 - E + p;
+  idx[A] = g.beg[A] - g.ext + (int)(valid ? line % nA : 0);
+  idx[B] = (D == 3) ? g.beg[B] - g.ext + (int)(valid ? line / nA : 0) : 0;
+  const long long cc = cidx(g, idx[2], idx[1], idx[0]);
+  const long long sd = g.s[DIR];
+  bool active_col = valid && idx[A] >= g.beg[A] && idx[A] < g.end[A];
+  if constexpr (D == 3) active_col = active_col && idx[B] >= g.beg[B] && idx[B] < g.end[B];
+  const bool update = active_col && t >= 1 + E && t <= npos - 2 && p >= 1 + E && p <= g.n[DIR] + E;
+  // what the last phase reads, on its way while the first two compute
+  if (update) {
+#pragma unroll
+    for (int n = 0; n < NU; n++) prefetch_l2(f.Uc + n * g.ncell + cc);
+  }
+  // ---- reconstruction -------------------------------------------------
+  T vl[NV], vr[NV];
+#pragma unroll
+  for (int n = 0; n < NV; n++) vl[n] = vr[n] = T(0);
+  if constexpr (ORDER == 4) {
+    T w[NV][5];
+    if (valid) {
+#pragma unroll
+      for (int n = 0; n < NV; n++) {
+        if (n == dd::BXn) continue;
+        const int s = n < dd::BXn ? n : n - 1;
+#pragma unroll
+        for (int m = 0; m < 4; m++) w[n][m + 1] = f.Vc[n * g.ncell + cc + (m - 1) * sd];
+        vr[n] = ppm_face(w[n][1], w[n][2], w[n][3], w[n][4]);
+        ss[s * nt + tid] = vr[n];
+      }
+    }
+    __syncthreads();
+    if (valid && t >= 1 && p >= 1) {
+#pragma unroll
+      for (int n = 0; n < NV; n++)
+        if (n != dd::BXn) vl[n] = ss[(n < dd::BXn ? n : n - 1) * nt + tid - cols];
+    }
+    __syncthreads();
+    if (valid) {
+#pragma unroll
+      for (int n = 0; n < NV; n++) {
+        if (n == dd::BXn) continue;
+        w[n][0] = ppm_diff2(w[n][1], w[n][2], w[n][3]);
+        ss[(n < dd::BXn ? n : n - 1) * nt + tid] = w[n][0];
+      }
+    }
+    __syncthreads();
+    if (valid && t >= 1 && p >= 1) {
+#pragma unroll
+      for (int n = 0; n < NV; n++) {
+        if (n == dd::BXn) continue;
+        const T before = ss[(n < dd::BXn ? n : n - 1) * nt + tid - cols];
+        ppm_cell(w[n][1], w[n][2], w[n][3], before, w[n][0], ppm_diff2(w[n][2], w[n][3], w[n][4]), vl[n], vr[n]);
+        if (n == v::RHO || n == v::PRS) Recon<4>::ppm_positive(w[n][1], w[n][2], w[n][3], vl[n], vr[n]);
+      }
+    }
+    __syncthreads();
+    if (valid) {
+#pragma unroll
+      for (int n = 0; n < NV; n++)
+        if (n != dd::BXn) ss[(n < dd::BXn ? n : n - 1) * nt + tid] = vr[n];
+    }
+  } else if (valid) {
+    const Recip l3{g.l3b[DIR], g.l3y[DIR]};
+    const T dxd = g.dx[DIR];
+    const bool shk = f.shock && f.shock[cc];
+#pragma unroll
+    for (int n = 0; n < NV; n++) {
+      if (n == dd::BXn) continue;
+      T w[2 * H + 1];
+#pragma unroll
+      for (int m = 0; m <= 2 * H; m++) w[m] = f.Vc[n * g.ncell + cc + (m - H) * sd];
+      Recon<ORDER>::cell(w, dxd, n == v::RHO || n == v::PRS, vl[n], vr[n], shk, l3);
+      ss[(n < dd::BXn ? n : n - 1) * nt + tid] = vr[n];
+    }
+  }
+  __syncthreads();
+  // ---- the face on the left of the cell -------------------------------
+  const bool face = valid && t >= 1 + E && p >= 1 + E;
+  T FA[NU], cm = T(0);
+#pragma unroll
+  for (int n = 0; n < NU; n++) FA[n] = T(0);
+  if (face) {
+    T vL[NV];
+#pragma unroll
+    for (int n = 0; n < NV; n++)
+      if (n != dd::BXn) vL[n] = ss[(n < dd::BXn ? n : n - 1) * nt + tid - cols];
+    const T bn = f.Vs[DIR * g.nface + fidx(g, idx[2], idx[1], idx[0])];
+    vL[dd::BXn] = bn;
+    vl[dd::BXn] = bn;
+    RiemannOut<D, T> r;
+    riemann<D, DIR, SOLVER>(g.gamma, g.rgm1, vL, vl, r);
+    store_emf<D, DIR>(g, f, cc, r, vL, vl);
+    if (active_col) {
+      const T area = g.A[DIR];
+#pragma unroll
+      for (int n = 0; n < NU; n++) {
+        FA[n] = r.F[n] * area;
+        sf[n * nt + tid] = FA[n];
+      }
+      cm = r.cmax;
+      sf[NU * nt + tid] = cm;
+    }
+  }
+  __syncthreads();
+  // ---- flux difference ------------------------------------------------
+  double run_max = 0.0;
+  if (update) {
+    const T dtdV = ctl->dtdV;
+#pragma unroll
+    for (int n = 0; n < NU; n++) {
+      const T rhs = -dtdV * (sf[n * nt + tid + cols] - FA[n]);
+      f.Uc[n * g.ncell + cc] = f.Uc[n * g.ncell + cc] + rhs;
+    }
+    if (invdt) {
+      const double prev = (invdt == 1) ? 0.0 : f.InvDt[cc];
+      const double inv = prev + quot(pow2x<-1>(sf[NU * nt + tid + cols] + cm), g.dx[DIR]);
+      f.InvDt[cc] = inv;
+      if (inv > run_max) run_max = inv;  // NaN never compares greater
+    }
+  }
+  // CFL maximum: reduced over the warp, then an atomic only where it raises
+  // the stored maximum (one atomic per warp on one address would queue)
+  if (last_dir && invdt) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      const double w = __shfl_xor_sync(0xffffffffu, run_max, o);
+      if (w > run_max) run_max = w;
+    }
+    unsigned long long* mx = (unsigned long long*)&((Ctl*)ctl)->invdt_max_bits;
+    if ((tid & 31) == 0 && (unsigned long long)__double_as_longlong(run_max) > *(volatile unsigned long long*)mx)
+      atomic_max_pos(mx, run_max);
+  }
+}
+
+template <int D, int DIR, int ORDER, int SOLVER>
+__global__ void __launch_bounds__(kCellThreads, 3)
+    k_sweep_cell(Geo g, Fields f, const Ctl* ctl, int invdt, int last_dir) {
+  extern __shared__ double cell_sm[];
+  d_sweep_cell<D, DIR, ORDER, SOLVER>(g, f, ctl, invdt, last_dir, blockIdx.x, cell_sm);
+}
+
+}  // namespace idfx

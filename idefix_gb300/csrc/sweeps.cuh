@@ -3,6 +3,7 @@
 #pragma once
 #include "engine.hpp"
 #include "ensemble.hpp"
+#include "sweep_cell.cuh"
 #include "sweep_tile.cuh"
 
 namespace idfx {
@@ -31,7 +32,11 @@ void launch_dir(Engine& e, int invdt, int last) {
   const int nseg = (g.n[DIR] + e.seg[DIR] - 1) / e.seg[DIR];
   const long long cols = (long long)(g.n[A] + 2 * g.ext) * (D == 3 ? g.n[B] + 2 * g.ext : 1);
   mark_begin(e, kKSweepX + DIR);
-  if constexpr (DIR == 0 && sizeof(T) == 4 && ORDER <= 4) {
+  if constexpr (sizeof(T) == 8) {
+    const int nt = cell_threads(e.sms, [&](int t) { return cell_tiles(g, DIR, t); });
+    k_sweep_cell<D, DIR, ORDER, SOLVER><<<(unsigned)cell_tiles(g, DIR, nt), nt, cell_smem_bytes(D, nt), e.stream>>>(
+        g, e.f, e.ctl, invdt, last);
+  } else if constexpr (DIR == 0 && sizeof(T) == 4 && ORDER <= 4) {
     // FP32 x sweep: warp chunks along each row (coalesced); staged by bulk
     // copies when rows and arrays are 16-byte aligned
     const unsigned blocks = (unsigned)((cols + kXW - 1) / kXW);
@@ -102,13 +107,31 @@ __global__ void __launch_bounds__(kTM) ke_sweep_march(const EnsBox* boxes, const
   d_sweep_march<D, DIR, ORDER, SOLVER, T>(B.g, B.f, B.ctl, invdt, last, B.seg[DIR], dim3(it.y, it.z, it.w));
 }
 
+template <int D, int DIR, int ORDER, int SOLVER>
+__global__ void __launch_bounds__(kCellThreads, 3)
+    ke_sweep_cell(const EnsBox* boxes, const int4* items, int invdt, int last) {
+  extern __shared__ double ens_cell_sm[];
+  const int4 it = items[blockIdx.x];
+  const EnsBox& B = boxes[it.x];
+  d_sweep_cell<D, DIR, ORDER, SOLVER>(B.g, B.f, B.ctl, invdt, last, (unsigned)it.y, ens_cell_sm);
+}
+
 template <int D, int ORDER, int SOLVER, typename T>
 void launch_ens_dir(EnsEngine& e, int dir, const EnsTable& t, int invdt, int last) {
   if (t.n == 0) return;
-  if (dir == 0) ke_sweep_march<D, 0, ORDER, SOLVER, T><<<t.n, kTM, 0, e.stream>>>(e.d_boxes, t.items, invdt, last);
-  if (dir == 1) ke_sweep_march<D, 1, ORDER, SOLVER, T><<<t.n, kTM, 0, e.stream>>>(e.d_boxes, t.items, invdt, last);
-  if constexpr (D == 3)
-    if (dir == 2) ke_sweep_march<D, 2, ORDER, SOLVER, T><<<t.n, kTM, 0, e.stream>>>(e.d_boxes, t.items, invdt, last);
+  if constexpr (sizeof(T) == 8) {
+    const int nt = e.cell_nt[dir];
+    const size_t sm = cell_smem_bytes(D, nt);
+    if (dir == 0) ke_sweep_cell<D, 0, ORDER, SOLVER><<<t.n, nt, sm, e.stream>>>(e.d_boxes, t.items, invdt, last);
+    if (dir == 1) ke_sweep_cell<D, 1, ORDER, SOLVER><<<t.n, nt, sm, e.stream>>>(e.d_boxes, t.items, invdt, last);
+    if constexpr (D == 3)
+      if (dir == 2) ke_sweep_cell<D, 2, ORDER, SOLVER><<<t.n, nt, sm, e.stream>>>(e.d_boxes, t.items, invdt, last);
+  } else {
+    if (dir == 0) ke_sweep_march<D, 0, ORDER, SOLVER, T><<<t.n, kTM, 0, e.stream>>>(e.d_boxes, t.items, invdt, last);
+    if (dir == 1) ke_sweep_march<D, 1, ORDER, SOLVER, T><<<t.n, kTM, 0, e.stream>>>(e.d_boxes, t.items, invdt, last);
+    if constexpr (D == 3)
+      if (dir == 2) ke_sweep_march<D, 2, ORDER, SOLVER, T><<<t.n, kTM, 0, e.stream>>>(e.d_boxes, t.items, invdt, last);
+  }
 }
 
 template <int SOLVER>
@@ -184,8 +207,10 @@ __device__ __forceinline__ bool any_due(const EnsBox* boxes, int nbox, int perio
 }
 
 template <int D, int ORDER, int SOLVER, typename T>
-__global__ void __launch_bounds__(kTM) ke_persistent(const EnsBox* boxes, EnsPersist P, int ncyc, GridBar* bar) {
+__global__ void __launch_bounds__(kTM, sizeof(T) == 8 ? 6 : 1)
+    ke_persistent(const EnsBox* boxes, EnsPersist P, int ncyc, GridBar* bar) {
   using E = T;  // EMF buffers in the arithmetic type of the sweeps
+  __shared__ double cell_sm[sizeof(T) == 8 ? cell_smem_bytes(D, kTM) / sizeof(double) : 1];
   const int stride = (int)gridDim.x;
   const int tstride = stride * (int)blockDim.x;
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
@@ -239,10 +264,18 @@ __global__ void __launch_bounds__(kTM) ke_persistent(const EnsBox* boxes, EnsPer
         for (int i = blockIdx.x; i < P.nsweep[d]; i += stride) {
           const int4 it = P.sweep[d][i];
           const EnsBox& B = boxes[it.x];
-          if (d == 0) d_sweep_march<D, 0, ORDER, SOLVER, T>(B.g, B.f, B.ctl, invdt, last, B.seg[0], dd(it));
-          if (d == 1) d_sweep_march<D, 1, ORDER, SOLVER, T>(B.g, B.f, B.ctl, invdt, last, B.seg[1], dd(it));
-          if constexpr (D == 3)
-            if (d == 2) d_sweep_march<D, 2, ORDER, SOLVER, T>(B.g, B.f, B.ctl, invdt, last, B.seg[2], dd(it));
+          if constexpr (sizeof(T) == 8) {
+            if (d == 0) d_sweep_cell<D, 0, ORDER, SOLVER>(B.g, B.f, B.ctl, invdt, last, (unsigned)it.y, cell_sm);
+            if (d == 1) d_sweep_cell<D, 1, ORDER, SOLVER>(B.g, B.f, B.ctl, invdt, last, (unsigned)it.y, cell_sm);
+            if constexpr (D == 3)
+              if (d == 2) d_sweep_cell<D, 2, ORDER, SOLVER>(B.g, B.f, B.ctl, invdt, last, (unsigned)it.y, cell_sm);
+            __syncthreads();  // the next item's states go where this one's were read
+          } else {
+            if (d == 0) d_sweep_march<D, 0, ORDER, SOLVER, T>(B.g, B.f, B.ctl, invdt, last, B.seg[0], dd(it));
+            if (d == 1) d_sweep_march<D, 1, ORDER, SOLVER, T>(B.g, B.f, B.ctl, invdt, last, B.seg[1], dd(it));
+            if constexpr (D == 3)
+              if (d == 2) d_sweep_march<D, 2, ORDER, SOLVER, T>(B.g, B.f, B.ctl, invdt, last, B.seg[2], dd(it));
+          }
         }
         ok = grid_barrier(bar);
       }
