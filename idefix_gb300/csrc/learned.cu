@@ -1,6 +1,5 @@
-// Learned interface-state correction (see learned.cuh): BF16 training
-// kernels on the 5th-generation tensor cores (forward, backward; Adam), the
-// training-data kernels (coarsening of fine snapshots, batch assembly) and
+// Learned interface-state correction (see learned.cuh): the trainer around
+// the training kernels (train_tile.cuh), the coarsening of fine snapshots and
 // the learned sweep of the ORDER 5 solver (network inference fused with the
 // reconstruction, the Riemann solve and the flux difference), with their C
 // ABI.
@@ -17,277 +16,13 @@
 #include "../../include/idefix_gb300.h"
 #include "engine.hpp"
 #include "learned.cuh"
+#include "train_tile.cuh"
 #include "umma.cuh"
 
 using namespace idfx;
 using namespace idfx::learn;
 
 namespace {
-
-// ---------------------------------------------------------------------------
-// BF16 GEMM of the training on the 5th-generation tensor cores:
-// C[M][N] = op(A)[M][K] . op(B)[K][N], FP32 accumulation in tensor memory.
-// A(m,k) = transA ? A[k*lda + m] : A[m*lda + k]
-// B(k,n) = transB ? B[n*ldb + k] : B[k*ldb + n]
-// CTA tile 128 x N (N <= 128, a multiple of 16); K in chunks of 64 staged
-// in the canonical K-major layout by all threads, two stages (the next chunk
-// is staged while the tensor core works on the current one); one thread
-// issues the MMAs and commits them to the stage's mbarrier; the epilogue
-// reads each row from tensor memory (thread = row).
-// ---------------------------------------------------------------------------
-enum Epi { kEpiF32 = 0, kEpiBiasSilu = 1, kEpiBias = 2, kEpiDsilu = 3 };
-
-struct EpiArgs {
-  int mode;
-  const float* bias;   // [N]           (kEpiBiasSilu, kEpiBias)
-  const float* zin;    // [M][ldo]      (kEpiDsilu: pre-activation)
-  float* out_f;        // [M][ldo]      FP32 result (Z, Y, dW, dZ)
-  __nv_bfloat16* out_b;  // [M][ldo]    BF16 result (H = silu(Z), dZ)
-  int ldo;
-};
-
-constexpr int GT_M = 128, GT_N = 128, GT_KC = 64;
-
-// One operand chunk (R rows x GT_KC columns of k) into the canonical K-major
-// layout, zero outside rows < Rmax and k < K.  kcontig: element (r, k) at
-// src[r * ld + k] - eight consecutive k are one 16-byte load and one 16-byte
-// core-matrix row in shared memory; else at src[k * ld + r] - eight
-// consecutive rows are one 16-byte load, scattered over a core matrix's rows.
-// Vector loads where ld and the base allow them (ld a multiple of 8, base
-// 16-byte aligned; chunk and tile origins are multiples of 8).
-__device__ __forceinline__ void stage_tile(__nv_bfloat16* dst, const __nv_bfloat16* __restrict__ src, int ld,
-                                           bool kcontig, int r0, int Rmax, int k0, int K, int R) {
-  const bool vec = (ld & 7) == 0 && (reinterpret_cast<uintptr_t>(src) & 15) == 0;
-  const __nv_bfloat16 zero = __float2bfloat16(0.f);
-  if (kcontig) {
-    for (int e = threadIdx.x; e < R * (GT_KC / 8); e += blockDim.x) {
-      const int r = e / (GT_KC / 8), kv = (e % (GT_KC / 8)) * 8;
-      const int gr = r0 + r, gk = k0 + kv;
-      alignas(16) __nv_bfloat16 t[8];
-      if (gr < Rmax && vec && gk + 8 <= K) {
-        *reinterpret_cast<uint4*>(t) = *reinterpret_cast<const uint4*>(src + (long long)gr * ld + gk);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 8; i++) t[i] = (gr < Rmax && gk + i < K) ? src[(long long)gr * ld + gk + i] : zero;
-      }
-      *reinterpret_cast<uint4*>(dst + umma::kmajor_offset(r, kv, GT_KC) / 2) = *reinterpret_cast<const uint4*>(t);
-    }
-  } else {
-    const int rg = R / 8;  // groups of eight rows; consecutive threads take consecutive groups
-    for (int e = threadIdx.x; e < rg * GT_KC; e += blockDim.x) {
-      const int rv = (e % rg) * 8, k = e / rg;
-      const int gr = r0 + rv, gk = k0 + k;
-      alignas(16) __nv_bfloat16 t[8];
-      if (gk < K && vec && gr + 8 <= Rmax) {
-        *reinterpret_cast<uint4*>(t) = *reinterpret_cast<const uint4*>(src + (long long)gk * ld + gr);
-      } else {
-#pragma unroll
-        for (int i = 0; i < 8; i++) t[i] = (gk < K && gr + i < Rmax) ? src[(long long)gk * ld + gr + i] : zero;
-      }
-#pragma unroll
-      for (int i = 0; i < 8; i++) dst[umma::kmajor_offset(rv + i, k, GT_KC) / 2] = t[i];
-    }
-  }
-}
-constexpr size_t GT_A = (size_t)GT_M * GT_KC * 2, GT_B = (size_t)GT_N * GT_KC * 2;
-constexpr size_t GT_STAGE = GT_A + GT_B;
-constexpr size_t GT_SMEM = 2 * GT_STAGE + 64;
-
-__global__ void __launch_bounds__(128, 1) k_gemm_tc(int M, int N, int K, const __nv_bfloat16* __restrict__ A,
-                                                    int lda, int transA, const __nv_bfloat16* __restrict__ B,
-                                                    int ldb, int transB, EpiArgs ep, int* status, int cps,
-                                                    float* __restrict__ part) {
-  extern __shared__ __align__(128) unsigned char sm[];
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + 2 * GT_STAGE);
-  uint32_t* slot = reinterpret_cast<uint32_t*>(bar + 2);
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int m0 = blockIdx.y * GT_M, n0 = blockIdx.x * GT_N;
-  const int nt = min(GT_N, N - n0);  // a multiple of 16
-  uint32_t ncols = 32;
-  while ((int)ncols < nt) ncols <<= 1;
-  if (warp == 0) umma::tmem_alloc(slot, ncols);
-  if (tid == 0) {
-    umma::mbar_init1(bar);
-    umma::mbar_init1(bar + 1);
-  }
-  umma::fence_before_sync();
-  __syncthreads();
-  umma::fence_after_sync();
-  const uint32_t taddr = *slot;
-  const uint32_t idesc = umma::idesc_bf16_f32(GT_M, nt);
-  // split K (blockIdx.z): this CTA's chunks of GT_KC start at q0
-  const int nq_all = (K + GT_KC - 1) / GT_KC;
-  const int q0 = blockIdx.z * cps;
-  const int nq = min(cps, nq_all - q0);
-  bool ok = true;
-  for (int q = 0; q < nq; q++) {
-    const int st = q & 1;
-    if (q >= 2) {  // stage st is free once the MMAs of chunk q - 2 have landed
-      const bool w = umma::mbar_wait_bounded(bar + st, (uint32_t)(((q - 2) >> 1) & 1), umma::kMmaSpin);
-      ok = __syncthreads_and(w);
-      if (!ok) break;
-    }
-    __nv_bfloat16* As = reinterpret_cast<__nv_bfloat16*>(sm + st * GT_STAGE);
-    __nv_bfloat16* Bs = reinterpret_cast<__nv_bfloat16*>(sm + st * GT_STAGE + GT_A);
-    const int k0 = (q0 + q) * GT_KC;
-    // A(m, k): k contiguous in memory unless transposed; B(k, n) as the
-    // N x K operand: k contiguous when transposed
-    stage_tile(As, A, lda, !transA, m0, M, k0, K, GT_M);
-    stage_tile(Bs, B, ldb, transB != 0, n0, N, k0, K, nt);
-    umma::fence_async_smem();
-    __syncthreads();
-    if (tid == 0) {
-      umma::fence_after_sync();
-      umma::mma_tile(taddr, umma::smem_addr(As), umma::smem_addr(Bs), GT_KC, idesc, q > 0);
-      umma::mma_commit(bar + st);
-    }
-  }
-  if (ok) {  // the last commit lands after every MMA issued before it
-    const int q = nq - 1;
-    const bool w = umma::mbar_wait_bounded(bar + (q & 1), (uint32_t)((q >> 1) & 1), umma::kMmaSpin);
-    ok = __syncthreads_and(w);
-  }
-  umma::fence_after_sync();
-  if (ok) {
-    const int m = m0 + 32 * warp + lane;
-    for (int c = 0; c < nt; c += 16) {
-      float v[16];
-      umma::tmem_ld16(taddr + ((uint32_t)(32 * warp) << 16) + (uint32_t)c, v);
-      if (m >= M) continue;
-#pragma unroll
-      for (int i = 0; i < 16; i++) {
-        const int n = n0 + c + i;
-        if (n >= N) continue;
-        const long long o = (long long)m * ep.ldo + n;
-        float x = v[i];
-        if (part) {  // split K: this split's partial product, summed by k_splitk_sum
-          part[((long long)blockIdx.z * M + m) * N + n] = x;
-          continue;
-        }
-        switch (ep.mode) {
-          case kEpiF32:
-            ep.out_f[o] = x;
-            break;
-          case kEpiBiasSilu:
-            x += ep.bias[n];
-            ep.out_f[o] = x;
-            ep.out_b[o] = __float2bfloat16(silu_f(x));
-            break;
-          case kEpiBias:
-            ep.out_f[o] = x + ep.bias[n];
-            break;
-          default:  // kEpiDsilu
-            x *= dsilu_f(ep.zin[o]);
-            ep.out_f[o] = x;
-            ep.out_b[o] = __float2bfloat16(x);
-            break;
-        }
-      }
-    }
-  } else if (tid == 0) {
-    atomicExch(status, 1);
-  }
-  umma::fence_before_sync();
-  __syncthreads();
-  if (warp == 0) umma::tmem_dealloc(taddr, ncols);
-}
-
-// out = sum over the S partial products, in split order (deterministic)
-__global__ void k_splitk_sum(const float* __restrict__ part, int S, int M, int N, float* __restrict__ out, int ldo) {
-  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= (long long)M * N) return;
-  float acc = 0.f;
-  for (int z = 0; z < S; z++) acc += part[(long long)z * M * N + e];
-  out[(e / N) * ldo + e % N] = acc;
-}
-
-constexpr int GT_MAX_SPLITS = 64;
-// split-K workspace of a trainer: GT_MAX_SPLITS partial products of up to
-// 256 x 128
-constexpr size_t GT_WS_FLOATS = (size_t)GT_MAX_SPLITS * 256 * 128;
-
-// N a multiple of 16 (every use: NH, NOUT); status: set when a bounded wait
-// of the tensor-core pipeline gave up.  A product with few output tiles and
-// a long K (the weight gradients: K = the batch) is split over K into up to
-// GT_MAX_SPLITS CTAs per tile, the partial products summed in split order
-// by a second kernel (ws: GT_WS_FLOATS floats).
-void gemm(cudaStream_t s, int M, int N, int K, const __nv_bfloat16* A, int lda, int transA, const __nv_bfloat16* B,
-          int ldb, int transB, const EpiArgs& ep, int* status, float* ws) {
-  dim3 grid((N + GT_N - 1) / GT_N, (M + GT_M - 1) / GT_M, 1);
-  const int nq = (K + GT_KC - 1) / GT_KC;
-  const int tiles = (int)(grid.x * grid.y);
-  int cps = nq;
-  if (ws && ep.mode == kEpiF32 && tiles < 64 && nq >= 4 && (size_t)M * N <= 256 * 128) {
-    int splits = std::min(std::min(GT_MAX_SPLITS, (128 + tiles - 1) / tiles), nq / 2);
-    cps = (nq + splits - 1) / splits;
-    grid.z = (unsigned)((nq + cps - 1) / cps);
-  }
-  float* part = grid.z > 1 ? ws : nullptr;
-  k_gemm_tc<<<grid, 128, GT_SMEM, s>>>(M, N, K, A, lda, transA, B, ldb, transB, ep, status, cps, part);
-  if (part) {
-    const long long mn = (long long)M * N;
-    k_splitk_sum<<<(unsigned)((mn + 255) / 256), 256, 0, s>>>(part, (int)grid.z, M, N, ep.out_f, ep.ldo);
-  }
-}
-
-// column sums (bias gradients): out[n] = sum_m in[m][n]
-__global__ void k_colsum(const float* __restrict__ in, int M, int N, float* __restrict__ out) {
-  const int n = blockIdx.x;
-  float s = 0.f;
-  for (int m = threadIdx.x; m < M; m += blockDim.x) s += in[(long long)m * N + n];
-  __shared__ float red[256];
-  red[threadIdx.x] = s;
-  __syncthreads();
-  for (int w = blockDim.x / 2; w > 0; w >>= 1) {
-    if ((int)threadIdx.x < w) red[threadIdx.x] += red[threadIdx.x + w];
-    __syncthreads();
-  }
-  if (threadIdx.x == 0) out[n] = red[0];
-}
-
-// masked squared error: dY = 2 (Y - T) / B (BF16 and FP32), loss += sum (Y - T)^2 / B
-__global__ void k_loss(const float* __restrict__ Y, const float* __restrict__ T, int B, float* __restrict__ dYf,
-                       __nv_bfloat16* __restrict__ dYb, double* __restrict__ loss) {
-  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  double l = 0.0;
-  if (e < (long long)B * NOUT) {
-    const int o = (int)(e % NOUT);
-    const float r = loss_masked(o) ? 0.f : Y[e] - T[e];
-    const float d = 2.f * r / (float)B;
-    dYf[e] = d;
-    dYb[e] = __float2bfloat16(d);
-    l = (double)r * r / B;
-  }
-  for (int w = 16; w > 0; w >>= 1) l += __shfl_down_sync(0xffffffffu, l, w);
-  if ((threadIdx.x & 31) == 0 && l != 0.0) atomicAdd(loss, l);
-}
-
-// Adam step over the packed FP32 parameters; refreshes the BF16 weights
-// (W1b has K1 rows, the last K1 - NIN stay zero)
-__global__ void k_adam(float* __restrict__ w, float* __restrict__ m, float* __restrict__ v, const float* __restrict__ g,
-                       float lr, float b1, float b2, float eps, float bc1, float bc2, __nv_bfloat16* __restrict__ W1b,
-                       __nv_bfloat16* __restrict__ W2b, __nv_bfloat16* __restrict__ W3b) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p >= NPARAM) return;
-  const float gp = g[p];
-  const float mp = b1 * m[p] + (1.f - b1) * gp;
-  const float vp = b2 * v[p] + (1.f - b2) * gp * gp;
-  m[p] = mp;
-  v[p] = vp;
-  const float wp = w[p] - lr * (mp / bc1) / (sqrtf(vp / bc2) + eps);
-  w[p] = wp;
-  if (p < OB1) W1b[p - OW1] = __float2bfloat16(wp);
-  else if (p >= OW2 && p < OB2) W2b[p - OW2] = __float2bfloat16(wp);
-  else if (p >= OW3 && p < OB3) W3b[p - OW3] = __float2bfloat16(wp);
-}
-
-__global__ void k_refresh_bf16(const float* __restrict__ w, __nv_bfloat16* __restrict__ W1b,
-                               __nv_bfloat16* __restrict__ W2b, __nv_bfloat16* __restrict__ W3b) {
-  const int p = blockIdx.x * blockDim.x + threadIdx.x;
-  if (p < K1 * NH) W1b[p] = __float2bfloat16(p < NIN * NH ? w[OW1 + p] : 0.f);
-  if (p < NH * NH) W2b[p] = __float2bfloat16(w[OW2 + p]);
-  if (p < NH * NOUT) W3b[p] = __float2bfloat16(w[OW3 + p]);
-}
 
 // ---------------------------------------------------------------------------
 // Coarsening of a fine snapshot (ghosted reference layout, 3-D, periodic):
@@ -381,85 +116,6 @@ __global__ void k_coarsen(const double* __restrict__ Vc, const double* __restric
     }
 }
 
-// order-preserving map of floats to unsigned keys (atomic min / max)
-__device__ __forceinline__ unsigned fkey(float f) {
-  const unsigned b = __float_as_uint(f);
-  return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
-}
-__host__ __device__ inline float fkey_inv(unsigned k) {
-  const unsigned b = (k & 0x80000000u) ? (k & 0x7fffffffu) : ~k;
-  float f;
-  memcpy(&f, &b, sizeof(f));
-  return f;
-}
-
-__device__ __forceinline__ unsigned long long mix64(unsigned long long z) {  // splitmix64 finaliser
-  z += 0x9e3779b97f4a7c15ull;
-  z = (z ^ (z >> 30)) * 0xbf58476d1ce4e5b9ull;
-  z = (z ^ (z >> 27)) * 0x94d049bb133111ebull;
-  return z ^ (z >> 31);
-}
-
-__device__ __forceinline__ float vanleer_f(float dvp, float dvm) {
-  return dvp * dvm > 0.f ? 2.f * dvp * dvm / (dvp + dvm) : 0.f;
-}
-
-// Batch assembly: sample i of the batch picks (snapshot, cell, direction)
-// from a counter-based hash; X = BF16 stencil features (K1 columns, the last
-// zero), T = normalised correction targets.  Optionally widens the trained
-// feature range.  prims/tgt: FP32 [S][8][nc^3] and [S][3][16][nc^3].
-__global__ void k_make_batch(const float* __restrict__ prims, const float* __restrict__ tgt, int S, int nc,
-                             float gamma, unsigned long long seed, long long base, int B,
-                             __nv_bfloat16* __restrict__ X, float* __restrict__ T, unsigned* __restrict__ kmin,
-                             unsigned* __restrict__ kmax) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= B) return;
-  const long long ncell = (long long)nc * nc * nc;
-  const unsigned long long h = mix64(seed ^ mix64((unsigned long long)(base + i)));
-  const int snap = (int)(h % (unsigned long long)S);
-  const long long cell = (long long)((h >> 16) % (unsigned long long)ncell);
-  const int d = (int)((h >> 48) % 3ull);
-  const float* P = prims + (long long)snap * 8 * ncell;
-  const int cx[3] = {(int)(cell % nc), (int)((cell / nc) % nc), (int)(cell / ((long long)nc * nc))};
-  auto at = [&](int rv, int o0, int o1, int o2) {
-    int q[3] = {cx[0], cx[1], cx[2]};
-    q[d] = (q[d] + o0 + nc) % nc;
-    q[(d + 1) % 3] = (q[(d + 1) % 3] + o1 + nc) % nc;
-    q[(d + 2) % 3] = (q[(d + 2) % 3] + o2 + nc) % nc;
-    return P[rot_var(rv, d) * ncell + ((long long)q[2] * nc + q[1]) * nc + q[0]];
-  };
-  float cen[8];
-  for (int rv = 0; rv < 8; rv++) cen[rv] = at(rv, 0, 0, 0);
-  const float rho_c = cen[0], p_c = cen[4];
-  const float cs = sqrtf(gamma * p_c / rho_c), sb = sqrtf(rho_c) * cs;
-  const float sc[8] = {rho_c, cs, cs, cs, p_c, sb, sb, sb};
-  __nv_bfloat16* xr = X + (long long)i * K1;
-  for (int rv = 0; rv < 8; rv++)
-    for (int o2 = -1; o2 <= 1; o2++)
-      for (int o1 = -1; o1 <= 1; o1++)
-        for (int o0 = -1; o0 <= 1; o0++) {
-          const float s = at(rv, o0, o1, o2);
-          float f;
-          if (rv == 0 || rv == 4) f = s / cen[rv] - 1.f;
-          else if (rv < 4) f = (s - cen[rv]) / cs;
-          else f = s / sb;
-          const int col = rv * 27 + (o2 + 1) * 9 + (o1 + 1) * 3 + (o0 + 1);
-          xr[col] = __float2bfloat16(f);
-          if (kmin) {
-            atomicMin(kmin + col, fkey(f));
-            atomicMax(kmax + col, fkey(f));
-          }
-        }
-  for (int col = NIN; col < K1; col++) xr[col] = __float2bfloat16(0.f);
-  const float* tg = tgt + ((long long)snap * 3 + d) * 16 * ncell + cell;
-  for (int rv = 0; rv < 8; rv++) {
-    const float w0 = at(rv, -1, 0, 0), w1 = cen[rv], w2 = at(rv, 1, 0, 0);
-    const float dd = vanleer_f(w2 - w1, w1 - w0);
-    T[(long long)i * NOUT + rv] = (tg[rv * ncell] - (w1 - 0.5f * dd)) / sc[rv];
-    T[(long long)i * NOUT + 8 + rv] = (tg[(8 + rv) * ncell] - (w1 + 0.5f * dd)) / sc[rv];
-  }
-}
-
 // ---------------------------------------------------------------------------
 // Learned sweep (ORDER 5): reconstruction with the network's correction,
 // Riemann solve and flux difference of one direction in one kernel, over
@@ -506,10 +162,12 @@ static_assert(LX_CM + (size_t)LT * 8 <= (size_t)LT * K1 * 2, "tile outputs excee
 static_assert(LS_X % 128 == 0 && LS_H % 128 == 0 && LS_W2 % 128 == 0 && LS_W3 % 128 == 0, "operand alignment");
 static_assert(SM_LEARN <= 227 * 1024, "learned sweep does not fit in shared memory");
 
+static_assert(LS_W2 - LS_W1 == (size_t)(PW2 - PW1) * 2 && LS_W3 - LS_W1 == (size_t)(PW3 - PW1) * 2 &&
+                  LS_X - LS_W1 == (size_t)NPACK * 2,
+              "the packed weights as they lie");
+
 struct LearnedDev {
-  const __nv_bfloat16* W1b;  // [K1][NH]
-  const __nv_bfloat16* W2b;  // [NH][NH]
-  const __nv_bfloat16* W3b;  // [NH][NOUT]
+  const __nv_bfloat16* Wp;   // packed weights
   const float* w;            // packed FP32 parameters (biases)
   const float* fmin;         // [NIN] trained feature range, or null
   const float* fmax;
@@ -573,19 +231,9 @@ __global__ void __launch_bounds__(256, 1) k_learned_sweep(Geo g, Fields f, Learn
   double* FA = reinterpret_cast<double*>(Xs + LX_FA);
   double* CM = reinterpret_cast<double*>(Xs + LX_CM);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // weights as the B operands (N x K, K-major): element (n, k) of layer l
-  for (int e = tid; e < K1 * NH; e += blockDim.x) {
-    const int k = e / NH, n = e % NH;
-    reinterpret_cast<__nv_bfloat16*>(W1s)[umma::kmajor_offset(n, k, K1) / 2] = L.W1b[e];
-  }
-  for (int e = tid; e < NH * NH; e += blockDim.x) {
-    const int k = e / NH, n = e % NH;
-    reinterpret_cast<__nv_bfloat16*>(W2s)[umma::kmajor_offset(n, k, NH) / 2] = L.W2b[e];
-  }
-  for (int e = tid; e < NH * NOUT; e += blockDim.x) {
-    const int k = e / NOUT, n = e % NOUT;
-    reinterpret_cast<__nv_bfloat16*>(W3s)[umma::kmajor_offset(n, k, NH) / 2] = L.W3b[e];
-  }
+  // weights as the B operands (N x K, K-major)
+  for (int e = tid; e < NPACK / 8; e += blockDim.x)
+    reinterpret_cast<uint4*>(W1s)[e] = reinterpret_cast<const uint4*>(L.Wp)[e];
   for (int e = tid; e < NH; e += blockDim.x) {
     bs[e] = L.w[OB1 + e];
     bs[NH + e] = L.w[OB2 + e];
@@ -819,14 +467,6 @@ __global__ void __launch_bounds__(256, 1) k_learned_sweep(Geo g, Fields f, Learn
   if (warp == 0) umma::tmem_dealloc(tmem, 256);
 }
 
-__global__ void k_sumsq_targets(const float* __restrict__ T, int B, double* __restrict__ out) {
-  const long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  double l = 0.0;
-  if (e < (long long)B * NOUT && !loss_masked((int)(e % NOUT))) l = (double)T[e] * T[e] / B;
-  for (int w = 16; w > 0; w >>= 1) l += __shfl_down_sync(0xffffffffu, l, w);
-  if ((threadIdx.x & 31) == 0 && l != 0.0) atomicAdd(out, l);
-}
-
 __global__ void k_init_keys(unsigned* kmin, unsigned* kmax) {
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i < NIN) {
@@ -889,7 +529,7 @@ __global__ void __launch_bounds__(128, 1) k_umma_check(int N, int K, const __nv_
 
 // the network as the engine holds it (ORDER 5)
 struct LearnedModel {
-  __nv_bfloat16 *W1b = nullptr, *W2b = nullptr, *W3b = nullptr;
+  __nv_bfloat16* Wp = nullptr;
   float* w = nullptr;
   float *fmin = nullptr, *fmax = nullptr;
   unsigned long long* counters = nullptr;
@@ -904,7 +544,7 @@ namespace idfx {
 // k_learned_sweep)
 static void launch_learned(Engine& e, int invdt, int fold_max, double* states) {
   LearnedModel* m = static_cast<LearnedModel*>(e.learned);
-  LearnedDev L{m->W1b, m->W2b, m->W3b, m->w, m->ranged ? m->fmin : nullptr, m->ranged ? m->fmax : nullptr};
+  LearnedDev L{m->Wp, m->w, m->ranged ? m->fmin : nullptr, m->ranged ? m->fmax : nullptr};
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
@@ -927,9 +567,7 @@ void launch_learned_sweeps(Engine& e, int invdt, int fold_max) { launch_learned(
 void free_learned(Engine& e) {
   LearnedModel* m = static_cast<LearnedModel*>(e.learned);
   if (!m) return;
-  cudaFree(m->W1b);
-  cudaFree(m->W2b);
-  cudaFree(m->W3b);
+  cudaFree(m->Wp);
   cudaFree(m->w);
   cudaFree(m->fmin);
   cudaFree(m->fmax);
@@ -947,13 +585,14 @@ struct idfx_mlp {
   int max_batch = 0;
   long long t = 0;  // Adam steps taken
   float *w = nullptr, *m = nullptr, *v = nullptr, *g = nullptr;
-  __nv_bfloat16 *W1b = nullptr, *W2b = nullptr, *W3b = nullptr;
-  __nv_bfloat16 *X = nullptr, *H1 = nullptr, *H2 = nullptr, *dYb = nullptr, *dZ2b = nullptr, *dZ1b = nullptr;
-  float *T = nullptr, *Z1 = nullptr, *Z2 = nullptr, *Y = nullptr, *dYf = nullptr, *dZ2f = nullptr, *dZ1f = nullptr;
+  __nv_bfloat16* Wp = nullptr;  // packed BF16 weights
+  Tile* tiles[2] = {nullptr, nullptr};  // assembled batches: the step's and the next one's
+  float* part = nullptr;        // weight gradients of every block of a batch
+  float* cols = nullptr;        // dZ1, dZ2, dY of every sample, by column
+  double* ploss = nullptr;      // losses of every block
   double* loss = nullptr;
   unsigned *kmin = nullptr, *kmax = nullptr;
-  int* status = nullptr;  // set by a GEMM whose bounded tensor-core wait gave up
-  float* ws = nullptr;    // split-K partial products of the weight-gradient GEMMs
+  int* status = nullptr;  // set by a block whose bounded wait gave up
   const float* prims = nullptr;
   const float* tgt = nullptr;
   int nsnap = 0, nc = 0;
@@ -970,22 +609,40 @@ bool dalloc(idfx_mlp* h, P** p, size_t n) {
   return cudaMemsetAsync(*p, 0, n * sizeof(P), h->stream) == cudaSuccess;
 }
 
-// forward + loss + backward of one batch held in h->X / h->T (loss added to *loss)
-void fwd_bwd(idfx_mlp* h, int B, double* loss) {
-  cudaStream_t s = h->stream;
-  gemm(s, B, NH, K1, h->X, K1, 0, h->W1b, NH, 0, EpiArgs{kEpiBiasSilu, h->w + OB1, nullptr, h->Z1, h->H1, NH}, h->status, h->ws);
-  gemm(s, B, NH, NH, h->H1, NH, 0, h->W2b, NH, 0, EpiArgs{kEpiBiasSilu, h->w + OB2, nullptr, h->Z2, h->H2, NH}, h->status, h->ws);
-  gemm(s, B, NOUT, NH, h->H2, NH, 0, h->W3b, NOUT, 0, EpiArgs{kEpiBias, h->w + OB3, nullptr, h->Y, nullptr, NOUT}, h->status, h->ws);
-  const int ne = B * NOUT;
-  k_loss<<<(ne + 255) / 256, 256, 0, s>>>(h->Y, h->T, B, h->dYf, h->dYb, loss);
-  gemm(s, NH, NOUT, B, h->H2, NH, 1, h->dYb, NOUT, 0, EpiArgs{kEpiF32, nullptr, nullptr, h->g + OW3, nullptr, NOUT}, h->status, h->ws);
-  k_colsum<<<NOUT, 256, 0, s>>>(h->dYf, B, NOUT, h->g + OB3);
-  gemm(s, B, NH, NOUT, h->dYb, NOUT, 0, h->W3b, NOUT, 1, EpiArgs{kEpiDsilu, nullptr, h->Z2, h->dZ2f, h->dZ2b, NH}, h->status, h->ws);
-  gemm(s, NH, NH, B, h->H1, NH, 1, h->dZ2b, NH, 0, EpiArgs{kEpiF32, nullptr, nullptr, h->g + OW2, nullptr, NH}, h->status, h->ws);
-  k_colsum<<<NH, 256, 0, s>>>(h->dZ2f, B, NH, h->g + OB2);
-  gemm(s, B, NH, NH, h->dZ2b, NH, 0, h->W2b, NH, 1, EpiArgs{kEpiDsilu, nullptr, h->Z1, h->dZ1f, h->dZ1b, NH}, h->status, h->ws);
-  gemm(s, NIN, NH, B, h->X, K1, 1, h->dZ1b, NH, 0, EpiArgs{kEpiF32, nullptr, nullptr, h->g + OW1, nullptr, NH}, h->status, h->ws);
-  k_colsum<<<NH, 256, 0, s>>>(h->dZ1f, B, NH, h->g + OB1);
+Dataset dataset(const idfx_mlp* h) { return Dataset{h->prims, h->tgt, h->nsnap, h->nc, (float)h->gamma}; }
+
+// the blocks of a launch: those that put a batch through the network
+// (compute) and those that assemble one into the trainer's tiles
+TrainArgs batch_args(const idfx_mlp* h, int B) {
+  TrainArgs a{};
+  a.B = B;
+  a.split = split_batch(B);
+  a.cols = h->cols;
+  a.ld = h->max_batch;
+  a.Wp = h->Wp;
+  a.w = h->w;
+  a.status = h->status;
+  a.D = dataset(h);
+  return a;
+}
+void launch_tiles(idfx_mlp* h, const TrainArgs& a) {
+  const unsigned n = (unsigned)(a.compute + (a.next ? a.split.blocks * a.split.tiles : 0));
+  k_train_tile<<<n, TT, SM_TRAIN, h->stream>>>(a);
+}
+// samples base .. base + B - 1 of a seed into the tiles of `slot`
+void launch_assemble(idfx_mlp* h, int B, unsigned long long seed, long long base, int slot, bool range) {
+  TrainArgs a = batch_args(h, B);
+  a.seed = seed;
+  a.base = base;
+  a.next = h->tiles[slot];
+  a.kmin = range ? h->kmin : nullptr;
+  a.kmax = range ? h->kmax : nullptr;
+  launch_tiles(h, a);
+}
+// the blocks' gradients and losses summed, and the Adam step where adam.w is set
+void launch_update(idfx_mlp* h, int B, bool grad, const AdamArgs& adam, double* loss) {
+  k_train_update<<<grad ? UPDATE_BLOCKS : 1, 256, 0, h->stream>>>(grad ? h->part : nullptr, h->cols, h->max_batch,
+                                                                 split_batch(B).blocks, h->g, adam, h->ploss, B, loss);
 }
 
 int sync_ok(idfx_mlp* h) {
@@ -1014,9 +671,7 @@ int idfx_gpu_set_learned(idfx_gpu* hg, const float* params, const float* fmin, c
     LearnedModel* m = new (std::nothrow) LearnedModel();
     if (!m) return IDFX_ERR_STATE;
     e.learned = m;
-    bool ok = cudaMalloc(&m->W1b, sizeof(__nv_bfloat16) * K1 * NH) == cudaSuccess;
-    ok = ok && cudaMalloc(&m->W2b, sizeof(__nv_bfloat16) * NH * NH) == cudaSuccess;
-    ok = ok && cudaMalloc(&m->W3b, sizeof(__nv_bfloat16) * NH * NOUT) == cudaSuccess;
+    bool ok = cudaMalloc(&m->Wp, sizeof(__nv_bfloat16) * NPACK) == cudaSuccess;
     ok = ok && cudaMalloc(&m->w, sizeof(float) * NPARAM) == cudaSuccess;
     ok = ok && cudaMalloc(&m->fmin, sizeof(float) * NIN) == cudaSuccess;
     ok = ok && cudaMalloc(&m->fmax, sizeof(float) * NIN) == cudaSuccess;
@@ -1042,7 +697,7 @@ int idfx_gpu_set_learned(idfx_gpu* hg, const float* params, const float* fmin, c
   }
   ok = ok && cudaMemsetAsync(m->counters, 0, sizeof(unsigned long long) * 2, e.stream) == cudaSuccess;
   if (!ok) return IDFX_ERR_CUDA;
-  k_refresh_bf16<<<(K1 * NH + 255) / 256, 256, 0, e.stream>>>(m->w, m->W1b, m->W2b, m->W3b);
+  k_pack_weights<<<(NPARAM + 255) / 256, 256, 0, e.stream>>>(m->w, m->Wp);
   if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(e.stream) != cudaSuccess) return IDFX_ERR_CUDA;
   return IDFX_OK;
 }
@@ -1124,17 +779,15 @@ int idfx_mlp_create(int max_batch, void* stream, idfx_mlp** out) {
     h->own_stream = true;
   }
   h->max_batch = max_batch;
+  // tiles of the worst batch: three chunks of 64 samples per block, two tiles
+  const size_t tiles = 2 * (((size_t)max_batch + 63) / 64 / 3 + 2);
   const size_t B = (size_t)max_batch;
   bool ok = dalloc(h, &h->w, NPARAM) && dalloc(h, &h->m, NPARAM) && dalloc(h, &h->v, NPARAM) &&
-            dalloc(h, &h->g, NPARAM) && dalloc(h, &h->W1b, (size_t)K1 * NH) && dalloc(h, &h->W2b, (size_t)NH * NH) &&
-            dalloc(h, &h->W3b, (size_t)NH * NOUT) && dalloc(h, &h->X, B * K1) && dalloc(h, &h->H1, B * NH) &&
-            dalloc(h, &h->H2, B * NH) && dalloc(h, &h->dYb, B * NOUT) && dalloc(h, &h->dZ2b, B * NH) &&
-            dalloc(h, &h->dZ1b, B * NH) && dalloc(h, &h->T, B * NOUT) && dalloc(h, &h->Z1, B * NH) &&
-            dalloc(h, &h->Z2, B * NH) && dalloc(h, &h->Y, B * NOUT) && dalloc(h, &h->dYf, B * NOUT) &&
-            dalloc(h, &h->dZ2f, B * NH) && dalloc(h, &h->dZ1f, B * NH) && dalloc(h, &h->loss, 2) &&
-            dalloc(h, &h->kmin, NIN) && dalloc(h, &h->kmax, NIN) && dalloc(h, &h->status, 1) &&
-            dalloc(h, &h->ws, GT_WS_FLOATS);
-  ok = ok && cudaFuncSetAttribute(k_gemm_tc, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)GT_SMEM) ==
+            dalloc(h, &h->g, NPARAM) && dalloc(h, &h->Wp, NPACK) && dalloc(h, &h->tiles[0], tiles) && dalloc(h, &h->tiles[1], tiles) &&
+            dalloc(h, &h->part, (size_t)MAX_BLOCKS * NPARAM) && dalloc(h, &h->cols, B * NBIAS) &&
+            dalloc(h, &h->ploss, MAX_BLOCKS * 2) && dalloc(h, &h->loss, 2) && dalloc(h, &h->kmin, NIN) &&
+            dalloc(h, &h->kmax, NIN) && dalloc(h, &h->status, 1);
+  ok = ok && cudaFuncSetAttribute(k_train_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_TRAIN) ==
                  cudaSuccess;
   if (ok) {
     k_init_keys<<<1, 256, 0, h->stream>>>(h->kmin, h->kmax);
@@ -1164,7 +817,7 @@ int idfx_mlp_set_params(idfx_mlp* h, const float* params) {
   cudaMemsetAsync(h->m, 0, sizeof(float) * NPARAM, h->stream);
   cudaMemsetAsync(h->v, 0, sizeof(float) * NPARAM, h->stream);
   h->t = 0;
-  k_refresh_bf16<<<(K1 * NH + 255) / 256, 256, 0, h->stream>>>(h->w, h->W1b, h->W2b, h->W3b);
+  k_pack_weights<<<(NPARAM + 255) / 256, 256, 0, h->stream>>>(h->w, h->Wp);
   return sync_ok(h);
 }
 
@@ -1188,9 +841,8 @@ int idfx_mlp_set_dataset_device(idfx_mlp* h, const float* prims, const float* ta
 
 int idfx_mlp_batch_device(idfx_mlp* h, int batch, unsigned long long seed, long long base, void* X, float* T) {
   if (!h || !h->prims || !X || !T || batch < 1) return IDFX_ERR_STATE;
-  k_make_batch<<<(batch + 127) / 128, 128, 0, h->stream>>>(h->prims, h->tgt, h->nsnap, h->nc, (float)h->gamma, seed,
-                                                           base, batch, static_cast<__nv_bfloat16*>(X), T, nullptr,
-                                                           nullptr);
+  k_make_batch<<<(batch + 31) / 32, 256, 0, h->stream>>>(dataset(h), seed, base, batch,
+                                                         static_cast<__nv_bfloat16*>(X), T);
   return sync_ok(h);
 }
 
@@ -1198,28 +850,38 @@ int idfx_mlp_train(idfx_mlp* h, int steps, int batch, float lr, float lr_end, un
                    float* losses) {
   if (!h || !h->prims || batch < 1 || batch > h->max_batch || steps < 0) return IDFX_ERR_STATE;
   double* dl = nullptr;
-  if (cudaMalloc(&dl, sizeof(double) * (steps > 0 ? steps : 1)) != cudaSuccess) return IDFX_ERR_CUDA;
-  cudaMemsetAsync(dl, 0, sizeof(double) * (steps > 0 ? steps : 1), h->stream);
+  if (cudaMalloc(&dl, sizeof(double) * 2 * (steps > 0 ? steps : 1)) != cudaSuccess) return IDFX_ERR_CUDA;
   const float b1 = 0.9f, b2 = 0.999f, eps = 1e-8f;
+  if (steps > 0) launch_assemble(h, batch, seed, h->t * (long long)batch, 0, true);
   for (int s = 0; s < steps; s++) {
-    const long long base = (h->t + s) * (long long)batch;
-    k_make_batch<<<(batch + 127) / 128, 128, 0, h->stream>>>(h->prims, h->tgt, h->nsnap, h->nc, (float)h->gamma,
-                                                             seed, base, batch, h->X, h->T, h->kmin, h->kmax);
-    fwd_bwd(h, batch, dl + s);
+    TrainArgs a = batch_args(h, batch);
+    a.compute = a.split.blocks;
+    a.tiles = h->tiles[s & 1];
+    a.part = h->part;
+    a.loss = h->ploss;
+    if (s + 1 < steps) {  // the next step's batch, meanwhile
+      a.next = h->tiles[(s + 1) & 1];
+      a.seed = seed;
+      a.base = (h->t + s + 1) * (long long)batch;
+      a.kmin = h->kmin;
+      a.kmax = h->kmax;
+    }
+    launch_tiles(h, a);
     const double tt = (double)(h->t + s + 1);
     const float frac = steps > 1 ? (float)s / (float)(steps - 1) : 1.f;
     const float lr_s = lr_end + 0.5f * (lr - lr_end) * (1.f + cosf(3.14159265f * frac));
-    k_adam<<<(NPARAM + 255) / 256, 256, 0, h->stream>>>(h->w, h->m, h->v, h->g, lr_s, b1, b2, eps,
-                                                        (float)(1.0 - std::pow((double)b1, tt)),
-                                                        (float)(1.0 - std::pow((double)b2, tt)), h->W1b, h->W2b,
-                                                        h->W3b);
+    launch_update(h, batch, true,
+                  AdamArgs{lr_s, b1, b2, eps, (float)(1.0 - std::pow((double)b1, tt)),
+                           (float)(1.0 - std::pow((double)b2, tt)), h->w, h->m, h->v, h->Wp},
+                  dl + 2 * s);
   }
   h->t += steps;
   int rc = sync_ok(h);
   if (!rc && losses && steps > 0) {
-    std::vector<double> hl(steps);
-    if (cudaMemcpy(hl.data(), dl, sizeof(double) * steps, cudaMemcpyDeviceToHost) != cudaSuccess) rc = IDFX_ERR_CUDA;
-    for (int s = 0; s < steps; s++) losses[s] = (float)hl[s];
+    std::vector<double> hl(2 * (size_t)steps);
+    if (cudaMemcpy(hl.data(), dl, sizeof(double) * 2 * steps, cudaMemcpyDeviceToHost) != cudaSuccess)
+      rc = IDFX_ERR_CUDA;
+    for (int s = 0; s < steps; s++) losses[s] = (float)hl[2 * s];
   }
   cudaFree(dl);
   return rc;
@@ -1227,18 +889,13 @@ int idfx_mlp_train(idfx_mlp* h, int steps, int batch, float lr, float lr_end, un
 
 int idfx_mlp_eval(idfx_mlp* h, int batch, unsigned long long seed, double* loss, double* loss_zero) {
   if (!h || !h->prims || batch < 1 || batch > h->max_batch) return IDFX_ERR_STATE;
-  cudaMemsetAsync(h->loss, 0, sizeof(double) * 2, h->stream);
-  k_make_batch<<<(batch + 127) / 128, 128, 0, h->stream>>>(h->prims, h->tgt, h->nsnap, h->nc, (float)h->gamma, seed,
-                                                           0, batch, h->X, h->T, nullptr, nullptr);
-  gemm(h->stream, batch, NH, K1, h->X, K1, 0, h->W1b, NH, 0,
-       EpiArgs{kEpiBiasSilu, h->w + OB1, nullptr, h->Z1, h->H1, NH}, h->status, h->ws);
-  gemm(h->stream, batch, NH, NH, h->H1, NH, 0, h->W2b, NH, 0,
-       EpiArgs{kEpiBiasSilu, h->w + OB2, nullptr, h->Z2, h->H2, NH}, h->status, h->ws);
-  gemm(h->stream, batch, NOUT, NH, h->H2, NH, 0, h->W3b, NOUT, 0,
-       EpiArgs{kEpiBias, h->w + OB3, nullptr, h->Y, nullptr, NOUT}, h->status, h->ws);
-  const int ne = batch * NOUT;
-  k_loss<<<(ne + 255) / 256, 256, 0, h->stream>>>(h->Y, h->T, batch, h->dYf, h->dYb, h->loss);
-  k_sumsq_targets<<<(ne + 255) / 256, 256, 0, h->stream>>>(h->T, batch, h->loss + 1);
+  launch_assemble(h, batch, seed, 0, 0, false);
+  TrainArgs a = batch_args(h, batch);
+  a.compute = a.split.blocks;
+  a.tiles = h->tiles[0];
+  a.loss = h->ploss;
+  launch_tiles(h, a);
+  launch_update(h, batch, false, AdamArgs{}, h->loss);
   double hl[2];
   if (cudaMemcpyAsync(hl, h->loss, sizeof(hl), cudaMemcpyDeviceToHost, h->stream) != cudaSuccess) return IDFX_ERR_CUDA;
   const int rc = sync_ok(h);
@@ -1262,10 +919,14 @@ int idfx_mlp_feature_range(idfx_mlp* h, float* fmin, float* fmax) {
 
 int idfx_mlp_grad_device(idfx_mlp* h, const void* X, const float* T, int batch, float* grad, double* loss) {
   if (!h || !X || !T || !grad || batch < 1 || batch > h->max_batch) return IDFX_ERR_STATE;
-  cudaMemcpyAsync(h->X, X, sizeof(__nv_bfloat16) * (size_t)batch * K1, cudaMemcpyDeviceToDevice, h->stream);
-  cudaMemcpyAsync(h->T, T, sizeof(float) * (size_t)batch * NOUT, cudaMemcpyDeviceToDevice, h->stream);
-  cudaMemsetAsync(h->loss, 0, sizeof(double), h->stream);
-  fwd_bwd(h, batch, h->loss);
+  TrainArgs a = batch_args(h, batch);
+  a.compute = a.split.blocks;
+  a.X = static_cast<const __nv_bfloat16*>(X);
+  a.T = T;
+  a.part = h->part;
+  a.loss = h->ploss;
+  launch_tiles(h, a);
+  launch_update(h, batch, true, AdamArgs{}, h->loss);
   cudaMemcpyAsync(grad, h->g, sizeof(float) * NPARAM, cudaMemcpyDeviceToHost, h->stream);
   double hl = 0.0;
   cudaMemcpyAsync(&hl, h->loss, sizeof(double), cudaMemcpyDeviceToHost, h->stream);
@@ -1276,13 +937,11 @@ int idfx_mlp_grad_device(idfx_mlp* h, const void* X, const float* T, int batch, 
 
 int idfx_mlp_forward_device(idfx_mlp* h, const void* X, int batch, float* Y) {
   if (!h || !X || !Y || batch < 1 || batch > h->max_batch) return IDFX_ERR_STATE;
-  cudaMemcpyAsync(h->X, X, sizeof(__nv_bfloat16) * (size_t)batch * K1, cudaMemcpyDeviceToDevice, h->stream);
-  gemm(h->stream, batch, NH, K1, h->X, K1, 0, h->W1b, NH, 0,
-       EpiArgs{kEpiBiasSilu, h->w + OB1, nullptr, h->Z1, h->H1, NH}, h->status, h->ws);
-  gemm(h->stream, batch, NH, NH, h->H1, NH, 0, h->W2b, NH, 0,
-       EpiArgs{kEpiBiasSilu, h->w + OB2, nullptr, h->Z2, h->H2, NH}, h->status, h->ws);
-  gemm(h->stream, batch, NOUT, NH, h->H2, NH, 0, h->W3b, NOUT, 0, EpiArgs{kEpiBias, h->w + OB3, nullptr, Y, nullptr,
-                                                                           NOUT}, h->status, h->ws);
+  TrainArgs a = batch_args(h, batch);
+  a.compute = a.split.blocks;
+  a.X = static_cast<const __nv_bfloat16*>(X);
+  a.Y = Y;
+  launch_tiles(h, a);
   return sync_ok(h);
 }
 

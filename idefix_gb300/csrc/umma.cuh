@@ -14,6 +14,11 @@
 // K (leading byte offset, LBO = 128), the 8-row groups follow each other
 // (stride byte offset, SBO).  One MMA consumes K = 16 (two core matrices
 // along K); the next K step starts 256 bytes further.
+// The same tile is the MN-major operand of its transpose (rows k = r, columns
+// m or n = c): the eight columns of a core matrix row are contiguous along
+// MN, 8-column groups follow each other 128 bytes apart (stride byte offset)
+// and 8-row groups K * 16 bytes apart (leading byte offset, along the MMA's
+// K); one MMA consumes 16 rows, 2 K * 16 bytes.
 #pragma once
 #include <cuda_bf16.h>
 #include <stdint.h>
@@ -40,8 +45,9 @@ __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr, uint32_t lbo, uint
 // instruction descriptor of kind::f16: D FP32 (bits 4-5 = 1), A and B BF16
 // (bits 7-9, 10-12 = 1), both K-major (bits 15, 16 = 0), N >> 3 (bits
 // 17-22), M >> 4 (bits 24-28)
-__host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N) {
-  return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+__host__ __device__ constexpr uint32_t idesc_bf16_f32(int M, int N, bool a_mn = false, bool b_mn = false) {
+  return (1u << 4) | (1u << 7) | (1u << 10) | ((a_mn ? 1u : 0u) << 15) | ((b_mn ? 1u : 0u) << 16) |
+         ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
 __device__ __forceinline__ uint32_t smem_addr(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -96,6 +102,17 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float* v) {
   for (int i = 0; i < 16; i++) v[i] = __uint_as_float(r[i]);
 }
 
+// and 16 columns of this thread's lane written
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const float* v) {
+  asm volatile(
+      "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};" ::"r"(
+          taddr),
+      "f"(v[0]), "f"(v[1]), "f"(v[2]), "f"(v[3]), "f"(v[4]), "f"(v[5]), "f"(v[6]), "f"(v[7]), "f"(v[8]), "f"(v[9]),
+      "f"(v[10]), "f"(v[11]), "f"(v[12]), "f"(v[13]), "f"(v[14]), "f"(v[15])
+      : "memory");
+  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
 __device__ __forceinline__ void mbar_init1(uint64_t* bar) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bar)) : "memory");
   asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -128,6 +145,28 @@ __device__ __forceinline__ void mma_tile(uint32_t d_tmem, uint32_t a_base, uint3
     const uint64_t bd = smem_desc(b_base + (uint32_t)k * 16u, 128u, sbo);
     mma_bf16(d_tmem, ad, bd, idesc, (accumulate || k > 0) ? 1u : 0u);
   }
+}
+
+// an operand over a tile of C columns at shared address `base`: as it lies
+// (K-major, the MMA's K along the columns) or transposed (MN-major, K along
+// the rows)
+struct Operand {
+  uint32_t base, lbo, sbo, step;
+  bool mn;
+};
+__device__ __forceinline__ Operand along_columns(uint32_t base, int C) {
+  return Operand{base, 128u, (uint32_t)C * 16u, 256u, false};
+}
+__device__ __forceinline__ Operand along_rows(uint32_t base, int C) {
+  return Operand{base, (uint32_t)C * 16u, 128u, (uint32_t)C * 32u, true};
+}
+// D (M x N, TMEM) (+)= A . B^T over K (a multiple of 16), issued by one thread
+__device__ __forceinline__ void mma_run(uint32_t d_tmem, const Operand& a, const Operand& b, int M, int N, int K,
+                                        bool accumulate = false) {
+  const uint32_t idesc = idesc_bf16_f32(M, N, a.mn, b.mn);
+  for (int q = 0; q < K / 16; q++)
+    mma_bf16(d_tmem, smem_desc(a.base + q * a.step, a.lbo, a.sbo), smem_desc(b.base + q * b.step, b.lbo, b.sbo), idesc,
+             accumulate || q > 0 ? 1u : 0u);
 }
 
 }  // namespace umma
