@@ -769,10 +769,12 @@ int idfx_gpu_create(const idfx_gpu_config* cfg, void* stream, idfx_gpu** out) {
   const int NV = 2 * g.D + 2;
   const size_t nc = (size_t)g.ncell, nf = (size_t)g.nface;
   const bool hll_emf = (g.emf == kEmfUctHll || g.emf == kEmfUctHlld);
+  // the mixed path's sweeps and the learned correction read the primitives in FP32
+  const bool vc32 = cfg->precision == IDFX_MIXED || cfg->order == IDFX_LEARNED;
   size_t len = 3 * NV * nc + 2 * g.D * nf + nc  // Vc, Uc, Uc0, Vs, Vs0, InvDt
                + 6 * nc + 3 * nc + 3 * nc + 3 * nc  // face EMFs, sv, cell EMFs, corner EMFs
                + (hll_emf ? 12 * nc : 0)
-               + (cfg->precision == IDFX_MIXED ? (NV * nc + 1) / 2 : 0)   // FP32 primitives
+               + (vc32 ? (NV * nc + 1) / 2 : 0)                           // FP32 primitives
                + (cfg->shock_flattening ? (nc + 7) / 8 : 0);               // shock flags
   int rc = IDFX_OK;
   if (stream) {
@@ -812,7 +814,7 @@ int idfx_gpu_create(const idfx_gpu_config* cfg, void* stream, idfx_gpu** out) {
     f.dL[d] = hll_emf ? take(nc) : nullptr;
     f.dR[d] = hll_emf ? take(nc) : nullptr;
   }
-  f.Vc32 = (cfg->precision == IDFX_MIXED) ? reinterpret_cast<float*>(take((NV * nc + 1) / 2)) : nullptr;
+  f.Vc32 = vc32 ? reinterpret_cast<float*>(take((NV * nc + 1) / 2)) : nullptr;
   f.shock = cfg->shock_flattening ? reinterpret_cast<unsigned char*>(take((nc + 7) / 8)) : nullptr;
   Ctl c{};
   c.t = 0.0;

@@ -16,6 +16,7 @@
 #include "../../include/idefix_gb300.h"
 #include "engine.hpp"
 #include "learned.cuh"
+#include "sweep_cell.cuh"
 #include "train_tile.cuh"
 #include "umma.cuh"
 
@@ -117,54 +118,43 @@ __global__ void k_coarsen(const double* __restrict__ Vc, const double* __restric
 }
 
 // ---------------------------------------------------------------------------
-// Learned sweep (ORDER 5): reconstruction with the network's correction,
-// Riemann solve and flux difference of one direction in one kernel, over
-// tiles of 128 cells laid along the sweep's pencils (lines of cells along
-// DIR: the active cells plus one ghost cell at each end, for every column
-// of the other two directions including the CT extension).  Per tile:
-//   1. stencil features of the 128 cells (BF16, canonical K-major layout);
-//   2. the three layers on the 5th-generation tensor cores - one thread
-//      issues tcgen05.mma over the shared-memory operands, the FP32
-//      accumulators live in tensor memory, the epilogues (bias, SiLU) read
-//      them back with tcgen05.ld and write the next layer's operand;
-//   3. each cell's PLM (van Leer) states plus the correction, or the plain
-//      PLM states where the stencil is outside the trained feature range or
-//      a corrected density / pressure is not positive (the cell's two faces
-//      together), kept in shared memory;
-//   4. the HLLD solve of every face between two cells of the tile, its EMF
-//      outputs, and the flux difference of every cell with both faces in the
-//      tile (the march's expressions, so that with a zero correction the
-//      sweep is bit-identical to the plain PLM march).
-// Pencils of up to 128 cells are packed whole into a tile; longer pencils
-// are cut into segments of 128 cells that overlap by two (the face between
-// them is solved by both, with the same result).  Persistent CTAs of 256
-// threads, the BF16 weights resident in shared memory.  With states != null
-// the kernel writes the face states ([3][16][ncell]: direction, face
-// (minus / plus) x variable) and stops before the Riemann solves.
+// Learned correction (ORDER 5): the network over every cell whose face states
+// a sweep reconstructs, for the three directions in one launch; the sweeps
+// (k_sweep_learned: the cell sweep of the FP64 path) then add the correction
+// to the PLM states.  Together in one kernel per direction, 128 of its 256
+// threads solved FP64 Riemann problems while the tensor core and the other
+// half waited, features were gathered from FP64 three times over, and a 32^3
+// box left 2.5 tiles per multiprocessor to each of six launches a cycle.
+// A tile is 128 consecutive cells of the box of those cells (x fastest):
+//   1. the scaled stencil of every cell once, as BF16, [variable][neighbour][cell];
+//      the three directions' inputs are permutations of it;
+//   2. per direction: its input in the canonical K-major layout, the three
+//      layers on the tensor cores (umma.cuh; the next layer's operand over the
+//      last one's), and the sixteen outputs to Y [3][16][ncell] - the first a
+//      NaN where the stencil leaves the trained range, which the sweep takes
+//      as it takes a correction that leaves a density or pressure not positive.
+// Persistent blocks of 512 threads (four per cell), the packed weights fetched
+// by one bulk copy; a block's share is a run of (tile, direction) pairs, so
+// that a small box is spread over all multiprocessors (12^3: 66 pairs of 22
+// tiles) and a middling one leaves no round nearly empty (32^3: 307 tiles are
+// three rounds of 152 blocks, 921 pairs seven of a third each).
+// Measured (32^3, both stages of a cycle): the three fused sweeps 434 / 469 /
+// 472 us; this launch 185 us (241 with whole tiles to a block and the range
+// looked up by column) and the three sweeps 91 / 93 / 95 us.  Two cycles with
+// their copies 3356 -> 1196 us, one cycle of 64^3 13978 -> 2792 us.
 // ---------------------------------------------------------------------------
-constexpr int LT = 128;  // cells (rows) per tile
-constexpr size_t LS_W1 = 0;                                  // W1: N 128 x K 224
-constexpr size_t LS_W2 = LS_W1 + (size_t)NH * K1 * 2;        // W2: 128 x 128
-constexpr size_t LS_W3 = LS_W2 + (size_t)NH * NH * 2;        // W3: 16 x 128
-constexpr size_t LS_X = LS_W3 + (size_t)NOUT * NH * 2;       // features 128 x 224 (reused)
-constexpr size_t LS_H = LS_X + (size_t)LT * K1 * 2;          // layer-1 output 128 x 128
-constexpr size_t LS_B = LS_H + (size_t)LT * NH * 2;          // biases
-constexpr size_t LS_R = LS_B + (size_t)(2 * NH + NOUT) * 4;  // trained range
-constexpr size_t LS_F = LS_R + (size_t)2 * NIN * 4;          // per-row fallback flags
-constexpr size_t LS_M = LS_F + (size_t)LT * 4;               // counter, mbarrier, TMEM slot
+constexpr int LT = 128;   // cells of a tile
+constexpr int LN = 512;   // threads
+constexpr size_t LS_W = 0;                                   // packed weights
+constexpr size_t LS_X = LS_W + (size_t)NPACK * 2;            // input 128 x 224, then the layers' outputs
+constexpr size_t LS_F = LS_X + (size_t)LT * K1 * 2;          // scaled stencil [216][128] BF16
+constexpr size_t LS_B = LS_F + (size_t)NIN * LT * 2;         // biases
+constexpr size_t LS_R = LS_B + (size_t)(2 * NH + NOUT) * 4;  // trained range of a stencil element, per direction
+constexpr size_t LS_O = LS_R + (size_t)3 * NIN * 8;          // cells outside it, per direction
+constexpr size_t LS_M = LS_O + (size_t)3 * LT * 4;           // mbarriers, TMEM slot
 constexpr size_t SM_LEARN = LS_M + 32;
-// inside the feature region once the network is done with it
-constexpr size_t LX_Y = 0;                                   // outputs 128 x 16 FP32
-constexpr size_t LX_S = LX_Y + (size_t)LT * NOUT * 4;        // face states 128 x 2 x 8 FP64
-constexpr size_t LX_FA = LX_S + (size_t)LT * 16 * 8;         // flux x area 128 x 5 FP64
-constexpr size_t LX_CM = LX_FA + (size_t)LT * 5 * 8;         // wave speed 128 FP64
-static_assert(LX_CM + (size_t)LT * 8 <= (size_t)LT * K1 * 2, "tile outputs exceed the feature region");
-static_assert(LS_X % 128 == 0 && LS_H % 128 == 0 && LS_W2 % 128 == 0 && LS_W3 % 128 == 0, "operand alignment");
-static_assert(SM_LEARN <= 227 * 1024, "learned sweep does not fit in shared memory");
-
-static_assert(LS_W2 - LS_W1 == (size_t)(PW2 - PW1) * 2 && LS_W3 - LS_W1 == (size_t)(PW3 - PW1) * 2 &&
-                  LS_X - LS_W1 == (size_t)NPACK * 2,
-              "the packed weights as they lie");
+static_assert(LS_X % 128 == 0 && LS_M % 8 == 0, "operand alignment");
+static_assert(SM_LEARN <= 227 * 1024, "learned correction does not fit in shared memory");
 
 struct LearnedDev {
   const __nv_bfloat16* Wp;   // packed weights
@@ -173,298 +163,213 @@ struct LearnedDev {
   const float* fmax;
 };
 
-// tiling of one direction's pencils into tiles of LT cells
-struct LTiles {
-  int L;              // cells per pencil: n[DIR] + 2
-  int per_tile;       // pencils per tile when L <= LT, else 0
-  int nseg;           // segments of LT cells per pencil when L > LT
-  int nA;             // pencils along the first transverse direction (with the CT extension)
-  long long npencil;  // pencils
-  long long ntiles;
+// the cells that get a correction: lo .. lo + m - 1 in every direction
+struct LBox {
+  int lo[3], m[3];
+  long long cells;
 };
-
-__host__ inline LTiles make_tiles(const Geo& g, int dir) {
-  const int A = (dir == 0) ? 1 : 0, B = (dir == 2) ? 1 : 2;
-  LTiles t{};
-  t.L = g.n[dir] + 2;
-  t.nA = g.n[A] + 2 * g.ext;
-  t.npencil = (long long)t.nA * (g.n[B] + 2 * g.ext);
-  if (t.L <= LT) {
-    t.per_tile = LT / t.L;
-    t.nseg = 1;
-    t.ntiles = (t.npencil + t.per_tile - 1) / t.per_tile;
-  } else {
-    t.per_tile = 0;
-    t.nseg = (t.L - 2 + (LT - 2) - 1) / (LT - 2);
-    t.ntiles = t.npencil * t.nseg;
+__host__ inline LBox learned_box(const Geo& g) {
+  LBox b{};
+  const int e = g.ext > 1 ? g.ext : 1;  // columns of the CT extension, the ghost cell at a line's ends
+  b.cells = 1;
+  for (int d = 0; d < 3; d++) {
+    b.lo[d] = g.beg[d] - e;
+    b.m[d] = g.n[d] + 2 * e;
+    b.cells *= b.m[d];
   }
+  return b;
+}
+
+// stencil element (solver variable * 27 + neighbour, x fastest) of feature
+// column col of direction d (rotated variable, then neighbour with the sweep
+// direction fastest)
+__host__ __device__ constexpr int stencil_of(int d, int col) {
+  const int rv = col / 27, q = col % 27;
+  int o[3] = {0, 0, 0};
+  o[d] = q % 3;
+  o[(d + 1) % 3] = q / 3 % 3;
+  o[(d + 2) % 3] = q / 9;
+  return rot_var(rv, d) * 27 + o[2] * 9 + o[1] * 3 + o[0];
+}
+struct StencilTable {
+  unsigned char at[3][K1];
+};
+constexpr StencilTable stencil_table() {
+  StencilTable t{};
+  for (int d = 0; d < 3; d++)
+    for (int c = 0; c < NIN; c++) t.at[d][c] = (unsigned char)stencil_of(d, c);
   return t;
 }
+__constant__ StencilTable kStencil = stencil_table();
+static_assert(NIN <= 256, "stencil element in a byte");
 
-// element (r, k) of a BF16 operand tile with K columns
-__device__ __forceinline__ void put_bf16(unsigned char* base, int r, int k, int K, float v) {
-  reinterpret_cast<__nv_bfloat16*>(base)[umma::kmajor_offset(r, k, K) / 2] = __float2bfloat16(v);
-}
-
-template <int DIR>
-__global__ void __launch_bounds__(256, 1) k_learned_sweep(Geo g, Fields f, LearnedDev L, const Ctl* ctl, LTiles T,
-                                                          int invdt, int last_dir, double* __restrict__ states,
-                                                          unsigned long long* __restrict__ counters) {
+__global__ void __launch_bounds__(LN, 1) k_learned_correct(Geo g, const float* __restrict__ Vc, LearnedDev L,
+                                                           Ctl* ctl, LBox box, float* __restrict__ Y) {
   if (ctl->done) return;
-  constexpr int A = (DIR == 0) ? 1 : 0, B = (DIR == 2) ? 1 : 2;
-  using v = Var<3>;
   extern __shared__ __align__(128) unsigned char sm[];
-  unsigned char* W1s = sm + LS_W1;
-  unsigned char* W2s = sm + LS_W2;
-  unsigned char* W3s = sm + LS_W3;
   unsigned char* Xs = sm + LS_X;
-  unsigned char* Hs = sm + LS_H;
+  __nv_bfloat16* Fs = reinterpret_cast<__nv_bfloat16*>(sm + LS_F);
   float* bs = reinterpret_cast<float*>(sm + LS_B);
-  float* rmin = reinterpret_cast<float*>(sm + LS_R);
-  float* rmax = rmin + NIN;
-  int* flag = reinterpret_cast<int*>(sm + LS_F);
-  int* nfall = reinterpret_cast<int*>(sm + LS_M);
-  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + LS_M + 8);
+  float2* range = reinterpret_cast<float2*>(sm + LS_R);
+  int* out = reinterpret_cast<int*>(sm + LS_O);
+  uint64_t* bar = reinterpret_cast<uint64_t*>(sm + LS_M);
   uint32_t* slot = reinterpret_cast<uint32_t*>(sm + LS_M + 16);
-  float* Ys = reinterpret_cast<float*>(Xs + LX_Y);
-  double* FS = reinterpret_cast<double*>(Xs + LX_S);
-  double* FA = reinterpret_cast<double*>(Xs + LX_FA);
-  double* CM = reinterpret_cast<double*>(Xs + LX_CM);
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  // weights as the B operands (N x K, K-major)
-  for (int e = tid; e < NPACK / 8; e += blockDim.x)
-    reinterpret_cast<uint4*>(W1s)[e] = reinterpret_cast<const uint4*>(L.Wp)[e];
-  for (int e = tid; e < NH; e += blockDim.x) {
+  const int row = 32 * (warp & 3) + lane, quarter = warp >> 2;
+  const uint32_t lanes = (uint32_t)(32 * (warp & 3)) << 16;
+  if (warp == 0) umma::tmem_alloc(slot, 256);  // layer 1: columns 0-127, layer 2: 128-255, layer 3: 0-15
+  if (tid == 0) {
+    umma::mbar_init1(bar);
+    mbar_init(bar + 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    mbar_expect(bar + 1, NPACK * 2);
+    bulk_to_smem(sm + LS_W, L.Wp, NPACK * 2, bar + 1);
+  }
+  for (int e = tid; e < NH; e += LN) {
     bs[e] = L.w[OB1 + e];
     bs[NH + e] = L.w[OB2 + e];
   }
   if (tid < NOUT) bs[2 * NH + tid] = L.w[OB3 + tid];
   const bool ranged = L.fmin != nullptr;
-  for (int e = tid; e < NIN; e += blockDim.x) {
-    rmin[e] = ranged ? L.fmin[e] : 0.f;
-    rmax[e] = ranged ? L.fmax[e] : 0.f;
+  if (ranged) {
+    for (int e = tid; e < 3 * NIN; e += LN) {
+      const int d = e / NIN, c = e % NIN;
+      range[3 * kStencil.at[d][c] + d] = make_float2(L.fmin[c], L.fmax[c]);
+    }
   }
-  if (warp == 0) umma::tmem_alloc(slot, 256);  // layer 1: columns 0-127, layer 2: 128-255, layer 3: 0-15
-  if (tid == 0) umma::mbar_init1(bar);
   umma::fence_before_sync();
   __syncthreads();
   umma::fence_after_sync();
   const uint32_t tmem = *slot;
+  const uint32_t xa = umma::smem_addr(Xs), w1 = umma::smem_addr(sm + LS_W), w2 = w1 + PW2 * 2, w3 = w1 + PW3 * 2;
   uint32_t phase = 0;
-  bool ok = true;
-  const int row = tid & (LT - 1), half = tid >> 7;
-  const int a1 = (DIR + 1) % 3, a2 = (DIR + 2) % 3;
-  const long long sd = g.s[DIR], s1 = g.s[a1], s2 = g.s[a2];
-  const double dtdV = ctl->dtdV;
-  const double areaT = g.A[DIR];
-  double run_max = 0.0;  // max of InvDt over this thread's cells
-  // one MMA run of a layer, then every thread waits (bounded) for it
-  auto layer = [&](uint32_t d_col, const unsigned char* a, const unsigned char* b, int K, int N) {
+  auto tensor = [&](uint32_t d_col, int K, uint32_t w, int N) -> bool {
     umma::fence_async_smem();
     umma::fence_before_sync();
     __syncthreads();
     umma::fence_after_sync();
     if (tid == 0) {
-      umma::mma_tile(tmem + d_col, umma::smem_addr(a), umma::smem_addr(b), K, umma::idesc_bf16_f32(LT, N), false);
+      umma::mma_run(tmem + d_col, umma::along_columns(xa, K), umma::along_columns(w, K), LT, N, K);
       umma::mma_commit(bar);
     }
-    const bool w = umma::mbar_wait_bounded(bar, phase, umma::kMmaSpin);
+    const bool in = umma::mbar_wait_bounded(bar, phase, umma::kMmaSpin);
     phase ^= 1u;
-    ok = __syncthreads_and(w) != 0;
+    const bool ok = __syncthreads_and(in) != 0;
     umma::fence_after_sync();
+    return ok;
   };
-  // hidden-layer epilogue: SiLU(acc + bias) -> BF16 operand of the next layer
-  // (warp w: rows 32 (w % 4) .., columns 64 (w / 4) ..)
-  auto hidden = [&](uint32_t d_col, const float* bias, unsigned char* out) {
-    const int r = 32 * (warp & 3) + lane, c0 = 64 * (warp >> 2);
-    for (int c = c0; c < c0 + 64; c += 16) {
+  // SiLU(acc + bias) -> BF16 operand of the next layer, in the input's place
+  auto hidden = [&](uint32_t d_col, const float* bias) {
+    for (int c = NH / 4 * quarter; c < NH / 4 * (quarter + 1); c += 16) {
       float x[16];
-      umma::tmem_ld16(tmem + ((uint32_t)(32 * (warp & 3)) << 16) + d_col + (uint32_t)c, x);
+      umma::tmem_ld16(tmem + lanes + d_col + (uint32_t)c, x);
 #pragma unroll
-      for (int i = 0; i < 16; i++) put_bf16(out, r, c + i, NH, silu_f(x[i] + bias[c + i]));
+      for (int i = 0; i < 16; i++) x[i] = silu_f(x[i] + bias[c + i]);
+      put8(Xs, row, c, NH, x);
+      put8(Xs, row, c + 8, NH, x + 8);
     }
   };
-  for (long long tile = blockIdx.x; tile < T.ntiles && ok; tile += gridDim.x) {
-    // ---- this thread's row: pencil, cell along DIR, segment ends --------
-    long long pencil;
-    int pos;
-    bool valid, first, last;
-    if (T.per_tile) {
-      const int q = row / T.L;
-      pos = row - q * T.L;
-      pencil = tile * T.per_tile + q;
-      valid = q < T.per_tile && pencil < T.npencil;
-      first = pos == 0;
-      last = pos == T.L - 1;
-    } else {
-      pencil = tile / T.nseg;
-      pos = (int)(tile % T.nseg) * (LT - 2) + row;
-      valid = pos < T.L;
-      first = row == 0;
-      last = row == LT - 1 || pos == T.L - 1;
-    }
-    if (!valid) {
-      pencil = 0;
-      pos = 1;
-    }
-    int ix[3];
-    ix[DIR] = g.beg[DIR] - 1 + pos;
-    ix[A] = g.beg[A] - g.ext + (int)(pencil % T.nA);
-    ix[B] = g.beg[B] - g.ext + (int)(pencil / T.nA);
-    const bool active_col = ix[A] >= g.beg[A] && ix[A] < g.end[A] && ix[B] >= g.beg[B] && ix[B] < g.end[B];
+  bool ok = __syncthreads_and(mbar_wait(bar + 1, 0u)) != 0;  // the weights
+  const int tiles = (int)((box.cells + LT - 1) / LT);
+  // this block's share of all tiles' directions, in a row
+  int item = (int)(3LL * tiles * blockIdx.x / gridDim.x);
+  const int end = (int)(3LL * tiles * (blockIdx.x + 1) / gridDim.x);
+  while (item < end && ok) {
+    const long long q = (long long)(item / 3) * LT + row;
+    const bool valid = q < box.cells;
+    const unsigned p = valid ? (unsigned)q : 0u;  // cells of a box fit 31 bits
+    const int ix[3] = {box.lo[0] + (int)(p % (unsigned)box.m[0]),
+                       box.lo[1] + (int)(p / (unsigned)box.m[0] % (unsigned)box.m[1]),
+                       box.lo[2] + (int)(p / (unsigned)box.m[0] / (unsigned)box.m[1])};
     const long long cc = cidx(g, ix[2], ix[1], ix[0]);
-    if (tid < LT) flag[tid] = valid ? 0 : 1;
-    if (tid == 0) *nfall = 0;
+    for (int e = tid; e < 3 * LT; e += LN) out[e] = 0;
     __syncthreads();
-    // ---- 1. stencil features (half 0: rotated variables 0-3, half 1: 4-7)
+    // ---- the scaled stencil, two variables per thread ------------------
     {
-      float cen[8];
-#pragma unroll
-      for (int rv = 0; rv < 8; rv++) cen[rv] = (float)f.Vc[rot_var(rv, DIR) * g.ncell + cc];
-      const float cs = sqrtf((float)g.gamma * cen[4] / cen[0]), sb = sqrtf(cen[0]) * cs;
+      const float rho = Vc[cc], prs = Vc[4 * g.ncell + cc];
+      const float cs = sqrtf((float)g.gamma * prs / rho), sb = sqrtf(rho) * cs;
       int bad = 0;
-      for (int q = 0; q < 4; q++) {
-        const int rv = half * 4 + q;
-        const double* base = f.Vc + rot_var(rv, DIR) * g.ncell + cc;
-        for (int o2 = -1; o2 <= 1; o2++)
-          for (int o1 = -1; o1 <= 1; o1++)
-            for (int o0 = -1; o0 <= 1; o0++) {
-              const float sv = valid ? (float)base[o0 * sd + o1 * s1 + o2 * s2] : 0.f;
+#pragma unroll
+      for (int k = 0; k < 2; k++) {
+        const int v = 2 * quarter + k;
+        const float* base = Vc + v * g.ncell;
+        const float cen = base[cc];
+#pragma unroll
+        for (int oz = -1; oz <= 1; oz++)
+#pragma unroll
+          for (int oy = -1; oy <= 1; oy++)
+#pragma unroll
+            for (int ox = -1; ox <= 1; ox++) {
+              // inside the array whatever the extension (uct_hll(d) takes a
+              // column more than the stencil has around it)
+              const int nx = min(max(ix[0] + ox, 0), g.nt[0] - 1), ny = min(max(ix[1] + oy, 0), g.nt[1] - 1),
+                        nz = min(max(ix[2] + oz, 0), g.nt[2] - 1);
+              const float s = base[cidx(g, nz, ny, nx)];
               float x;
-              if (rv == 0 || rv == 4) x = sv / cen[rv] - 1.f;
-              else if (rv < 4) x = (sv - cen[rv]) / cs;
-              else x = sv / sb;
-              const int col = rv * 27 + (o2 + 1) * 9 + (o1 + 1) * 3 + (o0 + 1);
-              if (!valid) x = 0.f;
-              if (ranged && !(x >= rmin[col] && x <= rmax[col])) bad = 1;
-              put_bf16(Xs, row, col, K1, x);
+              if (v == 0 || v == 4) x = s / cen - 1.f;
+              else if (v < 4) x = zdiv(s - cen, cs);
+              else x = zdiv(s, sb);
+              const int nb = (oz + 1) * 9 + (oy + 1) * 3 + (ox + 1);
+              Fs[(v * 27 + nb) * LT + row] = __float2bfloat16(valid ? x : 0.f);
+              if (ranged) {
+#pragma unroll
+                for (int d = 0; d < 3; d++) {
+                  const float2 r = range[3 * (v * 27 + nb) + d];
+                  if (!(x >= r.x && x <= r.y)) bad |= 1 << d;
+                }
+              }
             }
       }
-      if (half == 1)
-        for (int col = NIN; col < K1; col++) put_bf16(Xs, row, col, K1, 0.f);
-      if (bad) atomicOr(flag + row, 1);
+#pragma unroll
+      for (int d = 0; d < 3; d++)
+        if (bad & (1 << d)) out[d * LT + row] = 1;  // (any of the cell's threads)
     }
-    // ---- 2. the network on the tensor cores -----------------------------
-    layer(0, Xs, W1s, K1, NH);  // layer 1 -> TMEM columns 0-127
-    if (!ok) break;
-    hidden(0, bs, Hs);
-    layer(NH, Hs, W2s, NH, NH);  // layer 2 -> TMEM columns 128-255
-    if (!ok) break;
-    hidden(NH, bs + NH, Xs);     // layer-2 output over the features
-    layer(0, Xs, W3s, NH, NOUT);  // layer 3 -> TMEM columns 0-15
-    if (!ok) break;
-    if (warp < 4) {
+    __syncthreads();
+    for (int d = item % 3; d < 3 && item < end && ok; d++, item++) {
+      for (int c = 8 * quarter; c < K1; c += 32) {  // this direction's input, eight columns at a time
+        alignas(16) __nv_bfloat16 t[8];
+#pragma unroll
+        for (int i = 0; i < 8; i++)
+          t[i] = c + i < NIN ? Fs[(int)kStencil.at[d][c + i] * LT + row] : __float2bfloat16(0.f);
+        *reinterpret_cast<uint4*>(Xs + umma::kmajor_offset(row, c, K1)) = *reinterpret_cast<const uint4*>(t);
+      }
+      ok = tensor(0, K1, w1, NH);  // layer 1 -> TMEM columns 0-127
+      if (!ok) break;
+      hidden(0, bs);
+      ok = tensor(NH, NH, w2, NH);  // layer 2 -> TMEM columns 128-255
+      if (!ok) break;
+      hidden(NH, bs + NH);
+      ok = tensor(0, NH, w3, NOUT);  // layer 3 -> TMEM columns 0-15
+      if (!ok) break;
       float y[16];
-      umma::tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16), y);
+      umma::tmem_ld16(tmem + lanes, y);
+      if (valid) {
 #pragma unroll
-      for (int i = 0; i < 16; i++) Ys[row * NOUT + i] = y[i] + bs[2 * NH + i];
-    }
-    __syncthreads();
-    // ---- 3. corrected face states (thread: cell row, face = half) -------
-    {
-      double cen[8], vl[8], vr[8], st[8];
-      const double dxd = g.dx[DIR];
-#pragma unroll
-      for (int sv = 0; sv < 8; sv++) {
-        const double* base = f.Vc + sv * g.ncell + cc;
-        double w[3];
-        w[0] = valid ? base[-sd] : 1.0;
-        w[1] = valid ? base[0] : 1.0;
-        w[2] = valid ? base[sd] : 1.0;
-        cen[sv] = w[1];
-        Recon<2>::cell<double>(w, dxd, sv == 0 || sv == 4, vl[sv], vr[sv]);
-      }
-      const double cs = sqrt(g.gamma * cen[4] / cen[0]), sb = sqrt(cen[0]) * cs;
-      const double sc[8] = {cen[0], cs, cs, cs, cen[4], sb, sb, sb};
-#pragma unroll
-      for (int rv = 0; rv < 8; rv++) {
-        const int sv = rot_var(rv, DIR);
-        const double plm = half ? vr[sv] : vl[sv];
-        st[sv] = plm;
-        if (rv == 5) continue;  // normal field: the face value is used
-        st[sv] = plm + (double)Ys[row * NOUT + half * 8 + rv] * sc[rv];
-      }
-      if (!(st[0] > 0.0) || !(st[4] > 0.0)) atomicOr(flag + row, 1);
-      __syncthreads();
-      const bool fall = flag[row] != 0;
-      if (fall) {
-#pragma unroll
-        for (int sv = 0; sv < 8; sv++) st[sv] = half ? vr[sv] : vl[sv];
-      }
-#pragma unroll
-      for (int sv = 0; sv < 8; sv++) FS[(row * 2 + half) * 8 + sv] = st[sv];
-      if (valid && states) {
-#pragma unroll
-        for (int sv = 0; sv < 8; sv++) states[((long long)DIR * 16 + half * 8 + sv) * g.ncell + cc] = st[sv];
-      }
-      if (valid && half == 0 && fall) atomicAdd(nfall, 1);
-    }
-    __syncthreads();
-    if (tid == 0 && counters) {
-      long long nvalid;
-      if (T.per_tile) {
-        const long long left = T.npencil - tile * T.per_tile;
-        nvalid = (long long)T.L * (left < T.per_tile ? left : T.per_tile);
-      } else {
-        const long long p0 = (tile % T.nseg) * (LT - 2);
-        nvalid = (T.L - p0 < LT) ? (T.L - p0) : LT;
-      }
-      atomicAdd(counters, (unsigned long long)nvalid);
-      atomicAdd(counters + 1, (unsigned long long)*nfall);
-    }
-    if (states) continue;
-    // ---- 4. Riemann solve of the face between this row and the next -----
-    if (tid < LT && valid && !last) {
-      double vL[8], vR[8];
-#pragma unroll
-      for (int n = 0; n < 8; n++) {
-        vL[n] = FS[(row * 2 + 1) * 8 + n];        // plus-face state of this cell
-        vR[n] = FS[((row + 1) * 2 + 0) * 8 + n];  // minus-face state of the next
-      }
-      int jx[3] = {ix[0], ix[1], ix[2]};
-      jx[DIR] += 1;
-      const long long cn = cidx(g, jx[2], jx[1], jx[0]);  // the face is the next cell's minus face
-      const double bn = f.Vs[DIR * g.nface + fidx(g, jx[2], jx[1], jx[0])];
-      vL[v::BX1 + DIR] = bn;
-      vR[v::BX1 + DIR] = bn;
-      RiemannOut<3, double> r;
-      riemann<3, DIR, kHLLD>(g.gamma, g.rgm1, vL, vR, r);
-      store_emf<3, DIR>(g, f, cn, r, vL, vR);
-      if (active_col) {
-#pragma unroll
-        for (int n = 0; n < v::BX1; n++) FA[row * 5 + n] = r.F[n] * areaT;
-        CM[row] = r.cmax;
+        for (int o = 0; o < NOUT; o++) {
+          if (o / 4 != quarter) continue;
+          float z = y[o] + bs[2 * NH + o];
+          if (o == 0 && out[d * LT + row]) z = __int_as_float(0x7fffffff);
+          Y[((long long)d * NOUT + o) * g.ncell + cc] = z;
+        }
       }
     }
-    __syncthreads();
-    // ---- flux difference of the cells with both faces in the tile -------
-    if (tid < LT && valid && !first && !last && active_col) {
-#pragma unroll
-      for (int n = 0; n < v::BX1; n++) {
-        const double rhs = -dtdV * (FA[row * 5 + n] - FA[(row - 1) * 5 + n]);
-        f.Uc[n * g.ncell + cc] = f.Uc[n * g.ncell + cc] + rhs;
-      }
-      if (invdt) {
-        const double prev = (invdt == 1) ? 0.0 : f.InvDt[cc];
-        const double inv = prev + div_r(0.5 * (CM[row] + CM[row - 1]), Recip{g.dx[DIR], g.rdx[DIR]});
-        f.InvDt[cc] = inv;
-        if (inv > run_max) run_max = inv;  // NaN never compares greater
-      }
-    }
-    __syncthreads();  // the feature region is rewritten by the next tile
+    __syncthreads();  // the stencil and its flags are rewritten by the next tile
   }
-  if (!ok && tid == 0) report_wait_timeout(ctl);
-  if (last_dir && invdt && !states) {
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) {
-      const double w = __shfl_xor_sync(0xffffffffu, run_max, o);
-      if (w > run_max) run_max = w;
-    }
-    if (lane == 0 && run_max > 0.0) atomic_max_pos((unsigned long long*)&((Ctl*)ctl)->invdt_max_bits, run_max);
+  if (!ok && tid == 0) {
+    report_wait_timeout(ctl);
+    mbar_wait(bar + 1, 0u);  // no copy may land after the block has gone
   }
   umma::fence_before_sync();
   __syncthreads();
   if (warp == 0) umma::tmem_dealloc(tmem, 256);
+}
+
+// the cell sweep with PLM plus the correction (sweep_cell.cuh, ORDER 5)
+template <int DIR>
+__global__ void __launch_bounds__(kCellThreads, 3)
+    k_sweep_learned(Geo g, Fields f, const Ctl* ctl, int invdt, int last_dir, LearnedRecon lr) {
+  extern __shared__ double learned_cell_sm[];
+  d_sweep_cell<3, DIR, IDFX_LEARNED, kHLLD>(g, f, ctl, invdt, last_dir, blockIdx.x, learned_cell_sm, lr);
 }
 
 __global__ void k_init_keys(unsigned* kmin, unsigned* kmax) {
@@ -532,32 +437,38 @@ struct LearnedModel {
   __nv_bfloat16* Wp = nullptr;
   float* w = nullptr;
   float *fmin = nullptr, *fmax = nullptr;
+  float* Y = nullptr;  // corrections [3][NOUT][ncell]
   unsigned long long* counters = nullptr;
   bool ranged = false;
 };
 
 namespace idfx {
 
-// the learned sweeps of one stage, direction after direction (the same
-// InvDt modes as the march: 1 first contribution, 2 accumulate; the last
-// direction folds the CFL maximum); states: face states instead (see
-// k_learned_sweep)
+// the learned sweeps of one stage: the corrections of the three directions,
+// then direction after direction (the same InvDt modes as the plain sweeps: 1
+// first contribution, 2 accumulate; the last direction folds the CFL
+// maximum); states: face states instead
 static void launch_learned(Engine& e, int invdt, int fold_max, double* states) {
   LearnedModel* m = static_cast<LearnedModel*>(e.learned);
   LearnedDev L{m->Wp, m->w, m->ranged ? m->fmin : nullptr, m->ranged ? m->fmax : nullptr};
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  const LBox box = learned_box(e.g);
+  const long long tiles = (box.cells + LT - 1) / LT;
+  mark_begin(e, kKLearned);
+  k_learned_correct<<<(unsigned)(3 * tiles < e.sms ? 3 * tiles : e.sms), LN, SM_LEARN, e.stream>>>(e.g, e.f.Vc32, L, e.ctl,
+                                                                                          box, m->Y);
+  mark_end(e);
   for (int d = 0; d < 3; d++) {
     if (e.only_dir >= 0 && e.only_dir != d) continue;
-    const LTiles T = make_tiles(e.g, d);
-    const int grid = (int)(T.ntiles < sms ? T.ntiles : sms);
+    const int nt = cell_threads(e.sms, [&](int t) { return cell_tiles(e.g, d, t); });
+    const unsigned grid = (unsigned)cell_tiles(e.g, d, nt);
+    const size_t sm = cell_smem_bytes(3, nt);
     const int inv = (invdt == 0) ? 0 : (d == 0 ? invdt : 2);
     const int last = fold_max && d == 2;
+    const LearnedRecon lr{m->Y, states, m->counters};
     mark_begin(e, kKSweepX + d);
-    if (d == 0) k_learned_sweep<0><<<grid, 256, SM_LEARN, e.stream>>>(e.g, e.f, L, e.ctl, T, inv, last, states, m->counters);
-    if (d == 1) k_learned_sweep<1><<<grid, 256, SM_LEARN, e.stream>>>(e.g, e.f, L, e.ctl, T, inv, last, states, m->counters);
-    if (d == 2) k_learned_sweep<2><<<grid, 256, SM_LEARN, e.stream>>>(e.g, e.f, L, e.ctl, T, inv, last, states, m->counters);
+    if (d == 0) k_sweep_learned<0><<<grid, nt, sm, e.stream>>>(e.g, e.f, e.ctl, inv, last, lr);
+    if (d == 1) k_sweep_learned<1><<<grid, nt, sm, e.stream>>>(e.g, e.f, e.ctl, inv, last, lr);
+    if (d == 2) k_sweep_learned<2><<<grid, nt, sm, e.stream>>>(e.g, e.f, e.ctl, inv, last, lr);
     mark_end(e);
   }
 }
@@ -571,6 +482,7 @@ void free_learned(Engine& e) {
   cudaFree(m->w);
   cudaFree(m->fmin);
   cudaFree(m->fmax);
+  cudaFree(m->Y);
   cudaFree(m->counters);
   delete m;
   e.learned = nullptr;
@@ -676,12 +588,9 @@ int idfx_gpu_set_learned(idfx_gpu* hg, const float* params, const float* fmin, c
     ok = ok && cudaMalloc(&m->fmin, sizeof(float) * NIN) == cudaSuccess;
     ok = ok && cudaMalloc(&m->fmax, sizeof(float) * NIN) == cudaSuccess;
     ok = ok && cudaMalloc(&m->counters, sizeof(unsigned long long) * 2) == cudaSuccess;
-    ok = ok && cudaFuncSetAttribute(k_learned_sweep<0>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)SM_LEARN) == cudaSuccess;
-    ok = ok && cudaFuncSetAttribute(k_learned_sweep<1>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)SM_LEARN) == cudaSuccess;
-    ok = ok && cudaFuncSetAttribute(k_learned_sweep<2>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    (int)SM_LEARN) == cudaSuccess;
+    ok = ok && cudaMalloc(&m->Y, sizeof(float) * 3 * NOUT * e.g.ncell) == cudaSuccess;
+    ok = ok && cudaFuncSetAttribute(k_learned_correct, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_LEARN) ==
+                   cudaSuccess;
     if (!ok) {
       free_learned(e);
       e.err = "set_learned: CUDA allocation failed";

@@ -33,7 +33,7 @@ __host__ __device__ constexpr bool loss_masked(int o) { return o == 5 || o == 13
 
 // 3-D solver variable order: RHO, VX1..3, PRS, BX1..3.  Rotated variable r
 // of direction d -> solver variable.
-__host__ __device__ __forceinline__ int rot_var(int r, int d) {
+__host__ __device__ constexpr int rot_var(int r, int d) {
   if (r == 0 || r == 4) return r;
   const int base = (r < 4) ? 1 : 5;
   return base + (d + (r - base)) % 3;

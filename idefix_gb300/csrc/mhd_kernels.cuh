@@ -76,7 +76,7 @@ struct Fields {
   double *Ex1, *Ex2, *Ex3;
   double *ex, *ey, *ez;
   double *aL[3], *aR[3], *dL[3], *dR[3];
-  float* Vc32;  // FP32 copy of Vc read by the mixed-precision sweeps (else null)
+  float* Vc32;  // FP32 copy of Vc read by the mixed-precision sweeps and the learned correction (else null)
   unsigned char* shock;  // FlagShock per cell when shock flattening is on (else null)
 };
 

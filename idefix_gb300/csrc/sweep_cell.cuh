@@ -68,9 +68,18 @@ __host__ __device__ constexpr size_t cell_smem_bytes(int D, int nt) {
   return sizeof(double) * (size_t)((2 * D + 1) + (D + 2) + 1) * (size_t)nt;
 }
 
+// the learned order (5, 3-D): corrections Y [3][16][ncell] of the PLM states
+// (learned.cu), where the face states go instead of the sweep (or null), and
+// the counts of evaluated and fallen-back cells
+struct LearnedRecon {
+  const float* Y;
+  double* states;
+  unsigned long long* counters;
+};
+
 template <int D, int DIR, int ORDER, int SOLVER>
 __device__ __forceinline__ void d_sweep_cell(const Geo& g, const Fields& f, const Ctl* ctl, int invdt, int last_dir,
-                                             unsigned tile, double* sm) {
+                                             unsigned tile, double* sm, const LearnedRecon& lr = LearnedRecon{}) {
   if (ctl->done) return;
   using T = double;
   using v = Var<D>;
@@ -156,6 +165,54 @@ __device__ __forceinline__ void d_sweep_cell(const Geo& g, const Fields& f, cons
       for (int n = 0; n < NV; n++)
         if (n != dd::BXn) ss[(n < dd::BXn ? n : n - 1) * nt + tid] = vr[n];
     }
+  } else if constexpr (ORDER == 5) {
+    bool fall = false;
+    if (valid) {
+      T cen[NV];
+#pragma unroll
+      for (int n = 0; n < NV; n++) {
+        if (n == dd::BXn && !lr.states) continue;
+        const T w0 = f.Vc[n * g.ncell + cc - sd], w1 = f.Vc[n * g.ncell + cc], w2 = f.Vc[n * g.ncell + cc + sd];
+        cen[n] = w1;
+        Recon<2>::plm(w1, w1 - w0, w2 - w1, false, vl[n], vr[n]);
+      }
+      const T cs = root(quot(g.gamma * cen[v::PRS], cen[v::RHO])), sb = root(cen[v::RHO]) * cs;
+      const float* Y = lr.Y + (long long)DIR * 16 * g.ncell + cc;
+      T cl[NV], cr[NV];
+#pragma unroll
+      for (int rv = 0; rv < 8; rv++) {
+        if (rv == 5) continue;  // normal field: the face value is used
+        const int n = rv == 0 || rv == 4 ? rv : (rv < 4 ? 1 : 5) + (DIR + rv - (rv < 4 ? 1 : 5)) % 3;
+        const T sc = rv == 0 ? cen[v::RHO] : rv == 4 ? cen[v::PRS] : rv < 4 ? cs : sb;
+        cl[n] = vl[n] + f2d_exact(Y[rv * g.ncell]) * sc;
+        cr[n] = vr[n] + f2d_exact(Y[(8 + rv) * g.ncell]) * sc;
+      }
+      // plain PLM where the stencil is outside the trained range (a NaN) or a
+      // corrected density or pressure is not positive
+      fall = !(gt0(cl[v::RHO]) && gt0(cl[v::PRS]) && gt0(cr[v::RHO]) && gt0(cr[v::PRS]));
+#pragma unroll
+      for (int n = 0; n < NV; n++) {
+        if (n == dd::BXn) continue;
+        if (!fall) {
+          vl[n] = cl[n];
+          vr[n] = cr[n];
+        }
+        ss[(n < dd::BXn ? n : n - 1) * nt + tid] = vr[n];
+      }
+      if (lr.states) {
+#pragma unroll
+        for (int n = 0; n < NV; n++) {
+          lr.states[((long long)DIR * 16 + n) * g.ncell + cc] = vl[n];
+          lr.states[((long long)DIR * 16 + 8 + n) * g.ncell + cc] = vr[n];
+        }
+      }
+    }
+    // a position belongs to the tile it starts in; the last tile has the rest
+    const bool owner = valid && (t < npos - 2 || blockIdx.x == gridDim.x - 1);
+    const unsigned fell = __ballot_sync(0xffffffffu, owner && fall);
+    if ((tid & 31) == 0 && fell) atomicAdd(lr.counters + 1, (unsigned long long)__popc(fell));
+    if (tile == 0 && tid == 0) atomicAdd(lr.counters, (unsigned long long)nA * nB * P);
+    if (lr.states) return;
   } else if (valid) {
     const Recip l3{g.l3b[DIR], g.l3y[DIR]};
     const T dxd = g.dx[DIR];
