@@ -175,11 +175,12 @@ int upload_table(EnsEngine& e, EnsTable& t, const std::vector<int4>& items) {
   return IDFX_OK;
 }
 
-std::vector<int4> sweep_items(const EnsEngine& e, int dir, const std::vector<int>& boxes, int nt) {
+// cell: for the cell sweeps of blocks of nt threads, else for the march
+std::vector<int4> sweep_items(const EnsEngine& e, int dir, const std::vector<int>& boxes, bool cell, int nt) {
   std::vector<int4> v;
-  if (e.precision == IDFX_FP64) {  // one entry per tile of nt cells
+  if (cell) {  // one entry per tile of nt cells
     for (int b : boxes) {
-      const long long n = cell_tiles(e.boxes[b].g, dir, nt);
+      const long long n = cell_tiles(e.boxes[b].g, dir, nt, e.precision == IDFX_FP64 ? 8 : 4);
       for (long long x = 0; x < n; x++) v.push_back(make_int4(b, (int)x, 0, 0));
     }
     return v;
@@ -225,14 +226,18 @@ int build_tables(EnsEngine& e) {
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  long long cells = 0;
+  for (int b = 0; b < e.nbox; b++) cells += active_cells(e.boxes[b].g);
   for (int d = 0; d < e.D && !rc; d++) {
+    e.cell32[d] = e.precision != IDFX_FP64 && cell_sweep_wins(e.D, d, cells);
     e.cell_nt[d] = cell_threads(sms, [&](int t) {
       long long n = 0;
-      for (int b = 0; b < e.nbox; b++) n += cell_tiles(e.boxes[b].g, d, t);
+      for (int b = 0; b < e.nbox; b++) n += cell_tiles(e.boxes[b].g, d, t, e.precision == IDFX_FP64 ? 8 : 4);
       return n;
     });
-    rc = upload_table(e, e.sweep[d], sweep_items(e, d, order, e.cell_nt[d]));
-    if (!rc && e.precision == IDFX_FP64) rc = upload_table(e, e.sweep64[d], sweep_items(e, d, order, kTM));
+    const bool fp64 = e.precision == IDFX_FP64;
+    rc = upload_table(e, e.sweep[d], sweep_items(e, d, order, fp64 || e.cell32[d], e.cell_nt[d]));
+    if (!rc) rc = upload_table(e, e.sweep64[d], sweep_items(e, d, order, fp64, kTM));
   }
   return rc;
 }
@@ -446,13 +451,14 @@ int autotune(EnsEngine& e, int reps) {
     if (rc) break;
     const std::vector<int>& members = kv.second;
     for (int d = 0; d < e.D && !rc; d++) {
+      e.cell32[d] = false;  // (build_tables below decides again)
       int best_seg = e.boxes[members[0]].seg[d];
       float best_ms = 1e30f;
       for (int s = 2; s <= 64; s *= 2) {
         if (s > kv.first[d]) break;
         for (int b : members) e.boxes[b].seg[d] = s;
         rc = upload_boxes(e);
-        if (!rc) rc = upload_table(e, trial, sweep_items(e, d, members, e.cell_nt[d]));
+        if (!rc) rc = upload_table(e, trial, sweep_items(e, d, members, false, 0));
         if (rc) break;
         const float ms = time_sweep(e, d, trial, reps, ea, eb);
         if (ms < best_ms) {
@@ -520,7 +526,7 @@ EnsPersist ens_persist_args(const EnsEngine& e) {
   P.active = e.active64.items;
   P.nactive = e.active64.n;
   for (int d = 0; d < 3; d++) {
-    const EnsTable& t = e.precision == IDFX_FP64 ? e.sweep64[d] : e.sweep[d];
+    const EnsTable& t = e.sweep64[d];
     P.sweep[d] = t.items;
     P.nsweep[d] = d < e.D ? t.n : 0;
   }

@@ -61,8 +61,9 @@ struct EnsEngine {
   cudaStream_t stream = nullptr;
   bool own_stream = false;
   EnsTable fill, begin, sweep[3], edges, active;
-  EnsTable sweep64[3];                          // FP64 sweeps: tiles of 64 cells (persistent kernel)
-  int cell_nt[3] = {128, 128, 128};             // FP64 sweeps: threads of the batched launches' blocks
+  EnsTable sweep64[3];                          // the persistent kernel's sweeps: tiles of 64 cells (FP64), marches
+  bool cell32[3] = {false, false, false};       // FP32 batched sweeps with a thread per cell
+  int cell_nt[3] = {128, 128, 128};             // threads of the cell sweeps' blocks (batched launches)
   EnsTable fill64, begin64, edges64, active64;  // the same phases at 64 threads per item (persistent kernel)
   std::vector<EnsTable*> tables() {
     return {&fill, &begin, &sweep[0], &sweep[1], &sweep[2], &edges, &active, &sweep64[0], &sweep64[1],

@@ -366,10 +366,10 @@ __global__ void __launch_bounds__(LN, 1) k_learned_correct(Geo g, const float* _
 
 // the cell sweep with PLM plus the correction (sweep_cell.cuh, ORDER 5)
 template <int DIR>
-__global__ void __launch_bounds__(kCellThreads, 3)
+__global__ void __launch_bounds__(kCellThreads, cell_resident(8))
     k_sweep_learned(Geo g, Fields f, const Ctl* ctl, int invdt, int last_dir, LearnedRecon lr) {
   extern __shared__ double learned_cell_sm[];
-  d_sweep_cell<3, DIR, IDFX_LEARNED, kHLLD>(g, f, ctl, invdt, last_dir, blockIdx.x, learned_cell_sm, lr);
+  d_sweep_cell<3, DIR, IDFX_LEARNED, kHLLD, double>(g, f, ctl, invdt, last_dir, blockIdx.x, learned_cell_sm, lr);
 }
 
 __global__ void k_init_keys(unsigned* kmin, unsigned* kmax) {
@@ -459,9 +459,9 @@ static void launch_learned(Engine& e, int invdt, int fold_max, double* states) {
   mark_end(e);
   for (int d = 0; d < 3; d++) {
     if (e.only_dir >= 0 && e.only_dir != d) continue;
-    const int nt = cell_threads(e.sms, [&](int t) { return cell_tiles(e.g, d, t); });
-    const unsigned grid = (unsigned)cell_tiles(e.g, d, nt);
-    const size_t sm = cell_smem_bytes(3, nt);
+    const int nt = cell_threads(e.sms, [&](int t) { return cell_tiles(e.g, d, t, 8); });
+    const unsigned grid = (unsigned)cell_tiles(e.g, d, nt, 8);
+    const size_t sm = cell_smem_bytes(3, nt, 8);
     const int inv = (invdt == 0) ? 0 : (d == 0 ? invdt : 2);
     const int last = fold_max && d == 2;
     const LearnedRecon lr{m->Y, states, m->counters};

@@ -1,4 +1,5 @@
-// FP64 flux sweeps with one thread per cell (every direction, 2-D and 3-D).
+// Flux sweeps with one thread per cell (every direction, 2-D and 3-D): the
+// FP64 sweeps, and the FP32 sweeps of the mixed path up to a size.
 #pragma once
 #include "mhd_kernels.cuh"
 
@@ -37,12 +38,36 @@ namespace idfx {
 // changed the time by -6 to +10 %: the sweeps' instruction stream then waits on itself.
 // ---------------------------------------------------------------------------
 constexpr int kCellThreads = 128;  // largest block
+// blocks per multiprocessor that the registers allow, by the size of the arithmetic type
+__host__ __device__ constexpr int cell_resident(size_t size) { return size == 8 ? 3 : 5; }
 
-// columns side by side: lanes along x are neighbours in memory already; across
-// x, two share half a 32-byte sector and cost 2 of 64 positions (256^3 y and z
-// sweeps within 1 % of the x sweep; four columns the same there and 6 % slower
-// at 64^3, eight 4 % slower)
-__host__ __device__ constexpr int cell_cols(int dir) { return dir == 0 ? 1 : 2; }
+// whether the FP32 sweep along dir of a launch over `cells` active cells takes
+// this form; the others read each value once and win where they fill the GPU.
+// Measured, us per sweep, this form against the fastest segment of the march
+// (y, z), the tile sweep (large 3-D y, z) or the warp chunks (x):
+//   2-D x    64^2 8 / 11, 512^2 15 / 40, 2048^2 149 / 190
+//   2-D y    64^2 10 / 10, 512^2 20 / 36 (59 with the segment chosen untimed),
+//            1024^2 57 / 58 (78), 2048^2 204 / 159
+//   3-D x    32^3 10 / 11, 64^3 20 / 25, 128^3 105 / 113, 192^3 328 / 315
+//   3-D y,z  48^3 16, 17 / 15, 22 (17, 33), 64^3 24, 25 / 25, 29 (25, 63), 91 x 62 x 45
+//            PPM 40, 42 / 48, 53, 96^3 65, 67 / 42, 53
+// (across x a tile's overlap is 2 of its 16 positions.)  Ensembles the same by
+// the cells of all boxes: 20 boxes of 64^2 .. 384^2, 3 cycles 2423 -> 1911 us.
+inline bool cell_sweep_wins(int D, int dir, long long cells) {
+  if (dir == 0) return D == 2 || cells <= 1ll << 22;
+  return cells <= (D == 2 ? 1ll << 20 : 400000ll);
+}
+
+// columns side by side: lanes along x are neighbours in memory already.
+// Across x, FP64: two share half a 32-byte sector and cost 2 of 64 positions
+// (256^3 y and z sweeps within 1 % of the x sweep; four columns the same there
+// and 6 % slower at 64^3, eight 4 % slower).  FP32: half the bytes per value
+// and less arithmetic to hide them behind; eight columns of 16 positions a
+// block of 128 (128^3 y and z sweep 145 us; four columns 172, sixteen of a
+// block of 256 142 but 8 % slower at 32^3), fewer in smaller blocks.
+__host__ __device__ constexpr int cell_cols(int dir, size_t size, int nt) {
+  return dir == 0 ? 1 : size == 8 ? 2 : nt / 16;
+}
 // block size for a launch of tiles(nt) blocks of nt threads: smaller blocks
 // where fewer than two per multiprocessor would leave schedulers without a warp
 template <typename Tiles>
@@ -53,8 +78,8 @@ inline int cell_threads(int sms, Tiles tiles) {
 }
 
 // tiles of nt cells of the lines along dir
-__host__ inline long long cell_tiles(const Geo& g, int dir, int nt) {
-  const int a = (dir == 0) ? 1 : 0, b = (dir == 2) ? 1 : 2, cols = cell_cols(dir);
+__host__ inline long long cell_tiles(const Geo& g, int dir, int nt, size_t size) {
+  const int a = (dir == 0) ? 1 : 0, b = (dir == 2) ? 1 : 2, cols = cell_cols(dir, size, nt);
   const int lead = (g.order == 4) ? 1 : 0;  // PPM's extra position
   const int step = nt / cols - 2 - lead;
   const long long lines = (long long)(g.n[a] + 2 * g.ext) * (g.D == 3 ? g.n[b] + 2 * g.ext : 1);
@@ -64,8 +89,8 @@ __host__ inline long long cell_tiles(const Geo& g, int dir, int nt) {
 
 // shared memory of a block of nt threads: right-face states (PPM: before
 // them, face values and second differences), flux x area and wave speed
-__host__ __device__ constexpr size_t cell_smem_bytes(int D, int nt) {
-  return sizeof(double) * (size_t)((2 * D + 1) + (D + 2) + 1) * (size_t)nt;
+__host__ __device__ constexpr size_t cell_smem_bytes(int D, int nt, size_t size) {
+  return size * (size_t)((2 * D + 1) + (D + 2) + 1) * (size_t)nt;
 }
 
 // the learned order (5, 3-D): corrections Y [3][16][ncell] of the PLM states
@@ -77,21 +102,23 @@ struct LearnedRecon {
   unsigned long long* counters;
 };
 
-template <int D, int DIR, int ORDER, int SOLVER>
+template <int D, int DIR, int ORDER, int SOLVER, typename T>
 __device__ __forceinline__ void d_sweep_cell(const Geo& g, const Fields& f, const Ctl* ctl, int invdt, int last_dir,
-                                             unsigned tile, double* sm, const LearnedRecon& lr = LearnedRecon{}) {
+                                             unsigned tile, T* sm, const LearnedRecon& lr = LearnedRecon{}) {
   if (ctl->done) return;
-  using T = double;
   using v = Var<D>;
   using dd = Dir<D, DIR>;
   constexpr int NV = v::NV, NU = v::BX1, NS = NV - 1;
   constexpr int H = Recon<ORDER>::H;
   constexpr int E = (ORDER == 4) ? 1 : 0;
   constexpr int A = (DIR == 0) ? 1 : 0, B = (DIR == 2) ? 1 : 2;
-  constexpr int cols = cell_cols(DIR);
   const int nt = (int)blockDim.x, tid = (int)threadIdx.x;
-  double* ss = sm;            // [NS][nt] right-face states
-  double* sf = sm + NS * nt;  // [NU + 1][nt] flux x area, wave speed
+  const int cols = cell_cols(DIR, sizeof(T), nt);
+  T* ss = sm;            // [NS][nt] right-face states
+  T* sf = sm + NS * nt;  // [NU + 1][nt] flux x area, wave speed
+  const T* W;            // primitives
+  if constexpr (sizeof(T) == 8) W = f.Vc;
+  else W = f.Vc32;
   const int t = tid / cols, npos = nt / cols;
   // 32-bit indices: a position stands for a cell, of which a device holds
   // fewer than 2^31
@@ -129,7 +156,7 @@ __device__ __forceinline__ void d_sweep_cell(const Geo& g, const Fields& f, cons
         if (n == dd::BXn) continue;
         const int s = n < dd::BXn ? n : n - 1;
 #pragma unroll
-        for (int m = 0; m < 4; m++) w[n][m + 1] = f.Vc[n * g.ncell + cc + (m - 1) * sd];
+        for (int m = 0; m < 4; m++) w[n][m + 1] = W[n * g.ncell + cc + (m - 1) * sd];
         vr[n] = ppm_face(w[n][1], w[n][2], w[n][3], w[n][4]);
         ss[s * nt + tid] = vr[n];
       }
@@ -215,14 +242,14 @@ __device__ __forceinline__ void d_sweep_cell(const Geo& g, const Fields& f, cons
     if (lr.states) return;
   } else if (valid) {
     const Recip l3{g.l3b[DIR], g.l3y[DIR]};
-    const T dxd = g.dx[DIR];
+    const T dxd = (T)g.dx[DIR];
     const bool shk = f.shock && f.shock[cc];
 #pragma unroll
     for (int n = 0; n < NV; n++) {
       if (n == dd::BXn) continue;
       T w[2 * H + 1];
 #pragma unroll
-      for (int m = 0; m <= 2 * H; m++) w[m] = f.Vc[n * g.ncell + cc + (m - H) * sd];
+      for (int m = 0; m <= 2 * H; m++) w[m] = W[n * g.ncell + cc + (m - H) * sd];
       Recon<ORDER>::cell(w, dxd, n == v::RHO || n == v::PRS, vl[n], vr[n], shk, l3);
       ss[(n < dd::BXn ? n : n - 1) * nt + tid] = vr[n];
     }
@@ -238,14 +265,14 @@ __device__ __forceinline__ void d_sweep_cell(const Geo& g, const Fields& f, cons
 #pragma unroll
     for (int n = 0; n < NV; n++)
       if (n != dd::BXn) vL[n] = ss[(n < dd::BXn ? n : n - 1) * nt + tid - cols];
-    const T bn = f.Vs[DIR * g.nface + fidx(g, idx[2], idx[1], idx[0])];
+    const T bn = from_f64<T>(f.Vs[DIR * g.nface + fidx(g, idx[2], idx[1], idx[0])]);
     vL[dd::BXn] = bn;
     vl[dd::BXn] = bn;
     RiemannOut<D, T> r;
-    riemann<D, DIR, SOLVER>(g.gamma, g.rgm1, vL, vl, r);
+    riemann<D, DIR, SOLVER>((T)g.gamma, (T)g.rgm1, vL, vl, r);
     store_emf<D, DIR>(g, f, cc, r, vL, vl);
     if (active_col) {
-      const T area = g.A[DIR];
+      const T area = (T)g.A[DIR];
 #pragma unroll
       for (int n = 0; n < NU; n++) {
         FA[n] = r.F[n] * area;
@@ -259,15 +286,18 @@ __device__ __forceinline__ void d_sweep_cell(const Geo& g, const Fields& f, cons
   // ---- flux difference ------------------------------------------------
   double run_max = 0.0;
   if (update) {
-    const T dtdV = ctl->dtdV;
+    const T dtdV = (T)ctl->dtdV;
 #pragma unroll
     for (int n = 0; n < NU; n++) {
       const T rhs = -dtdV * (sf[n * nt + tid + cols] - FA[n]);
-      f.Uc[n * g.ncell + cc] = f.Uc[n * g.ncell + cc] + rhs;
+      f.Uc[n * g.ncell + cc] = f.Uc[n * g.ncell + cc] + to_f64(rhs);
     }
     if (invdt) {
       const double prev = (invdt == 1) ? 0.0 : f.InvDt[cc];
-      const double inv = prev + quot(pow2x<-1>(sf[NU * nt + tid + cols] + cm), g.dx[DIR]);
+      const T c2 = sf[NU * nt + tid + cols] + cm;
+      double inv;
+      if constexpr (sizeof(T) == 8) inv = prev + quot(pow2x<-1>(c2), g.dx[DIR]);
+      else inv = prev + to_f64(T(0.5) * c2 * (T(1) / (T)g.dx[DIR]));
       f.InvDt[cc] = inv;
       if (inv > run_max) run_max = inv;  // NaN never compares greater
     }
@@ -286,11 +316,11 @@ __device__ __forceinline__ void d_sweep_cell(const Geo& g, const Fields& f, cons
   }
 }
 
-template <int D, int DIR, int ORDER, int SOLVER>
-__global__ void __launch_bounds__(kCellThreads, 3)
+template <int D, int DIR, int ORDER, int SOLVER, typename T>
+__global__ void __launch_bounds__(kCellThreads, cell_resident(sizeof(T)))
     k_sweep_cell(Geo g, Fields f, const Ctl* ctl, int invdt, int last_dir) {
   extern __shared__ double cell_sm[];
-  d_sweep_cell<D, DIR, ORDER, SOLVER>(g, f, ctl, invdt, last_dir, blockIdx.x, cell_sm);
+  d_sweep_cell<D, DIR, ORDER, SOLVER, T>(g, f, ctl, invdt, last_dir, blockIdx.x, reinterpret_cast<T*>(cell_sm));
 }
 
 }  // namespace idfx

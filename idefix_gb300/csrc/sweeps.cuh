@@ -32,13 +32,14 @@ void launch_dir(Engine& e, int invdt, int last) {
   const int nseg = (g.n[DIR] + e.seg[DIR] - 1) / e.seg[DIR];
   const long long cols = (long long)(g.n[A] + 2 * g.ext) * (D == 3 ? g.n[B] + 2 * g.ext : 1);
   mark_begin(e, kKSweepX + DIR);
-  if constexpr (sizeof(T) == 8) {
-    const int nt = cell_threads(e.sms, [&](int t) { return cell_tiles(g, DIR, t); });
-    k_sweep_cell<D, DIR, ORDER, SOLVER><<<(unsigned)cell_tiles(g, DIR, nt), nt, cell_smem_bytes(D, nt), e.stream>>>(
-        g, e.f, e.ctl, invdt, last);
-  } else if constexpr (DIR == 0 && sizeof(T) == 4 && ORDER <= 4) {
-    // FP32 x sweep: warp chunks along each row (coalesced); staged by bulk
-    // copies when rows and arrays are 16-byte aligned
+  const long long cells = (long long)g.n[0] * g.n[1] * g.n[2];
+  if (sizeof(T) == 8 || (!e.tile[DIR] && cell_sweep_wins(D, DIR, cells))) {
+    const int nt = cell_threads(e.sms, [&](int t) { return cell_tiles(g, DIR, t, sizeof(T)); });
+    k_sweep_cell<D, DIR, ORDER, SOLVER, T><<<(unsigned)cell_tiles(g, DIR, nt, sizeof(T)), nt,
+                                             cell_smem_bytes(D, nt, sizeof(T)), e.stream>>>(g, e.f, e.ctl, invdt, last);
+  } else if constexpr (sizeof(T) == 4 && D == 3 && DIR == 0) {
+    // FP32 x sweep of a large box: warp chunks along each row (coalesced);
+    // staged by bulk copies when rows and arrays are 16-byte aligned
     const unsigned blocks = (unsigned)((cols + kXW - 1) / kXW);
     const bool aligned = g.nt[0] % 4 == 0 && (reinterpret_cast<uintptr_t>(e.f.Vc32) & 15) == 0 &&
                          (reinterpret_cast<uintptr_t>(e.f.Uc) & 15) == 0;
@@ -48,13 +49,12 @@ void launch_dir(Engine& e, int invdt, int last) {
     } else {
       k_sweep_xwarp<D, ORDER, SOLVER, T><<<blocks, 32 * kXW, 0, e.stream>>>(g, e.f, e.ctl, invdt, last);
     }
-  } else {
+  } else if constexpr (sizeof(T) == 4 && DIR > 0) {
     const SweepTileMaps* tm = nullptr;
-    if constexpr (D == 3 && DIR >= 1 && sizeof(T) == 4 && ORDER >= 2 && ORDER <= 4)
+    if constexpr (D == 3 && ORDER >= 2)
       if (e.tile[DIR]) tm = sweep_tile_maps(e);
     if (tm) {
-      if constexpr (D == 3 && DIR >= 1 && sizeof(T) == 4 && ORDER >= 2 && ORDER <= 4)
-        launch_tile<DIR, ORDER, SOLVER>(e, invdt, last, tm);
+      if constexpr (D == 3 && ORDER >= 2) launch_tile<DIR, ORDER, SOLVER>(e, invdt, last, tm);
     } else {
       dim3 grid((unsigned)((cols + kTM - 1) / kTM), nseg, 1);
       k_sweep_march<D, DIR, ORDER, SOLVER, T><<<grid, kTM, 0, e.stream>>>(g, e.f, e.ctl, invdt, last, e.seg[DIR]);
@@ -107,26 +107,27 @@ __global__ void __launch_bounds__(kTM) ke_sweep_march(const EnsBox* boxes, const
   d_sweep_march<D, DIR, ORDER, SOLVER, T>(B.g, B.f, B.ctl, invdt, last, B.seg[DIR], dim3(it.y, it.z, it.w));
 }
 
-template <int D, int DIR, int ORDER, int SOLVER>
-__global__ void __launch_bounds__(kCellThreads, 3)
+template <int D, int DIR, int ORDER, int SOLVER, typename T>
+__global__ void __launch_bounds__(kCellThreads, cell_resident(sizeof(T)))
     ke_sweep_cell(const EnsBox* boxes, const int4* items, int invdt, int last) {
   extern __shared__ double ens_cell_sm[];
   const int4 it = items[blockIdx.x];
   const EnsBox& B = boxes[it.x];
-  d_sweep_cell<D, DIR, ORDER, SOLVER>(B.g, B.f, B.ctl, invdt, last, (unsigned)it.y, ens_cell_sm);
+  d_sweep_cell<D, DIR, ORDER, SOLVER, T>(B.g, B.f, B.ctl, invdt, last, (unsigned)it.y,
+                                          reinterpret_cast<T*>(ens_cell_sm));
 }
 
 template <int D, int ORDER, int SOLVER, typename T>
 void launch_ens_dir(EnsEngine& e, int dir, const EnsTable& t, int invdt, int last) {
   if (t.n == 0) return;
-  if constexpr (sizeof(T) == 8) {
+  if (sizeof(T) == 8 || e.cell32[dir]) {
     const int nt = e.cell_nt[dir];
-    const size_t sm = cell_smem_bytes(D, nt);
-    if (dir == 0) ke_sweep_cell<D, 0, ORDER, SOLVER><<<t.n, nt, sm, e.stream>>>(e.d_boxes, t.items, invdt, last);
-    if (dir == 1) ke_sweep_cell<D, 1, ORDER, SOLVER><<<t.n, nt, sm, e.stream>>>(e.d_boxes, t.items, invdt, last);
+    const size_t sm = cell_smem_bytes(D, nt, sizeof(T));
+    if (dir == 0) ke_sweep_cell<D, 0, ORDER, SOLVER, T><<<t.n, nt, sm, e.stream>>>(e.d_boxes, t.items, invdt, last);
+    if (dir == 1) ke_sweep_cell<D, 1, ORDER, SOLVER, T><<<t.n, nt, sm, e.stream>>>(e.d_boxes, t.items, invdt, last);
     if constexpr (D == 3)
-      if (dir == 2) ke_sweep_cell<D, 2, ORDER, SOLVER><<<t.n, nt, sm, e.stream>>>(e.d_boxes, t.items, invdt, last);
-  } else {
+      if (dir == 2) ke_sweep_cell<D, 2, ORDER, SOLVER, T><<<t.n, nt, sm, e.stream>>>(e.d_boxes, t.items, invdt, last);
+  } else if constexpr (sizeof(T) == 4) {
     if (dir == 0) ke_sweep_march<D, 0, ORDER, SOLVER, T><<<t.n, kTM, 0, e.stream>>>(e.d_boxes, t.items, invdt, last);
     if (dir == 1) ke_sweep_march<D, 1, ORDER, SOLVER, T><<<t.n, kTM, 0, e.stream>>>(e.d_boxes, t.items, invdt, last);
     if constexpr (D == 3)
@@ -210,7 +211,7 @@ template <int D, int ORDER, int SOLVER, typename T>
 __global__ void __launch_bounds__(kTM, sizeof(T) == 8 ? 6 : 1)
     ke_persistent(const EnsBox* boxes, EnsPersist P, int ncyc, GridBar* bar) {
   using E = T;  // EMF buffers in the arithmetic type of the sweeps
-  __shared__ double cell_sm[sizeof(T) == 8 ? cell_smem_bytes(D, kTM) / sizeof(double) : 1];
+  __shared__ double cell_sm[sizeof(T) == 8 ? cell_smem_bytes(D, kTM, 8) / sizeof(double) : 1];
   const int stride = (int)gridDim.x;
   const int tstride = stride * (int)blockDim.x;
   const int t0 = blockIdx.x * blockDim.x + threadIdx.x;
@@ -265,10 +266,10 @@ __global__ void __launch_bounds__(kTM, sizeof(T) == 8 ? 6 : 1)
           const int4 it = P.sweep[d][i];
           const EnsBox& B = boxes[it.x];
           if constexpr (sizeof(T) == 8) {
-            if (d == 0) d_sweep_cell<D, 0, ORDER, SOLVER>(B.g, B.f, B.ctl, invdt, last, (unsigned)it.y, cell_sm);
-            if (d == 1) d_sweep_cell<D, 1, ORDER, SOLVER>(B.g, B.f, B.ctl, invdt, last, (unsigned)it.y, cell_sm);
+            if (d == 0) d_sweep_cell<D, 0, ORDER, SOLVER, T>(B.g, B.f, B.ctl, invdt, last, (unsigned)it.y, cell_sm);
+            if (d == 1) d_sweep_cell<D, 1, ORDER, SOLVER, T>(B.g, B.f, B.ctl, invdt, last, (unsigned)it.y, cell_sm);
             if constexpr (D == 3)
-              if (d == 2) d_sweep_cell<D, 2, ORDER, SOLVER>(B.g, B.f, B.ctl, invdt, last, (unsigned)it.y, cell_sm);
+              if (d == 2) d_sweep_cell<D, 2, ORDER, SOLVER, T>(B.g, B.f, B.ctl, invdt, last, (unsigned)it.y, cell_sm);
             __syncthreads();  // the next item's states go where this one's were read
           } else {
             if (d == 0) d_sweep_march<D, 0, ORDER, SOLVER, T>(B.g, B.f, B.ctl, invdt, last, B.seg[0], dd(it));
