@@ -79,6 +79,22 @@ IDFX_HD double half_of(double x) {
   return rare_mul(0.5, x);
 }
 
+// x[A] .. x[B - 1] halved; false, and some of x left undefined, where one of
+// them is neither zero nor far enough from the ends of the exponent range: one
+// rare branch for all of them
+template <int A, int B>
+IDFX_HD bool halve(double* x) {
+  bool ok = true;
+#pragma unroll
+  for (int n = A; n < B; n++) {
+    const uint64_t u = dbits(x[n]);
+    const uint32_t e = (uint32_t)(u >> 52) & 0x7ffu;
+    ok = ok && (e - 64u < 1920u || (u << 1) == 0ull);
+    x[n] = dfrom(e == 0u ? u : u - (1ull << 52));
+  }
+  return ok;
+}
+
 // x 2^K: on the FP64 path an add to the exponent field (the FP64 pipe is what
 // the sweeps wait for), zeros as they are, and the product, as a call, where
 // the result could leave the normal range; FP32 the product
@@ -202,6 +218,37 @@ IDFX_HD E upwind_term(E w, E a, E b) {
   } else {
     return (E(1) - w) * a + w * b;
   }
+}
+
+// upwind_term of the differences xa - ya and xb - yb.  FP64 path: for a weight
+// of 0 or 1 (away from stagnant faces) the term is the picked difference, so
+// only that one issues on the FP64 pipe - one operation instead of three; a
+// zero difference (its sign would depend on the other's), a non-finite value on the
+// other side (0 times it is NaN) and the weight 1/2 take the whole term, as a call.
+IDFX_RARE double upwind_whole(double w, double xa, double ya, double xb, double yb) {
+  return upwind_term(w, xa - ya, xb - yb);
+}
+template <typename E>
+IDFX_HD E upwind_diff(E w, E xa, E ya, E xb, E yb) {
+  if constexpr (sizeof(E) == 8) {
+    const uint64_t W = dbits(w);
+    const bool one = W == 0x3FF0000000000000ull;
+    const double d = (one ? xb : xa) - (one ? yb : ya);
+    const uint64_t ox = dbits(one ? xa : xb) << 1, oy = dbits(one ? ya : yb) << 1, F = 0x7FDull << 53;
+    if ((one || W == 0ull) && ox < F && oy < F && (dbits(d) << 1) != 0ull) return d;
+    return upwind_whole(w, xa, ya, xb, yb);
+  } else {
+    return upwind_term(w, xa - ya, xb - yb);
+  }
+}
+
+// x / 4, the product's value
+IDFX_HD float quarter(float x) { return 0.25f * x; }
+IDFX_HD double quarter(double x) {
+  const uint64_t u = dbits(x);
+  if (((uint32_t)(u >> 52) & 0x7ffu) - 64u < 1920u) return dfrom(u - (2ull << 52));
+  if ((u << 1) == 0ull) return x;
+  return rare_mul(0.25, x);
 }
 
 }  // namespace idfx

@@ -7,9 +7,10 @@
 // patterns (IEEE-754 binary32 / binary64 layouts):
 //   f2d_exact: binary32 -> binary64, exact (a rebias of the exponent and a
 //              shift of the significand);
-//   d2f_rn:    binary64 -> binary32, round to nearest, ties to even (the 29
-//              dropped significand bits decide; a carry out of the significand
-//              moves into the exponent, up to infinity as IEEE rounding does).
+//   d2f_rn:    binary64 -> binary32, round to nearest, ties to even (half a
+//              unit added before the 29 low significand bits are dropped; a
+//              carry out of the significand moves into the exponent, up to
+//              infinity as IEEE rounding does).
 // Zeros take the integer path too; subnormal, infinite and NaN operands (and
 // binary64 values outside the binary32 normal range) take the hardware
 // conversion.  Both are checked bit for bit against the host's and CUDA's
@@ -43,29 +44,23 @@ IDFX_HD float ffrom(uint32_t u) {
 }
 
 IDFX_HD double f2d_exact(float x) {
-  const uint32_t u = fbits(x);
-  const uint32_t e = (u >> 23) & 0xffu;
-  const uint64_t s = (uint64_t)(u & 0x80000000u) << 32;
-  if (e - 1u < 254u) return dfrom(s | ((uint64_t)(e + 896u) << 52) | ((uint64_t)(u & 0x7fffffu) << 29));
-  if ((u & 0x7fffffffu) == 0u) return dfrom(s);
-  return (double)x;
+  const uint32_t u = fbits(x), t = u & 0x7fffffffu, s = u & 0x80000000u;
+  if (t - 0x00800000u < 0x7f000000u) return dfrom(((uint64_t)(s | ((t >> 3) + (896u << 20))) << 32) | (u << 29));
+  if (t == 0u) return dfrom((uint64_t)s << 32);
+  return rare_widen(x);
 }
 
 IDFX_HD float d2f_rn(double x) {
   const uint64_t u = dbits(x);
-  const uint32_t e = (uint32_t)(u >> 52) & 0x7ffu;
   const uint32_t s = (uint32_t)(u >> 32) & 0x80000000u;
   // binary32 normal range: biased exponent 1..254 <=> binary64 897..1150
-  if (e - 897u < 254u) {
-    const uint64_t m = u & ((1ull << 52) - 1ull);
-    const uint32_t rest = (uint32_t)m & ((1u << 29) - 1u);
-    uint32_t r = ((e - 896u) << 23) | (uint32_t)(m >> 29);
-    const uint32_t half = 1u << 28;
-    if (rest > half || (rest == half && (r & 1u))) r += 1u;
-    return ffrom(s | r);
+  if (((uint32_t)(u >> 52) & 0x7ffu) - 897u < 254u) {
+    // half a unit of the last place kept, less one bit where that place is even
+    const uint64_t r = u + ((1u << 28) - 1u + ((uint32_t)(u >> 29) & 1u));
+    return ffrom(s | (((uint32_t)(r >> 29) - (896u << 23)) & 0x7fffffffu));
   }
   if ((u << 1) == 0ull) return ffrom(s);
-  return (float)x;
+  return rare_narrow(x);
 }
 
 }  // namespace idfx

@@ -12,11 +12,11 @@
 //     two Newton-Raphson steps R <- R + R (2^116 - x R) / 2^116 in 64/128-bit
 //     fixed point (quadratic convergence: 2^-21 -> 2^-42 -> 2^-63);
 //   * the quotient estimate q = floor(m R / 2^64) of the dividend
-//     significand m (scaled so that m / x is in [1, 2)) is within a few
-//     units of floor(m 2^52 / x); the exact remainder m 2^52 - q x (it fits
+//     significand m (scaled so that m / x is in [1, 2)) is within one unit
+//     of floor(m 2^52 / x); the exact remainder m 2^52 - q x (it fits
 //     in 64 bits) corrects it, and rounds to nearest even.
-// Operands that are zero, subnormal, infinite or NaN, and quotients outside
-// the normal exponent range, take the hardware division.
+// Subnormal, infinite and NaN operands, zero divisors and quotients outside
+// the normal exponent range take the hardware division.
 // Written for this
 // project from the textbook method (Newton-Raphson reciprocal refinement
 // followed by an exact remainder correction, as in J.-M. Muller et al.,
@@ -49,6 +49,8 @@ IDFX_RARE double rare_mul(double a, double b) { return a * b; }
 IDFX_RARE double rare_add(double a, double b) { return a + b; }
 IDFX_RARE double rare_div(double a, double b) { return a / b; }
 IDFX_RARE double rare_sqrt(double a) { return sqrt(a); }
+IDFX_RARE double rare_widen(float a) { return (double)a; }
+IDFX_RARE float rare_narrow(double a) { return (float)a; }
 
 IDFX_HD uint64_t umulhi64(uint64_t a, uint64_t b) {
 #ifdef __CUDA_ARCH__
@@ -106,8 +108,12 @@ IDFX_HD uint64_t nr_step(uint64_t x, uint64_t R) {
 IDFX_HD double div_rn(double a, double b) {
   const uint64_t A = dbits(a), B = dbits(b);
   const uint32_t ea = (uint32_t)(A >> 52) & 0x7ffu, eb = (uint32_t)(B >> 52) & 0x7ffu;
-  // zero, subnormal, infinite or NaN operands
-  if (ea - 1u >= 2046u || eb - 1u >= 2046u) return a / b;
+  // subnormal, infinite or NaN operands; zero dividends (states at rest) are
+  // common and need no division
+  if (ea - 1u >= 2046u || eb - 1u >= 2046u) {
+    if ((A << 1) == 0ull && eb - 1u < 2046u) return dfrom((A ^ B) & (1ull << 63));
+    return rare_div(a, b);
+  }
   const uint64_t H = 1ull << 52, M = H - 1ull;
   uint64_t m = (A & M) | H;
   const uint64_t x = (B & M) | H;
@@ -117,7 +123,7 @@ IDFX_HD double div_rn(double a, double b) {
     e -= 1;
   }
   // the quotient's biased exponent must leave room for a rounding carry
-  if ((uint32_t)(e - 1) >= 2045u) return a / b;
+  if ((uint32_t)(e - 1) >= 2045u) return rare_div(a, b);
   const uint64_t sign = (A ^ B) & (1ull << 63);
   uint64_t q;
   int64_t rem;
@@ -141,18 +147,17 @@ IDFX_HD double div_rn(double a, double b) {
     R = nr_step(x, R);
     q = umulhi64(m, R);
     rem = (int64_t)((m << 52) - q * x);
-    // bring the remainder into [0, x)
-    for (int k = 0; k < 2; k++)
-      if (rem < 0) {
-        rem += (int64_t)x;
-        q -= 1;
-      }
-    for (int k = 0; k < 4; k++)
-      if (rem >= (int64_t)x) {
-        rem -= (int64_t)x;
-        q += 1;
-      }
-    if (rem < 0 || rem >= (int64_t)x) return a / b;  // not reached
+    // R is within three units of 2^116 / x, so m R / 2^64 within 0.003 of the
+    // quotient and q within one of its floor: the remainder into [0, x)
+    if (rem < 0) {
+      rem += (int64_t)x;
+      q -= 1;
+    }
+    if (rem >= (int64_t)x) {
+      rem -= (int64_t)x;
+      q += 1;
+    }
+    if (rem < 0 || rem >= (int64_t)x) return rare_div(a, b);  // not reached
   }
   // round to nearest, ties to even
   const uint64_t twice = (uint64_t)rem << 1;

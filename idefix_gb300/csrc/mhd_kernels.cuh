@@ -89,6 +89,12 @@ template <typename E>
 __device__ __forceinline__ const E* emf(const double* p) {
   return reinterpret_cast<const E*>(p);
 }
+// a thread's number within the blocks bid.x of one grid row: 32 bits (cells and
+// faces of a box number fewer than 2^31 - a device holds 7 x 10^8 - and a
+// 64-bit division by a runtime extent is some hundred instructions where a
+// 32-bit one is twenty)
+__device__ __forceinline__ unsigned thread_index(dim3 bid) { return bid.x * blockDim.x + threadIdx.x; }
+
 // FP32 <-> FP64 on the integer pipe (fpconv.cuh); identity for doubles
 template <typename T>
 __device__ __forceinline__ double to_f64(T x) {
@@ -136,11 +142,11 @@ constexpr int kPrefetch = 4;  // steps ahead of the FP32 march
 template <int D>
 __device__ __forceinline__ void d_fill_faces(const Geo& g, const Fields& f, const Ctl* ctl, int save_begin, dim3 bid) {
   if (ctl->done) return;
-  const long long tid = (long long)bid.x * blockDim.x + threadIdx.x;
+  const unsigned tid = thread_index(bid);
   const int comp = bid.y;
   if (tid >= g.nface) return;
   int i = (int)(tid % g.ntv[0]);
-  long long r = tid / g.ntv[0];
+  unsigned r = tid / g.ntv[0];
   int j = (int)(r % g.ntv[1]);
   int k = (int)(r / g.ntv[1]);
   const int idx3[3] = {i, j, k};
@@ -183,11 +189,11 @@ __device__ __forceinline__ void d_fill_face_ghosts(const Geo& g, const Fields& f
   const int a = (dir == 0) ? 1 : 0, b = (dir == 2) ? 1 : 2;
   int ext[3];  // the face box of component comp without its padding
   for (int d = 0; d < 3; d++) ext[d] = (d < D) ? (d == comp ? g.nt[d] + 1 : g.nt[d]) : 1;
-  const long long per_side = (long long)g.ng * ext[a] * ext[b];
-  const long long tid = (long long)bid.x * blockDim.x + threadIdx.x;
-  if (tid >= 2 * per_side) return;
+  const unsigned per_side = (unsigned)g.ng * ext[a] * ext[b];
+  const unsigned tid = thread_index(bid);
+  if (tid >= 2u * per_side) return;
   const int side = (int)(tid / per_side);
-  long long r = tid % per_side;
+  unsigned r = tid % per_side;
   const int layer = (int)(r % g.ng);
   r /= g.ng;
   int idx[3];
@@ -307,10 +313,10 @@ __device__ __forceinline__ void stage_begin_cell(const Geo& g, const Fields& f, 
 template <int D, typename E = double>
 __device__ __forceinline__ void d_stage_begin(const Geo& g, const Fields& f, const Ctl* ctl, int flags, dim3 bid) {
   if (ctl->done) return;
-  const long long c = (long long)bid.x * blockDim.x + threadIdx.x;
+  const unsigned c = thread_index(bid);
   if (c >= g.ncell) return;
   const int i = (int)(c % g.nt[0]);
-  const long long r = c / g.nt[0];
+  const unsigned r = c / g.nt[0];
   const int j = (int)(r % g.nt[1]);
   const int k = (int)(r / g.nt[1]);
   stage_begin_cell<D, E>(g, f, ctl, flags, i, j, k);
@@ -327,11 +333,11 @@ __device__ __forceinline__ void d_stage_ghosts(const Geo& g, const Fields& f, co
   const int dir = bid.y;
   if (dir >= D) return;
   const int a = (dir == 0) ? 1 : 0, b = (dir == 2) ? 1 : 2;
-  const long long tid = (long long)bid.x * blockDim.x + threadIdx.x;
-  const long long per_side = (long long)g.ng * g.nt[a] * g.nt[b];
-  if (tid >= 2 * per_side) return;
+  const unsigned tid = thread_index(bid);
+  const unsigned per_side = (unsigned)g.ng * g.nt[a] * g.nt[b];
+  if (tid >= 2u * per_side) return;
   const int side = (int)(tid / per_side);
-  long long r = tid % per_side;
+  unsigned r = tid % per_side;
   const int layer = (int)(r % g.ng);
   r /= g.ng;
   const int ia = (int)(r % g.nt[a]);
@@ -384,11 +390,11 @@ __device__ __forceinline__ void d_bc_slab(const Geo& g, const Fields& f, const C
   if (ctl->done) return;
   using v = Var<D>;
   const int a = (dir == 0) ? 1 : 0, b = (dir == 2) ? 1 : 2;  // the two other directions
-  const long long tid = (long long)bid.x * blockDim.x + threadIdx.x;
-  const long long per_side = (long long)g.ng * g.ntv[a] * g.ntv[b];
-  if (tid >= 2 * per_side) return;
+  const unsigned tid = thread_index(bid);
+  const unsigned per_side = (unsigned)g.ng * g.ntv[a] * g.ntv[b];
+  if (tid >= 2u * per_side) return;
   const int side = (int)(tid / per_side);
-  long long r = tid - side * per_side;
+  unsigned r = tid - side * per_side;
   const int depth = (int)(r % g.ng);
   r /= g.ng;
   const int ia = (int)(r % g.ntv[a]);
@@ -442,7 +448,7 @@ template <int D>
 __device__ __forceinline__ void d_normal_field(const Geo& g, const Fields& f, const Ctl* ctl, int dir, dim3 bid) {
   if (ctl->done) return;
   const int a = (dir == 0) ? 1 : 0, b = (dir == 2) ? 1 : 2;
-  const long long tid = (long long)bid.x * blockDim.x + threadIdx.x;
+  const unsigned tid = thread_index(bid);
   if (tid >= (long long)g.nt[a] * g.nt[b]) return;
   const int ia = (int)(tid % g.nt[a]), ib = (int)(tid / g.nt[a]);
   const bool left = g.bc[dir][0] != 0, right = g.bc[dir][1] != 0;
@@ -515,7 +521,7 @@ __device__ __forceinline__ void d_find_shock(const Geo& g, const Fields& f, cons
   if (ctl->done) return;
   using v = Var<D>;
   const int m0 = g.n[0] + 2, m1 = g.n[1] + 2, m2 = (D == 3) ? g.n[2] + 2 : 1;
-  const long long tid = (long long)bid.x * blockDim.x + threadIdx.x;
+  const unsigned tid = thread_index(bid);
   if (tid >= (long long)m0 * m1 * m2) return;
   const int i = g.beg[0] - 1 + (int)(tid % m0);
   const int j = g.beg[1] - 1 + (int)((tid / m0) % m1);
@@ -1359,29 +1365,28 @@ __device__ __forceinline__ void corner_emfs_avg(int emf_mode, Get get, E& exv, E
   // uct_contact (calcCornerEmf.hpp:224-282)
   auto wsx = [&](int di, int dj, int dk) { return get(kEaSx, di, dj, dk); };
   auto wsy = [&](int di, int dj, int dk) { return get(kEaSy, di, dj, dk); };
-  const E q4 = E(0.25);
   if constexpr (CZ) {
-    const E ez_l2 = upwind_term(wsx(0, -1, 0), ezj(0, 0, 0) - Ex3(0, -1, 0), ezj(-1, 0, 0) - Ex3(-1, -1, 0));
-    const E ez_r2 = upwind_term(wsx(0, 0, 0), ezj(0, 0, 0) - Ex3(0, 0, 0), ezj(-1, 0, 0) - Ex3(-1, 0, 0));
-    const E ez_l1 = upwind_term(wsy(-1, 0, 0), ezi(0, 0, 0) - Ex3(-1, 0, 0), ezi(0, -1, 0) - Ex3(-1, -1, 0));
-    const E ez_r1 = upwind_term(wsy(0, 0, 0), ezi(0, 0, 0) - Ex3(0, 0, 0), ezi(0, -1, 0) - Ex3(0, -1, 0));
-    ezv = q4 * (ez_l2 + ez_r2 + ez_l1 + ez_r1 + ezi(0, 0, 0) + ezi(0, -1, 0) + ezj(0, 0, 0) + ezj(-1, 0, 0));
+    const E ez_l2 = upwind_diff(wsx(0, -1, 0), ezj(0, 0, 0), Ex3(0, -1, 0), ezj(-1, 0, 0), Ex3(-1, -1, 0));
+    const E ez_r2 = upwind_diff(wsx(0, 0, 0), ezj(0, 0, 0), Ex3(0, 0, 0), ezj(-1, 0, 0), Ex3(-1, 0, 0));
+    const E ez_l1 = upwind_diff(wsy(-1, 0, 0), ezi(0, 0, 0), Ex3(-1, 0, 0), ezi(0, -1, 0), Ex3(-1, -1, 0));
+    const E ez_r1 = upwind_diff(wsy(0, 0, 0), ezi(0, 0, 0), Ex3(0, 0, 0), ezi(0, -1, 0), Ex3(0, -1, 0));
+    ezv = quarter(ez_l2 + ez_r2 + ez_l1 + ez_r1 + ezi(0, 0, 0) + ezi(0, -1, 0) + ezj(0, 0, 0) + ezj(-1, 0, 0));
   }
   if constexpr (D == 3) {
     auto wsz = [&](int di, int dj, int dk) { return get(kEaSz, di, dj, dk); };
     if constexpr (CX) {
-      const E ex_l3 = upwind_term(wsy(0, 0, -1), exk(0, 0, 0) - Ex1(0, 0, -1), exk(0, -1, 0) - Ex1(0, -1, -1));
-      const E ex_r3 = upwind_term(wsy(0, 0, 0), exk(0, 0, 0) - Ex1(0, 0, 0), exk(0, -1, 0) - Ex1(0, -1, 0));
-      const E ex_l2 = upwind_term(wsz(0, -1, 0), exj(0, 0, 0) - Ex1(0, -1, 0), exj(0, 0, -1) - Ex1(0, -1, -1));
-      const E ex_r2 = upwind_term(wsz(0, 0, 0), exj(0, 0, 0) - Ex1(0, 0, 0), exj(0, 0, -1) - Ex1(0, 0, -1));
-      exv = q4 * (ex_l3 + ex_r3 + ex_l2 + ex_r2 + exj(0, 0, 0) + exj(0, 0, -1) + exk(0, 0, 0) + exk(0, -1, 0));
+      const E ex_l3 = upwind_diff(wsy(0, 0, -1), exk(0, 0, 0), Ex1(0, 0, -1), exk(0, -1, 0), Ex1(0, -1, -1));
+      const E ex_r3 = upwind_diff(wsy(0, 0, 0), exk(0, 0, 0), Ex1(0, 0, 0), exk(0, -1, 0), Ex1(0, -1, 0));
+      const E ex_l2 = upwind_diff(wsz(0, -1, 0), exj(0, 0, 0), Ex1(0, -1, 0), exj(0, 0, -1), Ex1(0, -1, -1));
+      const E ex_r2 = upwind_diff(wsz(0, 0, 0), exj(0, 0, 0), Ex1(0, 0, 0), exj(0, 0, -1), Ex1(0, 0, -1));
+      exv = quarter(ex_l3 + ex_r3 + ex_l2 + ex_r2 + exj(0, 0, 0) + exj(0, 0, -1) + exk(0, 0, 0) + exk(0, -1, 0));
     }
     if constexpr (CY) {
-      const E ey_l3 = upwind_term(wsx(0, 0, -1), eyk(0, 0, 0) - Ex2(0, 0, -1), eyk(-1, 0, 0) - Ex2(-1, 0, -1));
-      const E ey_r3 = upwind_term(wsx(0, 0, 0), eyk(0, 0, 0) - Ex2(0, 0, 0), eyk(-1, 0, 0) - Ex2(-1, 0, 0));
-      const E ey_l1 = upwind_term(wsz(-1, 0, 0), eyi(0, 0, 0) - Ex2(-1, 0, 0), eyi(0, 0, -1) - Ex2(-1, 0, -1));
-      const E ey_r1 = upwind_term(wsz(0, 0, 0), eyi(0, 0, 0) - Ex2(0, 0, 0), eyi(0, 0, -1) - Ex2(0, 0, -1));
-      eyv = q4 * (ey_l3 + ey_r3 + ey_l1 + ey_r1 + eyi(0, 0, 0) + eyi(0, 0, -1) + eyk(0, 0, 0) + eyk(-1, 0, 0));
+      const E ey_l3 = upwind_diff(wsx(0, 0, -1), eyk(0, 0, 0), Ex2(0, 0, -1), eyk(-1, 0, 0), Ex2(-1, 0, -1));
+      const E ey_r3 = upwind_diff(wsx(0, 0, 0), eyk(0, 0, 0), Ex2(0, 0, 0), eyk(-1, 0, 0), Ex2(-1, 0, 0));
+      const E ey_l1 = upwind_diff(wsz(-1, 0, 0), eyi(0, 0, 0), Ex2(-1, 0, 0), eyi(0, 0, -1), Ex2(-1, 0, -1));
+      const E ey_r1 = upwind_diff(wsz(0, 0, 0), eyi(0, 0, 0), Ex2(0, 0, 0), eyi(0, 0, -1), Ex2(0, 0, -1));
+      eyv = quarter(ey_l3 + ey_r3 + ey_l1 + ey_r1 + eyi(0, 0, 0) + eyi(0, 0, -1) + eyk(0, 0, 0) + eyk(-1, 0, 0));
     }
   }
 }
@@ -1448,11 +1453,11 @@ template <int D, typename E = double>
 __device__ __forceinline__ void d_ct_corner(const Geo& g, const Fields& f, const Ctl* ctl, dim3 bid) {
   if (ctl->done) return;
   const int nx = g.n[0] + 1, ny = g.n[1] + 1;
-  const long long tid = (long long)bid.x * blockDim.x + threadIdx.x;
+  const unsigned tid = thread_index(bid);
   const long long tot = (long long)nx * ny * (D == 3 ? g.n[2] + 1 : 1);
   if (tid >= tot) return;
   const int i = g.beg[0] + (int)(tid % nx);
-  const long long r = tid / nx;
+  const unsigned r = tid / nx;
   const int j = g.beg[1] + (int)(r % ny);
   const int k = (D == 3) ? g.beg[2] + (int)(r / ny) : 0;
   const long long c = cidx(g, k, j, i);
@@ -1465,8 +1470,12 @@ __device__ __forceinline__ void d_ct_corner(const Geo& g, const Fields& f, const
   emf<E>(f.ez)[c] = ezv;
 }
 
+// FP64 path: bound by the FP64 pipe (77 % busy); with the upwind side picked
+// before the difference (upwind_diff) and the quarter off that pipe 46 operations
+// per cell instead of 61, 256^3 3.91 -> 3.19 ms for both stages.  At least three
+// blocks per multiprocessor: two ran 4.52 instead of 3.91 ms.
 template <int D, typename E = double>
-__global__ void k_ct_corner(Geo g, Fields f, const Ctl* ctl) {
+__global__ void __launch_bounds__(256, 3) k_ct_corner(Geo g, Fields f, const Ctl* ctl) {
   d_ct_corner<D, E>(g, f, ctl, blockIdx);
 }
 
@@ -1484,13 +1493,17 @@ __global__ void k_ct_corner(Geo g, Fields f, const Ctl* ctl) {
 // blocks: the next cycle's face fill then passes over the ghosts alone)
 enum { kCtCombine = 1, kCtSaveBegin = 2 };
 
+// (weights compared by their bits: a comparison of doubles takes the FP64 pipe
+// for every thread and face.  256^3, both stages: the FP64 face update 1.53 ->
+// 1.34 ms, the mixed path's fused corner and face pass 1.45 -> 1.34 ms, and 1.30
+// with the shorter widening of its EMFs)
 template <typename E>
 __device__ __forceinline__ double rk_combine(double u, double u0, double wc, double w0) {
   if constexpr (sizeof(E) == 4) {
     // RK2's 1/2 (u + u0): the halving exact on the integer pipe
-    if (wc == w0) return wc == 0.5 ? half_of(u + u0) : wc * (u + u0);
+    if (dbits(wc) == dbits(w0)) return dbits(wc) == dbits(0.5) ? half_of(u + u0) : wc * (u + u0);
   }
-  if (wc == 0.5 && w0 == 0.5) return pow2x<-1>(u) + pow2x<-1>(u0);  // the products exact on the integer pipe
+  if (dbits(wc) == dbits(0.5) && dbits(w0) == dbits(0.5)) return pow2x<-1>(u) + pow2x<-1>(u0);  // the products exact on the integer pipe
   return wc * u + w0 * u0;
 }
 
@@ -1580,11 +1593,11 @@ template <int D, typename E = double>
 __device__ __forceinline__ void d_ct_faces(const Geo& g, const Fields& f, const Ctl* ctl, int combine, double wc, double w0, dim3 bid) {
   if (ctl->done) return;
   const int nx = g.n[0] + 1, ny = g.n[1] + 1;
-  const long long tid = (long long)bid.x * blockDim.x + threadIdx.x;
+  const unsigned tid = thread_index(bid);
   const long long tot = (long long)nx * ny * (D == 3 ? g.n[2] + 1 : 1);
   if (tid >= tot) return;
   const int i = g.beg[0] + (int)(tid % nx);
-  const long long r = tid / nx;
+  const unsigned r = tid / nx;
   const int j = g.beg[1] + (int)(r % ny);
   const int k = (D == 3) ? g.beg[2] + (int)(r / ny) : 0;
   const long long c = cidx(g, k, j, i);
@@ -1760,43 +1773,44 @@ __global__ void __launch_bounds__(kCtTI * kCtTJ, 3) k_ct_fused(Geo g, Fields f, 
 // path's sweeps and stage begins read the hydro variables of Uc alone; the
 // host rebuilds the field part from the faces before it hands Uc out).
 enum { kSeOutputs = 16, kSeSaveBegin = 32, kSeNoUcField = 64 };
-template <int D, typename E = double>
-__device__ __forceinline__ void d_stage_end(const Geo& g, const Fields& f, const Ctl* ctl, int combine, double wc,
-                                            double w0, dim3 bid, int out = 0) {
-  if (ctl->done) return;
+// half of a sum, or the sum of the halves, of any values
+IDFX_RARE double stage_rare(double a, double b, int of_sum) { return of_sum ? 0.5 * (a + b) : 0.5 * a + 0.5 * b; }
+// RK: 0 no combination, 1 RK2's 1/2 u + 1/2 u0, 2 wc u + w0 u0
+template <int D, typename E, int RK>
+__device__ __forceinline__ void stage_end_cell(const Geo& g, const Fields& f, double wc, double w0, long long c,
+                                               long long fc, int out) {
   using v = Var<D>;
   constexpr int NV = v::NV;
-  const long long tid = (long long)bid.x * blockDim.x + threadIdx.x;
-  const long long tot = (long long)g.n[0] * g.n[1] * (D == 3 ? g.n[2] : 1);
-  if (tid >= tot) return;
-  const int i = g.beg[0] + (int)(tid % g.n[0]);
-  const long long r = tid / g.n[0];
-  const int j = g.beg[1] + (int)(r % g.n[1]);
-  const int k = (D == 3) ? g.beg[2] + (int)(r / g.n[1]) : 0;
-  const long long c = cidx(g, k, j, i);
-  const long long fc = fidx(g, k, j, i);
-  if (tid == 0) ((Ctl*)ctl)->uc_fresh = 1;  // read by the next stage begin
   double U[NV], V[NV];
 #pragma unroll
   for (int n = 0; n < v::BX1; n++) {
     double u = f.Uc[n * g.ncell + c];
-    if (combine) {
-      // (this pass is not bound by the FP64 pipe: rk_combine's halves on the
-      // integer pipe made it 2.09 instead of 1.99 ms per 256^3 cycle, and 2.19
-      // instead of 1.96 on the mixed path)
+    if constexpr (RK != 0) {
       const double u0 = f.Uc0[n * g.ncell + c];
-      if (sizeof(E) == 4 && wc == w0) {
-        u = wc * (u + u0);
-      } else {
-        u = wc * u + w0 * u0;
-      }
+      if constexpr (RK == 1) u = u + u0;
+      else u = sizeof(E) == 4 && dbits(wc) == dbits(w0) ? wc * (u + u0) : wc * u + w0 * u0;
     }
     U[n] = u;
   }
 #pragma unroll
   for (int d = 0; d < D; d++) {
     const double* vs = f.Vs + d * g.nface;
-    U[v::BX1 + d] = 0.5 * (vs[fc] + vs[fc + g.fs[d]]);
+    U[v::BX1 + d] = vs[fc] + vs[fc + g.fs[d]];
+  }
+  // RK2's combination and the mean of two faces as half a sum: the same value
+  // where that is far from the ends of the exponent range, with one rare
+  // branch for all of them (a call per value had kept the loads from going
+  // out together and cost more than the products)
+  constexpr int H0 = RK == 1 ? 0 : v::BX1;
+  if (!halve<H0, NV>(U)) {
+#pragma unroll
+    for (int n = H0; n < v::BX1; n++)
+      U[n] = stage_rare(f.Uc[n * g.ncell + c], f.Uc0[n * g.ncell + c], sizeof(E) == 4);
+#pragma unroll
+    for (int d = 0; d < D; d++) {
+      const double* vs = f.Vs + d * g.nface;
+      U[v::BX1 + d] = stage_rare(vs[fc], vs[fc + g.fs[d]], true);
+    }
   }
   // mixed path (E = float): the fused FP64 pressure recovery
   cons_to_prim<D, true, double, sizeof(E) == 4>(g.gm1, V, U);
@@ -1813,7 +1827,34 @@ __device__ __forceinline__ void d_stage_end(const Geo& g, const Fields& f, const
 }
 
 template <int D, typename E = double>
-__global__ void k_stage_end(Geo g, Fields f, const Ctl* ctl, int combine, double wc, double w0, int out) {
+__device__ __forceinline__ void d_stage_end(const Geo& g, const Fields& f, const Ctl* ctl, int combine, double wc,
+                                            double w0, dim3 bid, int out = 0) {
+  if (ctl->done) return;
+  const unsigned tid = thread_index(bid);
+  const long long tot = (long long)g.n[0] * g.n[1] * (D == 3 ? g.n[2] : 1);
+  if (tid >= tot) return;
+  const int i = g.beg[0] + (int)(tid % g.n[0]);
+  const unsigned r = tid / g.n[0];
+  const int j = g.beg[1] + (int)(r % g.n[1]);
+  const int k = (D == 3) ? g.beg[2] + (int)(r / g.n[1]) : 0;
+  const long long c = cidx(g, k, j, i);
+  const long long fc = fidx(g, k, j, i);
+  if (tid == 0) ((Ctl*)ctl)->uc_fresh = 1;  // read by the next stage begin
+  if (!combine) stage_end_cell<D, E, 0>(g, f, wc, w0, c, fc, out);
+  else if (dbits(wc) == dbits(0.5) && dbits(w0) == dbits(0.5)) stage_end_cell<D, E, 1>(g, f, wc, w0, c, fc, out);
+  else stage_end_cell<D, E, 2>(g, f, wc, w0, c, fc, out);
+}
+
+// FP64 path: bound by the FP64 pipe (81 % busy of the 84 % it reaches); mixed:
+// by its instructions (1200-1360 per cell, most of them the quotients and
+// conversions) and bytes (200-290 per cell) together.  256^3, both stages: FP64
+// 1.99 -> 1.76 ms, mixed 1.92 -> 1.72 ms with the halves above, the shorter
+// division and conversions (intdiv.cuh, fpconv.cuh) and the thread's cell from
+// 32-bit divisions; 512^2 with a state at rest (zero dividends) 69 -> 32 us.
+// Six blocks per multiprocessor: 1.77 and 1.89 ms where five took 1.79 and
+// 1.95, four 1.85 and 2.04 (before the shorter division).
+template <int D, typename E = double>
+__global__ void __launch_bounds__(256, 6) k_stage_end(Geo g, Fields f, const Ctl* ctl, int combine, double wc, double w0, int out) {
   d_stage_end<D, E>(g, f, ctl, combine, wc, w0, blockIdx, out);
 }
 
@@ -1823,13 +1864,13 @@ __global__ void k_stage_end(Geo g, Fields f, const Ctl* ctl, int combine, double
 // ---------------------------------------------------------------------------
 template <int D>
 __device__ __forceinline__ void d_divb(const Geo& g, const Fields& f, Ctl* ctl, dim3 bid) {
-  const long long tid = (long long)bid.x * blockDim.x + threadIdx.x;
+  const unsigned tid = thread_index(bid);
   const long long tot = (long long)g.n[0] * g.n[1] * (D == 3 ? g.n[2] : 1);
   // every lane reaches the warp reduction below; lanes past the end give 0
   const bool in = tid < tot;
-  const long long t = in ? tid : 0;
+  const unsigned t = in ? tid : 0u;
   const int i = g.beg[0] + (int)(t % g.n[0]);
-  const long long r = t / g.n[0];
+  const unsigned r = t / g.n[0];
   const int j = g.beg[1] + (int)(r % g.n[1]);
   const int k = (D == 3) ? g.beg[2] + (int)(r / g.n[1]) : 0;
   const long long fc = fidx(g, k, j, i);
@@ -1872,12 +1913,12 @@ __global__ void k_divb(Geo g, Fields f, Ctl* ctl) {
 template <int D>
 __device__ __forceinline__ void d_nan_count(const Geo& g, const Fields& f, Ctl* ctl, dim3 bid) {
   using v = Var<D>;
-  const long long tid = (long long)bid.x * blockDim.x + threadIdx.x;
+  const unsigned tid = thread_index(bid);
   const int nx = g.n[0] + 1, ny = g.n[1] + 1;
   const long long tot = (long long)nx * ny * (D == 3 ? g.n[2] + 1 : 1);
   if (tid >= tot) return;
   const int i = g.beg[0] + (int)(tid % nx);
-  const long long r = tid / nx;
+  const unsigned r = tid / nx;
   const int j = g.beg[1] + (int)(r % ny);
   const int k = (D == 3) ? g.beg[2] + (int)(r / ny) : 0;
   unsigned long long n = 0;

@@ -98,8 +98,9 @@ __device__ __forceinline__ T rcp(T b) {
 
 // the quotient of the whole-array kernels (cons <-> prim) on the integer pipe
 // for FP64 (intdiv.cuh): their quotients share a divisor, whose 64-bit
-// reciprocal is formed once for all of them (the mixed stage end 1.96 ms per
-// 256^3 cycle; 2.17 with the sweeps' quotients, 2.29 with calls of them)
+// reciprocal is formed once for all of them (the mixed stage end, when it took
+// 1.96 ms per 256^3 cycle: 2.17 with the sweeps' quotients, 2.29 with calls of
+// them)
 template <typename T>
 __device__ __forceinline__ T dvi(T a, T b) {
   if constexpr (sizeof(T) == 8) {
@@ -198,7 +199,7 @@ __device__ __forceinline__ void cons_to_prim(T gm1, T* V, const T* U) {
     }
     const T e = fma(-q(T(0.5), U[v::RHO]), m2, U[v::ENG]);
     V[v::PRS] = fma(T(-0.5), b2, e) * gm1;
-    if (V[v::PRS] <= T(0)) V[v::PRS] = T(kSmallPressureFix);
+    if (le0(V[v::PRS])) V[v::PRS] = T(kSmallPressureFix);
     return;
   }
   V[v::RHO] = U[v::RHO];
@@ -221,7 +222,7 @@ __device__ __forceinline__ void cons_to_prim(T gm1, T* V, const T* U) {
   const T mag = T(0.5) * b2;
   V[v::PRS] = (U[v::ENG] - kin - mag) * gm1;
   // floor; the reference's energy repair only touches a discarded local copy
-  if (V[v::PRS] <= T(0)) V[v::PRS] = T(kSmallPressureFix);
+  if (le0(V[v::PRS])) V[v::PRS] = T(kSmallPressureFix);
 }
 
 // induction flux of the transverse and bi-transverse field components

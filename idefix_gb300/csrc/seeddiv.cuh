@@ -135,6 +135,9 @@ IDFX_HD bool try_quot(double a, const SeedDiv& D, double& q) {
 IDFX_HD double quot(double a, const SeedDiv& D) {
   double q;
   if (try_quot(a, D, q)) return q;
+  // zero dividends are common (states at rest, fields along an axis)
+  const uint64_t A = dbits(a), B = dbits(D.b);
+  if ((A << 1) == 0ull && seed_band((uint32_t)(B >> 52) & 0x7ffu)) return dfrom((A ^ B) & (1ull << 63));
   return rare_div(a, D.b);
 }
 // a / b, correctly rounded
