@@ -9,6 +9,7 @@
 #pragma once
 #include <stdint.h>
 
+#include "fpconv.cuh"
 #include "intdiv.cuh"  // dbits / dfrom, IDFX_HD
 
 namespace idfx {
@@ -189,6 +190,38 @@ IDFX_HD bool prod_le0(T x, T y) {
   }
 }
 
+// x * s for a factor used many times: where s is a power of two (the face areas of
+// boxes of 2^n cells a side) the product is an add to the exponent field on the
+// FP64 path, with the product itself, as a call, outside the normal range
+template <typename T>
+struct Scale {
+  T s;
+  int k;  // s = 2^k, or the smallest int
+};
+template <typename T>
+IDFX_HD Scale<T> scale_by(T s) {
+  Scale<T> r{s, 0};
+  if constexpr (sizeof(T) == 8) {
+    const uint64_t u = dbits(s);
+    const bool p = (u << 12) == 0ull && (u >> 52) - 1ull < 2046ull;  // positive, normal, a power of two
+    r.k = p ? (int)(u >> 52) - 1023 : (int)0x80000000;
+  }
+  return r;
+}
+template <typename T>
+IDFX_HD T scaled(T x, const Scale<T>& c) {
+  if constexpr (sizeof(T) == 8) {
+    if (c.k == (int)0x80000000) return x * c.s;
+    const uint64_t u = dbits(x);
+    const int e = (int)((uint32_t)(u >> 52) & 0x7ffu);
+    if ((uint32_t)(e - 1) < 2046u && (uint32_t)(e + c.k - 1) < 2046u) return dfrom(u + ((uint64_t)(int64_t)c.k << 52));
+    if ((u << 1) == 0ull) return x;
+    return rare_mul(x, c.s);
+  } else {
+    return x * c.s;
+  }
+}
+
 // One upwind term of CalcContactAverage, (1 - w) a + w b with the weight w
 // in {0, 1/2, 1} (storeFlux.hpp:40-43).  The FP64 path forms the two
 // products exactly on the integer pipe - a product by 1 is the value, by 0 a
@@ -239,6 +272,24 @@ IDFX_HD E upwind_diff(E w, E xa, E ya, E xb, E yb) {
     return upwind_whole(w, xa, ya, xb, yb);
   } else {
     return upwind_term(w, xa - ya, xb - yb);
+  }
+}
+
+// HLLD's degeneracy test, whether s1 - s < 1e-4 (sm - s) (left; right mirrored:
+// s - s1 < 1e-4 (s - sm)).  FP64 path: a margin that FP32 arithmetic can see
+// decides - each difference is within 2^-22 of the magnitudes of its FP64
+// value - and the test itself, four FP64 operations a face, is a call.
+IDFX_RARE bool degenerate_left(double s1, double s, double sm) { return lt(s1 - s, 1.e-4 * -(s - sm)); }
+IDFX_RARE bool degenerate_right(double s1, double s, double sm) { return lt(-1.e-4 * (s - sm), s1 - s); }
+template <bool LEFT, typename T>
+IDFX_HD bool degenerate(T s1, T s, T sm) {
+  if constexpr (sizeof(T) == 8) {
+    const float a = d2f_rn(s1), b = d2f_rn(s), m = d2f_rn(sm);
+    const float gap = LEFT ? a - b : b - a, all = LEFT ? m - b : b - m;
+    if (gap - 1.e-4f * all > 9.5367431640625e-7f * (fabsf(a) + fabsf(b) + fabsf(m))) return false;
+    return LEFT ? degenerate_left(s1, s, sm) : degenerate_right(s1, s, sm);
+  } else {
+    return LEFT ? lt(s1 - s, T(1.e-4) * -(s - sm)) : lt(T(-1.e-4) * (s - sm), s1 - s);
   }
 }
 

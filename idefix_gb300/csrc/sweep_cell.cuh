@@ -272,10 +272,10 @@ __device__ __forceinline__ void d_sweep_cell(const Geo& g, const Fields& f, cons
     riemann<D, DIR, SOLVER>((T)g.gamma, (T)g.rgm1, vL, vl, r);
     store_emf<D, DIR>(g, f, cc, r, vL, vl);
     if (active_col) {
-      const T area = (T)g.A[DIR];
+      const Scale<T> area = scale_by((T)g.A[DIR]);
 #pragma unroll
       for (int n = 0; n < NU; n++) {
-        FA[n] = r.F[n] * area;
+        FA[n] = scaled(r.F[n], area);
         sf[n * nt + tid] = FA[n];
       }
       cm = r.cmax;

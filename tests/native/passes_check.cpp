@@ -1,7 +1,8 @@
 // Host check of the helpers of the whole-array FP64 passes (exact_ops.cuh)
 // against the IEEE-754 expressions they stand for: halved sums (RK2's
-// combination, the mean of two faces), quarters, and upwind terms whose side
-// is picked before the difference.  Prints the number of mismatches.
+// combination, the mean of two faces), quarters, upwind terms whose side is
+// picked before the difference, products by a power of two, and HLLD's
+// degeneracy tests.  Prints the number of mismatches.
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -56,6 +57,15 @@ int main(int argc, char** argv) {
     check("quarter", idfx::quarter(a), 0.25 * a, a, 0.0);
     const double ya = i % 8 == 1 ? a : any(i + 2), xb = any(i + 3), yb = i % 8 == 2 ? xb : any(i + 4);
     const double w = i % 4 == 0 ? 0.0 : i % 4 == 1 ? 1.0 : i % 4 == 2 ? 0.5 : 0.3;
+    const double sf = i % 3 ? std::ldexp(1.0, (int)(rng() % 140) - 120) : i % 9 ? value(1000, 1040) : any(i + 5);
+    check("scaled", idfx::scaled(a, idfx::scale_by(sf)), a * sf, a, sf);
+    // wave speeds: apart, nearly equal, at the threshold
+    const double sl = i % 32 == 4 ? any(i) : value(1000, 1030), sm = i % 32 == 5 ? any(i + 1) : sl + value(1000, 1030);
+    double s1 = i % 32 == 6 ? any(i + 2) : sl + (sm - sl) * (i % 2 ? 1e-4 : 1e-3 * (double)(rng() % 1000));
+    for (uint64_t k = rng() % 4; k > 0; k--) s1 = std::nextafter(s1, i % 4 < 2 ? 1e300 : -1e300);
+    if (i % 8 == 7) s1 += value(960, 1000);
+    check("degenerate left", idfx::degenerate<true>(s1, sl, sm) ? 1 : 0, (s1 - sl) < 1.e-4 * -(sl - sm) ? 1 : 0, s1, sl);
+    check("degenerate right", idfx::degenerate<false>(s1, sl, sm) ? 1 : 0, -1.e-4 * (sl - sm) < (s1 - sl) ? 1 : 0, s1, sl);
     check("upwind", idfx::upwind_diff(w, a, ya, xb, yb), (1.0 - w) * (a - ya) + w * (xb - yb), a, xb);
   }
   std::printf("%llu mismatches of %llu\n", mism, total);

@@ -1,5 +1,5 @@
-"""Halved sums, quarters and upwind terms of the whole-array FP64 passes
-(csrc/exact_ops.cuh) must equal the IEEE-754 expressions bit for bit over
+"""Halved sums, quarters, upwind terms, products by powers of two and HLLD's
+degeneracy tests of the FP64 kernels (csrc/exact_ops.cuh) must equal the IEEE-754 expressions bit for bit over
 random bit patterns, zeros, subnormals, infinities and NaNs."""
 import os
 import shutil
