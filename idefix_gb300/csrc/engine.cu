@@ -302,13 +302,15 @@ void launch_boundaries(Engine& e) {
   if (!e.g.nonper) return;
   for (int dir = 0; dir < e.g.D; dir++) {
     const int a = (dir == 0) ? 1 : 0, b = (dir == 2) ? 1 : 2;
+    const bool normal = e.g.bc[dir][0] != 0;
+    const int images = e.g.n[dir] >= e.g.ng;  // of every ghost in the active range
+    const unsigned x = nblocks(2LL * e.g.ng * e.g.ntv[a] * e.g.ntv[b]), roles = 1 + e.g.D;
     mark_begin(e, kKFillFaces);
-    dim3 grid(nblocks(2LL * e.g.ng * e.g.ntv[a] * e.g.ntv[b]), 1 + e.g.D);
-    IDFX_DISPATCH_D(k_bc_slab, grid, kThreads, e.g, e.f, e.ctl, dir);
+    IDFX_DISPATCH_D(k_bc_slab, dim3(x, roles + (normal && images ? 1 : 0)), kThreads, e.g, e.f, e.ctl, dir, 0, images);
     mark_end(e);
-    if (e.g.bc[dir][0] != 0) {
+    if (normal && !images) {
       mark_begin(e, kKFillFaces);
-      IDFX_DISPATCH_D(k_normal_field, nblocks((long long)e.g.nt[a] * e.g.nt[b]), kThreads, e.g, e.f, e.ctl, dir);
+      IDFX_DISPATCH_D(k_bc_slab, dim3(x, 1), kThreads, e.g, e.f, e.ctl, dir, (int)roles, images);
       mark_end(e);
     }
   }
@@ -406,7 +408,7 @@ void queue_cycle(Engine& e, int use_tstop) {
   const Region cycle_region("TimeIntegrator::Cycle");
   const Geo& g = e.g;
   const bool cell_emf = (g.emf == kEmfContact || g.emf == kEmfUct0);
-  const bool fused = (e.precision == IDFX_MIXED) && !g.nonper;
+  const bool fused = e.precision == IDFX_MIXED;
   k_cycle_begin<<<1, 1, 0, e.stream>>>(g, e.ctl, use_tstop);
   if (e.log_period > 0 && e.ncycles % e.log_period == 0) launch_divb_check(e);
   const bool nan_check = e.check_nan_period > 0 && e.ncycles % e.check_nan_period == 0;
@@ -415,17 +417,19 @@ void queue_cycle(Engine& e, int use_tstop) {
     {
       const Region r("Boundary::SetBoundaries");
       launch_boundaries(e);
-      // periodic block: a Runge-Kutta begin copy of the faces that the
-      // previous cycle's last face update already wrote leaves the ghosts
-      if (!g.nonper && (!save || e.faces_saved)) launch_fill_face_ghosts(e);
-      else launch_fill_faces(e, save);
+      // a Runge-Kutta begin copy of the faces that the previous cycle's last
+      // face update already wrote leaves the ghosts, which a non-periodic
+      // block has already (2-D rotor at 512^2: 10 launches of 87 us a cycle
+      // became 4)
+      if (save && !e.faces_saved) launch_fill_faces(e, save);
+      else if (!g.nonper) launch_fill_face_ghosts(e);
     }
     // mixed path: Uc carried over from the previous stage end when it is
     // still the state Vc came from (Ctl::uc_fresh); the FP64 path rebuilds it
     // as the reference does
     const int cons = kSbCons | (e.precision == IDFX_MIXED ? kSbKeepCons : 0);
     const int sb_flags = cons | (save ? kSbSaveBegin : 0) | (cell_emf ? kSbCellEmf : 0);
-    // mixed path, periodic block: once a stage end of this run has written
+    // mixed path: once a stage end of this run has written
     // the active cells' FP32 primitives, cell EMF and Runge-Kutta begin copy,
     // the stage begin fills the ghost cells alone
     {
@@ -456,9 +460,9 @@ void queue_cycle(Engine& e, int use_tstop) {
         }
         e.faces_saved = false;
       } else {
-        // periodic block: the last stage's face update also writes the next
-        // cycle's Runge-Kutta begin copy of the faces
-        const bool save_next = !g.nonper && e.nstages > 1 && stage == e.nstages - 1;
+        // the last stage's face update also writes the next cycle's
+        // Runge-Kutta begin copy of the faces
+        const bool save_next = e.nstages > 1 && stage == e.nstages - 1;
         launch_ct(e, (combine ? kCtCombine : 0) | (save_next ? kCtSaveBegin : 0), wc, w0);
         if (save_next) e.faces_saved = true;
       }

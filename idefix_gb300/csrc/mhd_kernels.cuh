@@ -322,7 +322,7 @@ __device__ __forceinline__ void d_stage_begin(const Geo& g, const Fields& f, con
   stage_begin_cell<D, E>(g, f, ctl, flags, i, j, k);
 }
 
-// Stage begin of the ghost cells only (periodic blocks, mixed path, when the
+// Stage begin of the ghost cells only (mixed path, when the
 // previous stage end left Uc, Vc, the FP32 primitives and the cell EMF of
 // every active cell): the two ghost slabs of direction bid.y, each over the
 // full extent of the other two directions (cells in two slabs get the same
@@ -363,10 +363,10 @@ __global__ void k_stage_begin(Geo g, Fields f, const Ctl* ctl, int flags) {
 // Non-periodic blocks: Boundary::SetBoundaries (boundary.hpp:240-280) one
 // direction after the other, each direction's pass reading what the passes
 // of the previous directions wrote (its loops span their ghosts too):
-//   k_bc_slab(dir)     ghost cells of the non-field variables and ghost faces
+//   d_bc_slab(dir)     ghost cells of the non-field variables and ghost faces
 //                      (both sides; boundary.hpp:575-809, loop ranges of
 //                      BoundaryForAll / BoundaryForX?s, boundary.hpp:971-1100)
-//   k_normal_field(dir) the normal field in the ghost faces of a reflective or
+//   d_normal_field(dir) the normal field in the ghost faces of a reflective or
 //                      outflow direction from div B = 0, marching outwards
 //                      (ReconstructNormalField, boundary.hpp:408-532)
 // then fill_faces / stage_begin run without the periodic copy.  The cell-
@@ -407,7 +407,7 @@ __device__ __forceinline__ void d_bc_slab(const Geo& g, const Fields& f, const C
   // along dir: ghosts [0, ng) on the left; on the right [ng + n, 2 ng + n) for
   // cells and tangential faces, one further for the normal faces
   const int shift = (comp == dir) ? 1 : 0;
-  if (comp == dir && type != 0) return;  // rebuilt by k_normal_field
+  if (comp == dir && type != 0) return;  // rebuilt by d_normal_field
   const int id = side ? g.ng + g.n[dir] + shift + depth : depth;
   const int is = bc_src(type, id, g.ng, g.n[dir], side);
   int dst[3], src[3];
@@ -436,78 +436,65 @@ __device__ __forceinline__ void d_bc_slab(const Geo& g, const Fields& f, const C
   }
 }
 
+// One thread per side and line along dir (all locations of the two other
+// directions); the recurrence runs outwards from the boundary face, each step
+// from the face it set before.  Face areas are uniform on a Cartesian grid.
+// images: the tangential ghost faces are read as the active faces they are
+// images of (d_bc_slab writes them in the same launch), else as they lie.
 template <int D>
-__global__ void k_bc_slab(Geo g, Fields f, const Ctl* ctl, int dir) {
-  d_bc_slab<D>(g, f, ctl, dir, blockIdx);
-}
-
-// One thread per line along dir (all locations of the two other directions);
-// the recurrence runs outwards from the boundary face, each step reading the
-// face it wrote before.  Face areas are uniform on a Cartesian grid.
-template <int D>
-__device__ __forceinline__ void d_normal_field(const Geo& g, const Fields& f, const Ctl* ctl, int dir, dim3 bid) {
+__device__ __forceinline__ void d_normal_field(const Geo& g, const Fields& f, const Ctl* ctl, int dir, int images,
+                                               dim3 bid) {
   if (ctl->done) return;
   const int a = (dir == 0) ? 1 : 0, b = (dir == 2) ? 1 : 2;
-  const unsigned tid = thread_index(bid);
-  if (tid >= (long long)g.nt[a] * g.nt[b]) return;
-  const int ia = (int)(tid % g.nt[a]), ib = (int)(tid / g.nt[a]);
-  const bool left = g.bc[dir][0] != 0, right = g.bc[dir][1] != 0;
-  double* V1 = f.Vs;
-  double* V2 = f.Vs + g.nface;
-  double* V3 = f.Vs + 2 * g.nface;  // read only when D == 3
-  const double A1 = g.A[0], A2 = g.A[1], A3 = g.A[2];
-  const long long s0 = g.fs[0], s1 = g.fs[1], s2 = g.fs[2];
-  const int nb = g.beg[dir] - 1, ne = g.end[dir], nt = g.nt[dir];
-  if (dir == 0) {
-    const int j = ia, k = ib;
-    if (left)
-      for (int i = nb; i >= 0; i--) {
-        const long long q = fidx(g, k, j, i);
-        double t = 0.0 + A2 * V2[q + s1] - A2 * V2[q];
-        if constexpr (D == 3) t = t + A3 * V3[q + s2] - A3 * V3[q];
-        V1[q] = 1.0 / A1 * (A1 * V1[q + s0] + (t));
-      }
-    if (right)
-      for (int i = ne; i < nt; i++) {
-        const long long q = fidx(g, k, j, i);
-        double t = 0.0 + A2 * V2[q + s1] - A2 * V2[q];
-        if constexpr (D == 3) t = t + A3 * V3[q + s2] - A3 * V3[q];
-        V1[q + s0] = 1.0 / A1 * (A1 * V1[q] - (t));
-      }
-  } else if (dir == 1) {
-    const int i = ia, k = ib;
-    if (left)
-      for (int j = nb; j >= 0; j--) {
-        const long long q = fidx(g, k, j, i);
-        double t = A1 * V1[q + s0] - A1 * V1[q];
-        if constexpr (D == 3) t = t + 1 * (A3 * V3[q + s2] - A3 * V3[q]);
-        V2[q] = 1.0 / A2 * (A2 * V2[q + s1] + (t));
-      }
-    if (right)
-      for (int j = ne; j < nt; j++) {
-        const long long q = fidx(g, k, j, i);
-        double t = A1 * V1[q + s0] - A1 * V1[q];
-        if constexpr (D == 3) t = t + 1 * (A3 * V3[q + s2] - A3 * V3[q]);
-        V2[q + s1] = 1.0 / A2 * (A2 * V2[q] - (t));
-      }
-  } else if constexpr (D == 3) {
-    const int i = ia, j = ib;
-    if (left)
-      for (int k = nb; k >= 0; k--) {
-        const long long q = fidx(g, k, j, i);
-        V3[q] = 1.0 / A3 * (A3 * V3[q + s2] + (A1 * V1[q + s0] - A1 * V1[q] + A2 * V2[q + s1] - A2 * V2[q]));
-      }
-    if (right)
-      for (int k = ne; k < nt; k++) {
-        const long long q = fidx(g, k, j, i);
-        V3[q + s2] = 1.0 / A3 * (A3 * V3[q] - (A1 * V1[q + s0] - A1 * V1[q] + A2 * V2[q + s1] - A2 * V2[q]));
-      }
+  const unsigned tid = thread_index(bid), lines = (unsigned)g.nt[a] * (unsigned)g.nt[b];
+  if (tid >= 2u * lines) return;
+  const int side = tid >= lines ? 1 : 0;
+  const unsigned line = tid - (side ? lines : 0u);
+  const int type = g.bc[dir][side];
+  if (type == 0) return;
+  int p[3];
+  p[a] = (int)(line % g.nt[a]);
+  p[b] = (int)(line / g.nt[a]);
+  p[dir] = 0;
+  const long long l0 = fidx(g, p[2], p[1], p[0]), sd = g.fs[dir];
+  double* V = f.Vs + dir * g.nface;
+  const double A = g.A[dir];
+  double face = V[l0 + (side ? g.end[dir] : g.beg[dir]) * sd];
+  for (int step = 0; step < g.ng; step++) {
+    const int m = side ? g.end[dir] + step : g.beg[dir] - 1 - step;  // ghost cell
+    const int ms = images ? bc_src(type, m, g.ng, g.n[dir], side) : m;
+    const long long q = l0 + ms * sd;
+    // A_c V_c difference across the cell along direction c (signs of a mirror
+    // image as d_bc_slab writes them)
+    auto at = [&](int c, long long x) {
+      const double y = f.Vs[(long long)c * g.nface + x];
+      return images && type == 1 ? -y : y;
+    };
+    double t;
+    if (dir == 0) {
+      t = 0.0 + g.A[1] * at(1, q + g.fs[1]) - g.A[1] * at(1, q);
+      if constexpr (D == 3) t = t + g.A[2] * at(2, q + g.fs[2]) - g.A[2] * at(2, q);
+    } else if (dir == 1) {
+      t = g.A[0] * at(0, q + g.fs[0]) - g.A[0] * at(0, q);
+      if constexpr (D == 3) t = t + 1 * (g.A[2] * at(2, q + g.fs[2]) - g.A[2] * at(2, q));
+    } else {
+      t = g.A[0] * at(0, q + g.fs[0]) - g.A[0] * at(0, q) + g.A[1] * at(1, q + g.fs[1]) - g.A[1] * at(1, q);
+    }
+    face = 1.0 / A * (side ? A * face - (t) : A * face + (t));
+    V[l0 + (side ? m + 1 : m) * sd] = face;
   }
 }
 
+// blockIdx.y + y0: 0 the cells, 1 + c the faces of component c, 1 + D the
+// normal field.  One launch where every image lies in the active range (the
+// pass took 6 and 7 us of a 512^2 rotor's 238 us cycle as two launches a
+// direction); a box with fewer cells than ghosts keeps two, whose second reads
+// the ghosts that the first wrote.
 template <int D>
-__global__ void k_normal_field(Geo g, Fields f, const Ctl* ctl, int dir) {
-  d_normal_field<D>(g, f, ctl, dir, blockIdx);
+__global__ void k_bc_slab(Geo g, Fields f, const Ctl* ctl, int dir, int y0, int images) {
+  const int role = (int)blockIdx.y + y0;
+  if (role <= D) d_bc_slab<D>(g, f, ctl, dir, dim3(blockIdx.x, role, 0));
+  else d_normal_field<D>(g, f, ctl, dir, images, blockIdx);
 }
 
 // ---------------------------------------------------------------------------
@@ -1489,8 +1476,8 @@ __global__ void __launch_bounds__(256, 3) k_ct_corner(Geo g, Fields f, const Ctl
 // type) writes equal weights (RK2: 1/2, 1/2) as one product of the sum.
 // combine argument of the face update: kCtCombine = the Runge-Kutta
 // combination with Vs0; kCtSaveBegin = also write the updated face as the
-// next cycle's Runge-Kutta begin copy (last stage of a cycle, periodic
-// blocks: the next cycle's face fill then passes over the ghosts alone)
+// next cycle's Runge-Kutta begin copy (last stage of a cycle: the next
+// cycle's face fill then passes over the ghosts alone, if it has any to fill)
 enum { kCtCombine = 1, kCtSaveBegin = 2 };
 
 // (weights compared by their bits: a comparison of doubles takes the FP64 pipe
@@ -1765,7 +1752,7 @@ __global__ void __launch_bounds__(kCtTI * kCtTJ, 3) k_ct_fused(Geo g, Fields f, 
 // ConvertConsToPrim.  Writes Uc and Vc.
 // ---------------------------------------------------------------------------
 // E: EMF type of the path (FP32: mixed path, see rk_combine).  out (mixed
-// path, periodic blocks): kSeOutputs also writes what the next stage begin
+// path): kSeOutputs also writes what the next stage begin
 // derives for the active cells - the FP32 primitives and (kSbCellEmf) the
 // cell EMF - and kSeSaveBegin the Runge-Kutta begin copy of the next cycle
 // (Uc0 = Uc), so that the next stage begin only fills the ghost cells.
