@@ -49,6 +49,7 @@ __global__ void __launch_bounds__(kCtTI * kCtTJ, 3) k_ct_tile(Geo g, Fields f, c
   constexpr int D = 3;
   using E = float;
   extern __shared__ __align__(128) unsigned char csm[];
+  chain_wait();
   if (ctl->done) return;
   float* ring = reinterpret_cast<float*>(csm);
   CtPlanes<E>& P = *reinterpret_cast<CtPlanes<E>*>(csm + ct_tile_planes_off());

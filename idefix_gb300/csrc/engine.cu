@@ -174,7 +174,10 @@ __global__ void k_invdt_max(Geo g, Fields f, Ctl* ctl) {
 // step's result with a cycle).  A kernel writes the pinned host mirror
 // directly, and a Ctl passed by value is taken at launch.
 __global__ void k_ctl_put(Ctl* ctl, Ctl v) { *ctl = v; }
-__global__ void k_ctl_get(const Ctl* ctl, Ctl* host) { *host = *ctl; }
+__global__ void k_ctl_get(const Ctl* ctl, Ctl* host) {
+  chain_wait();
+  *host = *ctl;
+}
 enum { kClrUcFresh = 1, kClrDone = 2, kClrNan = 4, kClrDivB = 8, kClrInvDt = 16 };
 __global__ void k_ctl_clear(Ctl* ctl, int what) {
   if (what & kClrUcFresh) ctl->uc_fresh = 0;
@@ -264,6 +267,24 @@ long long n_edges(const Geo& g) {
     else K<3><<<GRID, BLOCK, 0, e.stream>>>(__VA_ARGS__);                   \
   } while (0)
 
+// the same for kernels that begin with chain_wait()
+#define IDFX_CHAIN_D(K, GRID, BLOCK, ...)                                             \
+  do {                                                                                \
+    if (e.g.D == 2) launch_chained(e.stream, K<2>, GRID, BLOCK, 0, __VA_ARGS__);      \
+    else launch_chained(e.stream, K<3>, GRID, BLOCK, 0, __VA_ARGS__);                 \
+  } while (0)
+#define IDFX_CHAIN_DE(K, GRID, BLOCK, ...)                                                        \
+  do {                                                                                            \
+    const bool f32 = (e.precision == IDFX_MIXED);                                                 \
+    if (e.g.D == 2) {                                                                             \
+      if (f32) launch_chained(e.stream, K<2, float>, GRID, BLOCK, 0, __VA_ARGS__);                \
+      else launch_chained(e.stream, K<2, double>, GRID, BLOCK, 0, __VA_ARGS__);                   \
+    } else {                                                                                      \
+      if (f32) launch_chained(e.stream, K<3, float>, GRID, BLOCK, 0, __VA_ARGS__);                \
+      else launch_chained(e.stream, K<3, double>, GRID, BLOCK, 0, __VA_ARGS__);                   \
+    }                                                                                             \
+  } while (0)
+
 // dimension and EMF type (FP32 EMF buffers on the mixed path)
 #define IDFX_DISPATCH_DE(K, GRID, BLOCK, ...)                                              \
   do {                                                                                     \
@@ -280,7 +301,7 @@ long long n_edges(const Geo& g) {
 void launch_fill_faces(Engine& e, int save_begin) {
   dim3 grid(nblocks(e.g.nface), e.g.D);
   mark_begin(e, kKFillFaces);
-  IDFX_DISPATCH_D(k_fill_faces, grid, kThreads, e.g, e.f, e.ctl, save_begin);
+  IDFX_CHAIN_D(k_fill_faces, grid, kThreads, e.g, e.f, e.ctl, save_begin);
   mark_end(e);
 }
 // the ghost faces alone (periodic block, no Runge-Kutta begin copy due)
@@ -294,7 +315,7 @@ void launch_fill_face_ghosts(Engine& e) {
       if (n > slab) slab = n;
     }
   mark_begin(e, kKFillFaces);
-  IDFX_DISPATCH_D(k_fill_face_ghosts, dim3(nblocks(slab), e.g.D * e.g.D), kThreads, e.g, e.f, e.ctl);
+  IDFX_CHAIN_D(k_fill_face_ghosts, dim3(nblocks(slab), e.g.D * e.g.D), kThreads, e.g, e.f, e.ctl);
   mark_end(e);
 }
 // Boundary::SetBoundaries of a block with a reflective or outflow direction
@@ -306,18 +327,18 @@ void launch_boundaries(Engine& e) {
     const int images = e.g.n[dir] >= e.g.ng;  // of every ghost in the active range
     const unsigned x = nblocks(2LL * e.g.ng * e.g.ntv[a] * e.g.ntv[b]), roles = 1 + e.g.D;
     mark_begin(e, kKFillFaces);
-    IDFX_DISPATCH_D(k_bc_slab, dim3(x, roles + (normal && images ? 1 : 0)), kThreads, e.g, e.f, e.ctl, dir, 0, images);
+    IDFX_CHAIN_D(k_bc_slab, dim3(x, roles + (normal && images ? 1 : 0)), kThreads, e.g, e.f, e.ctl, dir, 0, images);
     mark_end(e);
     if (normal && !images) {
       mark_begin(e, kKFillFaces);
-      IDFX_DISPATCH_D(k_bc_slab, dim3(x, 1), kThreads, e.g, e.f, e.ctl, dir, (int)roles, images);
+      IDFX_CHAIN_D(k_bc_slab, dim3(x, 1), kThreads, e.g, e.f, e.ctl, dir, (int)roles, images);
       mark_end(e);
     }
   }
 }
 void launch_stage_begin(Engine& e, int flags) {
   mark_begin(e, kKStageBegin);
-  IDFX_DISPATCH_DE(k_stage_begin, nblocks(e.g.ncell), kThreads, e.g, e.f, e.ctl, flags);
+  IDFX_CHAIN_DE(k_stage_begin, nblocks(e.g.ncell), kThreads, e.g, e.f, e.ctl, flags);
   mark_end(e);
 }
 // the ghost cells alone (mixed path, periodic block, after a stage end that
@@ -330,7 +351,7 @@ void launch_stage_ghosts(Engine& e, int flags) {
     if (n > slab) slab = n;
   }
   mark_begin(e, kKStageBegin);
-  IDFX_DISPATCH_DE(k_stage_ghosts, dim3(nblocks(slab), e.g.D), kThreads, e.g, e.f, e.ctl, flags);
+  IDFX_CHAIN_DE(k_stage_ghosts, dim3(nblocks(slab), e.g.D), kThreads, e.g, e.f, e.ctl, flags);
   mark_end(e);
 }
 void launch_ct(Engine& e, int combine, double wc, double w0) {
@@ -351,11 +372,12 @@ void launch_ct(Engine& e, int combine, double wc, double w0) {
       static const bool smem_set = cudaFuncSetAttribute(k_ct_tile, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                         ct_tile_smem()) == cudaSuccess;
       (void)smem_set;
-      k_ct_tile<<<grid, dim3(kCtTI, kCtTJ), ct_tile_smem(), e.stream>>>(g, e.f, e.ctl, combine, wc, w0, cm->emf);
+      launch_chained(e.stream, k_ct_tile, grid, dim3(kCtTI, kCtTJ), ct_tile_smem(), g, e.f, e.ctl, combine, wc, w0,
+                     cm->emf);
     } else if (g.D == 2) {
-      k_ct_fused<2, float><<<grid, dim3(kCtTI, kCtTJ), 0, e.stream>>>(g, e.f, e.ctl, combine, wc, w0);
+      launch_chained(e.stream, k_ct_fused<2, float>, grid, dim3(kCtTI, kCtTJ), 0, g, e.f, e.ctl, combine, wc, w0);
     } else {
-      k_ct_fused<3, float><<<grid, dim3(kCtTI, kCtTJ), 0, e.stream>>>(g, e.f, e.ctl, combine, wc, w0);
+      launch_chained(e.stream, k_ct_fused<3, float>, grid, dim3(kCtTI, kCtTJ), 0, g, e.f, e.ctl, combine, wc, w0);
     }
     mark_end(e);
     return;
@@ -363,12 +385,12 @@ void launch_ct(Engine& e, int combine, double wc, double w0) {
   {
     const Region r("ConstrainedTransport::CalcCornerEMF");
     mark_begin(e, kKCtCorner);
-    IDFX_DISPATCH_DE(k_ct_corner, nblocks(n_edges(e.g)), kThreads, e.g, e.f, e.ctl);
+    IDFX_CHAIN_DE(k_ct_corner, nblocks(n_edges(e.g)), kThreads, e.g, e.f, e.ctl);
     mark_end(e);
   }
   const Region r("ConstrainedTransport::EvolveMagField");
   mark_begin(e, kKCtFaces);
-  IDFX_DISPATCH_DE(k_ct_faces, nblocks(n_edges(e.g)), kThreads, e.g, e.f, e.ctl, combine, wc, w0);
+  IDFX_CHAIN_DE(k_ct_faces, nblocks(n_edges(e.g)), kThreads, e.g, e.f, e.ctl, combine, wc, w0);
   mark_end(e);
 }
 void launch_find_shock(Engine& e) {
@@ -409,7 +431,7 @@ void queue_cycle(Engine& e, int use_tstop) {
   const Geo& g = e.g;
   const bool cell_emf = (g.emf == kEmfContact || g.emf == kEmfUct0);
   const bool fused = e.precision == IDFX_MIXED;
-  k_cycle_begin<<<1, 1, 0, e.stream>>>(g, e.ctl, use_tstop);
+  launch_chained(e.stream, k_cycle_begin, 1, 1, 0, g, e.ctl, use_tstop);
   if (e.log_period > 0 && e.ncycles % e.log_period == 0) launch_divb_check(e);
   const bool nan_check = e.check_nan_period > 0 && e.ncycles % e.check_nan_period == 0;
   for (int stage = 0; stage < e.nstages; stage++) {
@@ -474,17 +496,17 @@ void queue_cycle(Engine& e, int use_tstop) {
     {
       const Region r("Fluid::ConvertConsToPrim");
       mark_begin(e, kKStageEnd);
-      IDFX_DISPATCH_DE(k_stage_end, nblocks(n_active(g)), kThreads, g, e.f, e.ctl, combine, wc, w0, out);
+      IDFX_CHAIN_DE(k_stage_end, nblocks(n_active(g)), kThreads, g, e.f, e.ctl, combine, wc, w0, out);
       mark_end(e);
     }
     if (fused) e.stage_outputs = true;
   }
-  k_cycle_end<<<1, 1, 0, e.stream>>>(e.ctl);
+  launch_chained(e.stream, k_cycle_end, 1, 1, 0, e.ctl);
   e.ncycles++;
 }
 
 int read_ctl(Engine& e) {
-  k_ctl_get<<<1, 1, 0, e.stream>>>(e.ctl, e.ctl_host_dev);
+  launch_chained(e.stream, k_ctl_get, 1, 1, 0, e.ctl, e.ctl_host_dev);
   IDFX_CK(cudaGetLastError());
   IDFX_CK(cudaStreamSynchronize(e.stream));
   return IDFX_OK;

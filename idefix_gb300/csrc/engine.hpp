@@ -74,6 +74,23 @@ enum KernelClass {
 int block_geometry(const idfx_gpu_config* cfg, Geo& g);
 void choose_segments(Engine& e);
 
+// k behind the work queued on s, its blocks taking their places while the last
+// kernel there ends; k begins with chain_wait()
+template <typename... P, typename... A>
+inline void launch_chained(cudaStream_t s, void (*k)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c{};
+  c.gridDim = grid;
+  c.blockDim = block;
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = at;
+  c.numAttrs = 1;
+  cudaLaunchKernelEx(&c, k, P(args)...);
+}
+
 cudaEvent_t take_event(Engine& e);
 void mark_begin(Engine& e, int cls);
 void mark_end(Engine& e);

@@ -320,6 +320,7 @@ template <int D, int DIR, int ORDER, int SOLVER, typename T>
 __global__ void __launch_bounds__(kCellThreads, cell_resident(sizeof(T)))
     k_sweep_cell(Geo g, Fields f, const Ctl* ctl, int invdt, int last_dir) {
   extern __shared__ double cell_sm[];
+  chain_wait();
   d_sweep_cell<D, DIR, ORDER, SOLVER, T>(g, f, ctl, invdt, last_dir, blockIdx.x, reinterpret_cast<T*>(cell_sm));
 }
 
