@@ -186,20 +186,50 @@ __global__ void k_ctl_clear(Ctl* ctl, int what) {
   if (what & kClrDivB) ctl->divb_bits = 0ull;
   if (what & kClrInvDt) ctl->invdt_max_bits = 0ull;
 }
+// the fields that a caller sets, and those that the start of a run sets,
+// written where they lie: no control block is read back and sent again for
+// them (with the state's two arrays in one launch, upload + set_time + one FP64
+// cycle of 64^2 + download + get_time 208 -> 166 us)
+__global__ void k_ctl_time(Ctl* ctl, double t, double dt, long long ncycles) {
+  chain_wait();
+  ctl->t = t;
+  ctl->dt = dt;
+  ctl->ncycles = ncycles;
+  ctl->done = 0;
+  ctl->status = 0;
+}
+__global__ void k_ctl_run(Ctl* ctl, double tstop) {
+  chain_wait();
+  ctl->tstop = tstop;
+  ctl->done = 0;
+  ctl->status = 0;
+}
 // n doubles from src to dst (device memory), 16-byte vectors where both
 // addresses allow it
-__global__ void k_copy_f64(double* __restrict__ dst, const double* __restrict__ src, long long n) {
+struct CopyF64 {
+  double* dst;
+  const double* src;
+  long long n;
+};
+__device__ __forceinline__ void copy_f64(const CopyF64& c) {
   const long long stride = (long long)gridDim.x * blockDim.x;
   long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-  if (((reinterpret_cast<uintptr_t>(dst) | reinterpret_cast<uintptr_t>(src)) & 15) == 0) {
-    const long long n2 = n / 2;
-    double2* d2 = reinterpret_cast<double2*>(dst);
-    const double2* s2 = reinterpret_cast<const double2*>(src);
+  if (((reinterpret_cast<uintptr_t>(c.dst) | reinterpret_cast<uintptr_t>(c.src)) & 15) == 0) {
+    const long long n2 = c.n / 2;
+    double2* d2 = reinterpret_cast<double2*>(c.dst);
+    const double2* s2 = reinterpret_cast<const double2*>(c.src);
     for (long long q = t; q < n2; q += stride) d2[q] = s2[q];
-    if (t == 0 && (n & 1)) dst[n - 1] = src[n - 1];
+    if (t == 0 && (c.n & 1)) c.dst[c.n - 1] = c.src[c.n - 1];
   } else {
-    for (long long q = t; q < n; q += stride) dst[q] = src[q];
+    for (long long q = t; q < c.n; q += stride) c.dst[q] = c.src[q];
   }
+}
+// the two parts of a block's state (blockIdx.y), one launch; ctl (or null):
+// Uc is no longer Vc's
+__global__ void k_copy_state(CopyF64 a, CopyF64 b, Ctl* ctl) {
+  chain_wait();
+  if (ctl && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) ctl->uc_fresh = 0;
+  copy_f64(blockIdx.y == 0 ? a : b);
 }
 
 // Bounded-wait probe: the wait of the bulk-copy staged sweep (mbar_wait)
@@ -404,14 +434,13 @@ void ctl_clear(Engine& e, int what) { k_ctl_clear<<<1, 1, 0, e.stream>>>(e.ctl, 
 void ctl_push(Engine& e) { k_ctl_put<<<1, 1, 0, e.stream>>>(e.ctl, *e.ctl_host); }
 
 // device -> device copy of n doubles on the engine's stream (SMs, not a copy engine)
-void copy_f64(Engine& e, double* dst, const double* src, long long n) {
-  if (n <= 0) return;
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  const long long want = (n / 2 + kThreads - 1) / kThreads;
-  const unsigned blocks = (unsigned)(want < (long long)sms * 8 ? (want > 0 ? want : 1) : (long long)sms * 8);
-  k_copy_f64<<<blocks, kThreads, 0, e.stream>>>(dst, src, n);
+// Vc and Vs (null: not that part) on the device
+void copy_device(Engine& e, double* vc, const double* vc0, double* vs, const double* vs0, Ctl* ctl) {
+  const CopyF64 a{vc, vc0, vc && vc0 ? (2LL * e.g.D + 2) * e.g.ncell : 0LL};
+  const CopyF64 b{vs, vs0, vs && vs0 ? (long long)e.g.D * e.g.nface : 0LL};
+  const long long want = ((a.n > b.n ? a.n : b.n) / 2 + kThreads - 1) / kThreads;
+  const unsigned blocks = (unsigned)(want < (long long)e.sms * 8 ? (want > 0 ? want : 1) : (long long)e.sms * 8);
+  launch_chained(e.stream, k_copy_state, dim3(blocks, 2), kThreads, 0, a, b, ctl);
 }
 
 void launch_nan_check(Engine& e) {
@@ -1061,17 +1090,15 @@ static int copy_state(idfx_gpu* h, const double* Vc, const double* Vs, cudaMemcp
   const size_t bs = sizeof(double) * e.g.D * e.g.nface;
   const bool d2d = (kind == cudaMemcpyDeviceToDevice);  // by a kernel (see k_copy_f64)
   if (up) {
-    ctl_clear(e, kClrUcFresh);  // Uc no longer Vc's
     if (d2d) {
-      if (Vc) copy_f64(e, e.f.Vc, Vc, (long long)(bc / sizeof(double)));
-      if (Vs) copy_f64(e, e.f.Vs, Vs, (long long)(bs / sizeof(double)));
+      copy_device(e, e.f.Vc, Vc, e.f.Vs, Vs, e.ctl);
     } else {
+      ctl_clear(e, kClrUcFresh);  // Uc no longer Vc's
       if (Vc) IDFX_CK(cudaMemcpyAsync(e.f.Vc, Vc, bc, kind, e.stream));
       if (Vs) IDFX_CK(cudaMemcpyAsync(e.f.Vs, Vs, bs, kind, e.stream));
     }
   } else if (d2d) {
-    if (Vc) copy_f64(e, (double*)Vc, e.f.Vc, (long long)(bc / sizeof(double)));
-    if (Vs) copy_f64(e, (double*)Vs, e.f.Vs, (long long)(bs / sizeof(double)));
+    copy_device(e, (double*)Vc, e.f.Vc, (double*)Vs, e.f.Vs, nullptr);
   } else {
     if (Vc) IDFX_CK(cudaMemcpyAsync((void*)Vc, e.f.Vc, bc, kind, e.stream));
     if (Vs) IDFX_CK(cudaMemcpyAsync((void*)Vs, e.f.Vs, bs, kind, e.stream));
@@ -1109,17 +1136,9 @@ int idfx_gpu_download_cons(idfx_gpu* h, double* Uc) {
 int idfx_gpu_set_time(idfx_gpu* h, double t, double dt, long long ncycles) {
   if (!h) return IDFX_ERR_STATE;
   Engine& e = h->e;
-  int rc = read_ctl(e);
-  if (rc) return rc;
-  e.ctl_host->t = t;
-  e.ctl_host->dt = dt;
-  e.ctl_host->ncycles = ncycles;
-  e.ctl_host->done = 0;
-  e.ctl_host->status = 0;
-  e.ncycles = ncycles;
-  ctl_push(e);
+  launch_chained(e.stream, k_ctl_time, 1, 1, 0, e.ctl, t, dt, ncycles);
   IDFX_CK(cudaGetLastError());
-  IDFX_CK(cudaStreamSynchronize(e.stream));
+  e.ncycles = ncycles;
   return IDFX_OK;
 }
 
@@ -1139,13 +1158,8 @@ static int run_cycles(idfx_gpu* h, double tstop, long long max_cycles) {
   Engine& e = h->e;
   if (e.g.order == IDFX_LEARNED && !e.learned)
     return fail(e, IDFX_ERR_STATE, "the learned reconstruction needs idfx_gpu_set_learned first");
-  int rc = read_ctl(e);
-  if (rc) return rc;
-  e.ctl_host->tstop = tstop;
-  e.ctl_host->done = 0;
-  e.ctl_host->status = 0;
-  e.ncycles = e.ctl_host->ncycles;
-  ctl_push(e);
+  int rc = IDFX_OK;
+  launch_chained(e.stream, k_ctl_run, 1, 1, 0, e.ctl, tstop);
   e.stage_outputs = false;  // the run's first stage begin rebuilds from the stored state
   e.faces_saved = false;    // and its first face fill takes the Runge-Kutta begin copy
   const int use_tstop = tstop >= 0.0;

@@ -504,7 +504,8 @@ struct idfx_mlp {
   double* ploss = nullptr;      // losses of every block
   double* loss = nullptr;
   unsigned *kmin = nullptr, *kmax = nullptr;
-  int* status = nullptr;  // set by a block whose bounded wait gave up
+  int* status = nullptr;       // set by a block whose bounded wait gave up: mapped host memory, read
+  int* status_host = nullptr;  // without another copy
   const float* prims = nullptr;
   const float* tgt = nullptr;
   int nsnap = 0, nc = 0;
@@ -560,10 +561,7 @@ void launch_update(idfx_mlp* h, int B, bool grad, const AdamArgs& adam, double* 
 int sync_ok(idfx_mlp* h) {
   if (cudaGetLastError() != cudaSuccess) return IDFX_ERR_CUDA;
   if (cudaStreamSynchronize(h->stream) != cudaSuccess) return IDFX_ERR_CUDA;
-  if (h->status) {  // a bounded tensor-core wait that gave up
-    int st = 0;
-    if (cudaMemcpy(&st, h->status, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess || st) return IDFX_ERR_CUDA;
-  }
+  if (h->status_host && *(volatile int*)h->status_host) return IDFX_ERR_CUDA;  // a bounded tensor-core wait gave up
   return IDFX_OK;
 }
 
@@ -695,7 +693,10 @@ int idfx_mlp_create(int max_batch, void* stream, idfx_mlp** out) {
             dalloc(h, &h->g, NPARAM) && dalloc(h, &h->Wp, NPACK) && dalloc(h, &h->tiles[0], tiles) && dalloc(h, &h->tiles[1], tiles) &&
             dalloc(h, &h->part, (size_t)MAX_BLOCKS * NPARAM) && dalloc(h, &h->cols, B * NBIAS) &&
             dalloc(h, &h->ploss, MAX_BLOCKS * 2) && dalloc(h, &h->loss, 2) && dalloc(h, &h->kmin, NIN) &&
-            dalloc(h, &h->kmax, NIN) && dalloc(h, &h->status, 1);
+            dalloc(h, &h->kmax, NIN);
+  ok = ok && cudaHostAlloc(&h->status_host, sizeof(int), cudaHostAllocMapped) == cudaSuccess;
+  if (ok) *h->status_host = 0;
+  ok = ok && cudaHostGetDevicePointer(reinterpret_cast<void**>(&h->status), h->status_host, 0) == cudaSuccess;
   ok = ok && cudaFuncSetAttribute(k_train_tile, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_TRAIN) ==
                  cudaSuccess;
   if (ok) {
@@ -714,6 +715,7 @@ int idfx_mlp_destroy(idfx_mlp* h) {
   if (!h) return IDFX_ERR_STATE;
   if (h->stream) cudaStreamSynchronize(h->stream);
   for (void* p : h->allocs) cudaFree(p);
+  if (h->status_host) cudaFreeHost(h->status_host);
   if (h->own_stream) cudaStreamDestroy(h->stream);
   delete h;
   return IDFX_OK;

@@ -237,7 +237,7 @@ struct TrainArgs {
   int ld;
   double* loss;      // per block: summed squared error, summed squared targets; or null
   unsigned *kmin, *kmax;  // feature range, or null
-  int* status;       // set when a bounded wait gave up
+  int* status;       // set when a bounded wait gave up (the host's memory, mapped)
 };
 
 // eight BF16 values of row r, columns c .. c + 7 of a tile with C columns
@@ -539,7 +539,8 @@ __device__ __forceinline__ void train_tile(const TrainArgs& a, unsigned char* sm
     }
   }
   if (!ok && tid == 0) {
-    atomicExch(a.status, 1);
+    *(volatile int*)a.status = 1;
+    __threadfence_system();
     mbar_wait(bar + 1, (uint32_t)((t - 1) & 1));  // no copy may land after the block has gone
   }
   umma::fence_before_sync();
