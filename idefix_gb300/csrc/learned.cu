@@ -540,7 +540,7 @@ TrainArgs batch_args(const idfx_mlp* h, int B) {
 }
 void launch_tiles(idfx_mlp* h, const TrainArgs& a) {
   const unsigned n = (unsigned)(a.compute + (a.next ? a.split.blocks * a.split.tiles : 0));
-  k_train_tile<<<n, TT, SM_TRAIN, h->stream>>>(a);
+  launch_chained(h->stream, k_train_tile, n, TT, SM_TRAIN, a);
 }
 // samples base .. base + B - 1 of a seed into the tiles of `slot`
 void launch_assemble(idfx_mlp* h, int B, unsigned long long seed, long long base, int slot, bool range) {
@@ -554,8 +554,8 @@ void launch_assemble(idfx_mlp* h, int B, unsigned long long seed, long long base
 }
 // the blocks' gradients and losses summed, and the Adam step where adam.w is set
 void launch_update(idfx_mlp* h, int B, bool grad, const AdamArgs& adam, double* loss) {
-  k_train_update<<<grad ? UPDATE_BLOCKS : 1, 256, 0, h->stream>>>(grad ? h->part : nullptr, h->cols, h->max_batch,
-                                                                 split_batch(B).blocks, h->g, adam, h->ploss, B, loss);
+  launch_chained(h->stream, k_train_update, grad ? UPDATE_BLOCKS : 1, 256, 0, grad ? h->part : nullptr, h->cols,
+                 h->max_batch, split_batch(B).blocks, h->g, adam, h->ploss, B, loss);
 }
 
 int sync_ok(idfx_mlp* h) {

@@ -158,9 +158,11 @@ __device__ __forceinline__ void assemble(const Dataset& D, const Sample& mine, i
 // last bits of a gradient near zero into steps of full size, so a training
 // run is only as repeatable as its sums.
 // Measured, with the copies around them: sixteen steps at batch 8192 8351 ->
-// 876 us, at 256 7252 -> 719 us; loss and gradients of a given batch of 8192
-// 437 -> 80 us.  With the gather inside the computing blocks this launch took
-// 105 us (256 threads) or 78 us (512), beside them 30 us.
+// 876 us, 833 with the status word in mapped memory, 786 with each launch in
+// place while the one before ends; at 256 7252 -> 719 -> 613 us; loss and
+// gradients of a given batch of 8192 437 -> 69 us.  With the gather inside the
+// computing blocks this launch took 105 us (256 threads) or 78 us (512), beside
+// them 30 us.
 // ---------------------------------------------------------------------------
 constexpr int TR = 128;  // samples of a block
 constexpr int TT = 512;  // its threads: four warps per 32 samples, a quarter of the columns each
@@ -550,6 +552,7 @@ __device__ __forceinline__ void train_tile(const TrainArgs& a, unsigned char* sm
 
 __global__ void __launch_bounds__(TT, 1) k_train_tile(TrainArgs a) {
   extern __shared__ __align__(128) unsigned char train_sm[];
+  chain_wait();
   if ((int)blockIdx.x < a.compute) train_tile(a, train_sm);
   else assemble_tile(a, (int)blockIdx.x - a.compute, train_sm);
 }
@@ -592,6 +595,7 @@ __global__ void __launch_bounds__(256) k_train_update(const float* __restrict__ 
                                                       const double* __restrict__ loss, int B,
                                                       double* __restrict__ loss_out) {
   __shared__ float in[MAX_BLOCKS][64];
+  chain_wait();
   const int tid = threadIdx.x;
   if (part && blockIdx.x < NBIAS) {
     const int n = blockIdx.x;
