@@ -1,10 +1,11 @@
 // Correctly rounded FP64 division on the integer pipe.
 //
 // GB300 issues FP64 at about 2 thread-operations per clock and SM, and a
-// hardware-sequence FP64 division costs about nine of them; the integer
-// pipe is much wider.  Its dependency chain is longer, so it pays in
-// kernels with many resident warps (the memory-bound whole-array passes)
-// and not in the low-occupancy flux sweeps, which keep the hardware division.  div_rn(a, b) returns the IEEE-754 round-to-nearest-
+// hardware-sequence FP64 division costs about seven of them; the integer
+// pipe is much wider.  The divisor's 64-bit reciprocal serves all quotients
+// of a cell, which pays in the whole-array passes (three momenta and one half
+// over one density); the flux sweeps, whose divisors differ, take the shorter
+// form from FP32 seeds (seeddiv.cuh).  div_rn(a, b) returns the IEEE-754 round-to-nearest-
 // even quotient, bit-identical to a / b, computing the significand quotient
 // with 64-bit integer arithmetic:
 //   * the divisor significand x in [2^52, 2^53) gets a reciprocal

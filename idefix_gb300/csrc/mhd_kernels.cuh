@@ -996,12 +996,7 @@ __device__ __forceinline__ void d_sweep_xwarp(const Geo& g, const Fields& f, con
       }
       if (invdt) {
         const double prev = (invdt == 1) ? 0.0 : cI;
-        double inv;
-        if constexpr (sizeof(T) == 8) {
-          inv = prev + div_r(0.5 * (cm + cp), Recip{g.dx[0], g.rdx[0]});
-        } else {
-          inv = prev + to_f64(T(0.5) * (cm + cp) * invdxT);
-        }
+        const double inv = prev + to_f64(T(0.5) * (cm + cp) * invdxT);
         f.InvDt[cu] = inv;
         if (inv > run_max) run_max = inv;
       }

@@ -1,10 +1,10 @@
 // FP64 division by a divisor whose correctly rounded reciprocal is known.
 //
 // The FP64 pipe of this GPU is narrow and the flux sweeps are bound by it;
-// a hardware-sequence division costs several of its instructions.  When a
-// divisor is a constant of the run (gamma - 1, a cell width) or is shared by
-// several quotients of one Riemann problem, its reciprocal is formed once
-// and each quotient takes three FP64 operations, bit-identical to a / b:
+// a hardware-sequence division costs several of its instructions.  Where a
+// divisor is a constant of the run (LimO3's cell width and its three), its
+// reciprocal is formed once and each quotient takes three FP64 operations,
+// bit-identical to a / b:
 //   y = RN(1/b)            (host division, or the device's correctly rounded
 //                           reciprocal __drcp_rn)
 //   q = RN(a y)            (within one ulp of a / b)

@@ -32,8 +32,9 @@ namespace idfx {
 // 0.10 -> 0.045 ms, 91 x 62 x 45 PPM + HLL (RK3) 3.8 / 3.9 / 3.9 -> 1.5 / 1.7 /
 // 1.8 ms (the segments the block chose for itself); with the quotients and roots off the FP64 pipe
 // (seeddiv.cuh) 256^3 19.1 / 19.4 / 19.2 ms, at the pipe's rate (81 % busy of
-// the 84 % it reaches; 156 registers, 12 warps per multiprocessor; 16 warps at
-// 128 registers were 3 % slower).  Products emulated on the integer pipe
+// the 84 % it reaches; 160 registers, 12 warps per multiprocessor; 16 warps at
+// 128 registers were 3 % slower), and with less to do for the side of a face
+// that is not taken (riemann_hlld) 17.9 / 18.3 / 18.0 ms, 76-80 % busy.  Products emulated on the integer pipe
 // beside it (69 issue slots each) took a quarter of the pipe's work away and
 // changed the time by -6 to +10 %: the sweeps' instruction stream then waits on itself.
 // ---------------------------------------------------------------------------
@@ -114,6 +115,9 @@ __device__ __forceinline__ void d_sweep_cell(const Geo& g, const Fields& f, cons
   constexpr int A = (DIR == 0) ? 1 : 0, B = (DIR == 2) ? 1 : 2;
   const int nt = (int)blockDim.x, tid = (int)threadIdx.x;
   const int cols = cell_cols(DIR, sizeof(T), nt);
+  // (the block's constants become FP32 through from_f64: a conversion
+  // instruction would take a turn of the FP64 pipe in every thread, 17 of them and of
+  // comparisons per cell where 8 are left)
   T* ss = sm;            // [NS][nt] right-face states
   T* sf = sm + NS * nt;  // [NU + 1][nt] flux x area, wave speed
   const T* W;            // primitives
@@ -242,7 +246,7 @@ __device__ __forceinline__ void d_sweep_cell(const Geo& g, const Fields& f, cons
     if (lr.states) return;
   } else if (valid) {
     const Recip l3{g.l3b[DIR], g.l3y[DIR]};
-    const T dxd = (T)g.dx[DIR];
+    const T dxd = from_f64<T>(g.dx[DIR]);
     const bool shk = f.shock && f.shock[cc];
 #pragma unroll
     for (int n = 0; n < NV; n++) {
@@ -269,10 +273,10 @@ __device__ __forceinline__ void d_sweep_cell(const Geo& g, const Fields& f, cons
     vL[dd::BXn] = bn;
     vl[dd::BXn] = bn;
     RiemannOut<D, T> r;
-    riemann<D, DIR, SOLVER>((T)g.gamma, (T)g.rgm1, vL, vl, r);
+    riemann<D, DIR, SOLVER>(from_f64<T>(g.gamma), from_f64<T>(g.rgm1), vL, vl, r);
     store_emf<D, DIR>(g, f, cc, r, vL, vl);
     if (active_col) {
-      const Scale<T> area = scale_by((T)g.A[DIR]);
+      const Scale<T> area = scale_by(from_f64<T>(g.A[DIR]));
 #pragma unroll
       for (int n = 0; n < NU; n++) {
         FA[n] = scaled(r.F[n], area);
@@ -286,7 +290,7 @@ __device__ __forceinline__ void d_sweep_cell(const Geo& g, const Fields& f, cons
   // ---- flux difference ------------------------------------------------
   double run_max = 0.0;
   if (update) {
-    const T dtdV = (T)ctl->dtdV;
+    const T dtdV = from_f64<T>(ctl->dtdV);
 #pragma unroll
     for (int n = 0; n < NU; n++) {
       const T rhs = -dtdV * (sf[n * nt + tid + cols] - FA[n]);
@@ -297,9 +301,9 @@ __device__ __forceinline__ void d_sweep_cell(const Geo& g, const Fields& f, cons
       const T c2 = sf[NU * nt + tid + cols] + cm;
       double inv;
       if constexpr (sizeof(T) == 8) inv = prev + quot(pow2x<-1>(c2), g.dx[DIR]);
-      else inv = prev + to_f64(T(0.5) * c2 * (T(1) / (T)g.dx[DIR]));
+      else inv = prev + to_f64(T(0.5) * c2 * (T(1) / from_f64<T>(g.dx[DIR])));
       f.InvDt[cc] = inv;
-      if (inv > run_max) run_max = inv;  // NaN never compares greater
+      if (lt(run_max, inv)) run_max = inv;  // NaN never compares greater
     }
   }
   // CFL maximum: reduced over the warp, then an atomic only where it raises
@@ -308,7 +312,7 @@ __device__ __forceinline__ void d_sweep_cell(const Geo& g, const Fields& f, cons
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
       const double w = __shfl_xor_sync(0xffffffffu, run_max, o);
-      if (w > run_max) run_max = w;
+      if (dbits(w) > dbits(run_max)) run_max = w;  // neither negative nor NaN: ordered as their bits
     }
     unsigned long long* mx = (unsigned long long*)&((Ctl*)ctl)->invdt_max_bits;
     if ((tid & 31) == 0 && (unsigned long long)__double_as_longlong(run_max) > *(volatile unsigned long long*)mx)

@@ -159,6 +159,8 @@ int idfx_gpu_profile_read(idfx_gpu* h, double* ms, long long* launches, int ncla
  * the sweep kernel (below) and its segment length (cells per thread or per
  * tile along the sweep) of the fastest sweep, timed over reps launches; the
  * state is saved and restored, and the results do not depend on the choice.
+ * FP64 sweeps, and the mixed path's march of a small box, take one thread per
+ * cell whatever the segment is.
  * get/set_segments read and set the segment lengths. */
 int idfx_gpu_autotune(idfx_gpu* h, int reps);
 int idfx_gpu_get_segments(const idfx_gpu* h, int* seg);
