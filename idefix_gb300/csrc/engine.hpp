@@ -29,6 +29,7 @@ struct Engine {
   long long ncycles = 0;     // host mirror of the cycle counter
   int seg[3] = {32, 32, 32}; // marching segment per direction
   int sms = 152;             // multiprocessors of the device
+  bool chain = true;         // sweeps launched behind one another (off where the caller may be capturing the stream)
   int only_dir = -1;         // >= 0: sweeps launch that direction alone (autotuner)
   bool stage_outputs = false;  // mixed path: a stage end queued in this run wrote the next stage's inputs
   bool faces_saved = false;    // the last face update queued wrote the next cycle's Vs0
@@ -74,10 +75,10 @@ enum KernelClass {
 int block_geometry(const idfx_gpu_config* cfg, Geo& g);
 void choose_segments(Engine& e);
 
-// k behind the work queued on s, its blocks taking their places while the last
-// kernel there ends; k begins with chain_wait()
+// k behind the work queued on s; chain: its blocks taking their places while
+// the last kernel there ends (k begins with chain_wait())
 template <typename... P, typename... A>
-inline void launch_chained(cudaStream_t s, void (*k)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
+inline void launch_kernel(bool chain, cudaStream_t s, void (*k)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
@@ -87,8 +88,12 @@ inline void launch_chained(cudaStream_t s, void (*k)(P...), dim3 grid, dim3 bloc
   c.dynamicSmemBytes = smem;
   c.stream = s;
   c.attrs = at;
-  c.numAttrs = 1;
+  c.numAttrs = chain ? 1 : 0;
   cudaLaunchKernelEx(&c, k, P(args)...);
+}
+template <typename... P, typename... A>
+inline void launch_chained(cudaStream_t s, void (*k)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
+  launch_kernel(true, s, k, grid, block, smem, args...);
 }
 
 cudaEvent_t take_event(Engine& e);

@@ -139,6 +139,7 @@ extern "C" int idfx_evolve_stage_noalloc(const idfx_gpu_config* cfg, const doubl
     return rc;
   }
   e.stream = (cudaStream_t)stream;
+  e.chain = false;  // the caller may be capturing the stream
   // work arrays and control block inside the scratch
   double* p = scratch;
   auto take = [&](long long n) { double* q = p; p += n; return q; };

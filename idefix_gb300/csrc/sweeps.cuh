@@ -35,8 +35,9 @@ void launch_dir(Engine& e, int invdt, int last) {
   const long long cells = (long long)g.n[0] * g.n[1] * g.n[2];
   if (sizeof(T) == 8 || (!e.tile[DIR] && cell_sweep_wins(D, DIR, cells))) {
     const int nt = cell_threads(e.sms, [&](int t) { return cell_tiles(g, DIR, t, sizeof(T)); });
-    launch_chained(e.stream, k_sweep_cell<D, DIR, ORDER, SOLVER, T>, (unsigned)cell_tiles(g, DIR, nt, sizeof(T)), nt,
-                   cell_smem_bytes(D, nt, sizeof(T)), g, e.f, e.ctl, invdt, last);
+    launch_kernel(e.chain, e.stream, k_sweep_cell<D, DIR, ORDER, SOLVER, T>,
+                  (unsigned)cell_tiles(g, DIR, nt, sizeof(T)), nt, cell_smem_bytes(D, nt, sizeof(T)), g, e.f, e.ctl,
+                  invdt, last);
   } else if constexpr (sizeof(T) == 4 && D == 3 && DIR == 0) {
     // FP32 x sweep of a large box: warp chunks along each row (coalesced);
     // staged by bulk copies when rows and arrays are 16-byte aligned
