@@ -46,8 +46,8 @@ BYTES_PER_ZONE_CYCLE = 320.0  # 8 FP64 state values x 5 transfers per RK2 cycle
 # sweep launches of the first cycle), the instructions scaled to 256^3 by the
 # lines a sweep processes (the CT-extension columns add 1.6 % of the cells at
 # 256^3 against 3.1 % at 128^3, the cells at a line's ends 0.8 % against 1.6 %).
-FP64_INST_PER_CELL = {"sweep_x": 245.0, "sweep_y": 245.0, "sweep_z": 241.0}
-DRAM_BYTES_PER_CELL = {"sweep_x": 161.0, "sweep_y": 173.0, "sweep_z": 174.0}
+FP64_INST_PER_CELL = {"sweep_x": 244.7, "sweep_y": 244.8, "sweep_z": 241.5}
+DRAM_BYTES_PER_CELL = {"sweep_x": 161.6, "sweep_y": 171.6, "sweep_z": 173.1}
 # FP64 operations per active zone and RK2 cycle of the reference algorithm on
 # this workload at 256^3, each add/sub, mul, div and sqrt counted once
 # (1465.5 + 1662.8 + 215.5 + 35.8): the operation-counting build of the CPU
@@ -59,8 +59,8 @@ def fp64_flop_roof(value, peak_gops):
     """The algorithmic FP64 rate of one GPU running `value` zone-cycles/s,
     against the FP64 issue rate measured on it (Gop/s), and the zone-cycle
     rate that issue rate allows if every counted operation took a single FP64
-    instruction (an upper bound: a correctly rounded division or square root
-    takes several)."""
+    instruction.  Quotients, roots, exact scalings and comparisons run on the
+    integer and FP32 pipes, so the fraction can pass 1."""
     if not peak_gops or peak_gops <= 0.0:
         return None
     ach = value * FP64_FLOP_PER_ZONE_CYCLE / 1e9
