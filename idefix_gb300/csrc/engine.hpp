@@ -76,7 +76,9 @@ int block_geometry(const idfx_gpu_config* cfg, Geo& g);
 void choose_segments(Engine& e);
 
 // k behind the work queued on s; chain: its blocks taking their places while
-// the last kernel there ends (k begins with chain_wait())
+// the last kernel there ends.  Such a kernel begins with chain_wait() and takes
+// no __restrict__ pointer: the qualifier says that nobody else writes the data
+// while the kernel is resident, and the launch before it does
 template <typename... P, typename... A>
 inline void launch_kernel(bool chain, cudaStream_t s, void (*k)(P...), dim3 grid, dim3 block, size_t smem, A... args) {
   cudaLaunchAttribute at[1];

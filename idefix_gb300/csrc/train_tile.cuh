@@ -590,10 +590,11 @@ static_assert(OB1 % 64 == 0 && OW2 % 64 == 0 && OB2 % 64 == 0 && OW3 % 64 == 0 &
 //            one adds them up
 //   biases   the column sum of dZ or dY: thread t every 256th sample from t on,
 //            then a tree over the threads
-__global__ void __launch_bounds__(256) k_train_update(const float* __restrict__ part, const float* __restrict__ cols,
-                                                      int ld, int blocks, float* __restrict__ g, AdamArgs adam,
-                                                      const double* __restrict__ loss, int B,
-                                                      double* __restrict__ loss_out) {
+//   (no __restrict__: the launch before writes part, cols and loss while this
+//   one's blocks are resident, see launch_chained)
+__global__ void __launch_bounds__(256) k_train_update(const float* part, const float* cols, int ld, int blocks,
+                                                      float* g, AdamArgs adam, const double* loss, int B,
+                                                      double* loss_out) {
   __shared__ float in[MAX_BLOCKS][64];
   chain_wait();
   const int tid = threadIdx.x;
