@@ -278,7 +278,9 @@ IDFX_HD E upwind_diff(E w, E xa, E ya, E xb, E yb) {
 // HLLD's degeneracy test, whether s1 - s < 1e-4 (sm - s) (left; right mirrored:
 // s - s1 < 1e-4 (s - sm)).  FP64 path: a margin that FP32 arithmetic can see
 // decides - each difference is within 2^-22 of the magnitudes of its FP64
-// value - and the test itself, four FP64 operations a face, is a call.
+// value, and where a magnitude is below FP32's normal range within 2^-148, which
+// the smallest normal number in the margin covers - and the test itself, four
+// FP64 operations a face, is a call.
 IDFX_RARE bool degenerate_left(double s1, double s, double sm) { return lt(s1 - s, 1.e-4 * -(s - sm)); }
 IDFX_RARE bool degenerate_right(double s1, double s, double sm) { return lt(-1.e-4 * (s - sm), s1 - s); }
 template <bool LEFT, typename T>
@@ -286,7 +288,7 @@ IDFX_HD bool degenerate(T s1, T s, T sm) {
   if constexpr (sizeof(T) == 8) {
     const float a = d2f_rn(s1), b = d2f_rn(s), m = d2f_rn(sm);
     const float gap = LEFT ? a - b : b - a, all = LEFT ? m - b : b - m;
-    if (gap - 1.e-4f * all > 9.5367431640625e-7f * (fabsf(a) + fabsf(b) + fabsf(m))) return false;
+    if (gap - 1.e-4f * all > 9.5367431640625e-7f * (fabsf(a) + fabsf(b) + fabsf(m)) + 1.17549435e-38f) return false;
     return LEFT ? degenerate_left(s1, s, sm) : degenerate_right(s1, s, sm);
   } else {
     return LEFT ? lt(s1 - s, T(1.e-4) * -(s - sm)) : lt(T(-1.e-4) * (s - sm), s1 - s);
