@@ -149,6 +149,24 @@ IDFX_HD bool abs_ge(T x, T y) {
   }
 }
 
+// neither infinite nor a NaN
+template <typename T>
+IDFX_HD bool is_finite(T x) {
+  if constexpr (sizeof(T) == 8) {
+    return (dbits(x) << 1) < (0x7FFull << 53);
+  } else {
+    return (fbits(x) << 1) < 0xFF000000u;
+  }
+}
+template <typename T>
+IDFX_HD T not_a_number() {
+  if constexpr (sizeof(T) == 8) {
+    return dfrom(0x7FF8000000000000ull);
+  } else {
+    return ffrom(0x7FC00000u);
+  }
+}
+
 // the sign of x: -1, 0 (zeros, NaN) or 1; and s |x| for such a sign and
 // x >= 0, the product's value (0 x where s is 0)
 template <typename T>

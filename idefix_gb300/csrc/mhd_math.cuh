@@ -764,10 +764,15 @@ __device__ __forceinline__ void riemann_hlld(T gamma, T rgm1, const T* vL, const
     const uint64_t sgnb = sideL ? (sBxb ^ (1ull << 63)) : sBxb;
     uss[ENG] = us[ENG] + times_sign(sq * scrh, sgn, sgnb);
     const T S1 = sideL ? S1L : S1R;
-    // density and normal momentum are the single star's: no contribution
+    // density and normal momentum are the single star's: S1 times zero, which
+    // is nothing or, where one of the two is not finite, a NaN (FP64: from the
+    // bits, the two terms as they stand would be six FP64 operations a face)
+    const bool fin = is_finite(S1);
 #pragma unroll
-    for (int n = 0; n < NV; n++)
-      if (n != RHO && n != Xn) F[n] = mad(S1, uss[n] - us[n], F[n]);
+    for (int n = 0; n < NV; n++) {
+      if (sizeof(T) == 4 || (n != RHO && n != Xn)) F[n] = mad(S1, uss[n] - us[n], F[n]);
+      else if (!(fin && is_finite(us[n]))) F[n] = not_a_number<T>();
+    }
   }
   // F += s (us - u) of the chosen side: single star F = Fs + s (us - u),
   // double star F = (Fs + S1 (uss - us)) + s (us - u), the reference's order
