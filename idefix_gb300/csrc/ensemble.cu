@@ -164,26 +164,42 @@ std::vector<int> schedule(const EnsEngine& e) {
   return order;
 }
 
-int upload_table(EnsEngine& e, EnsTable& t, const std::vector<int4>& items) {
+void free_table(EnsTable& t) {
   if (t.items) cudaFree(t.items);
-  t.items = nullptr;
-  t.n = (int)items.size();
-  if (t.n == 0) return IDFX_OK;
-  if (cudaMalloc(&t.items, items.size() * sizeof(int4)) != cudaSuccess) return IDFX_ERR_CUDA;
-  if (cudaMemcpy(t.items, items.data(), items.size() * sizeof(int4), cudaMemcpyHostToDevice) != cudaSuccess)
+  t = EnsTable{};
+}
+
+// a list and the kernel that it is for (EnsTable::nt)
+struct EnsList {
+  std::vector<int4> items;
+  int nt = 0;
+};
+
+int upload_table(EnsTable& t, const EnsList& list) {
+  free_table(t);
+  if (list.items.empty()) return IDFX_OK;
+  const size_t bytes = list.items.size() * sizeof(int4);
+  if (cudaMalloc(&t.items, bytes) != cudaSuccess) return IDFX_ERR_CUDA;
+  if (cudaMemcpy(t.items, list.items.data(), bytes, cudaMemcpyHostToDevice) != cudaSuccess) {
+    free_table(t);
     return IDFX_ERR_CUDA;
+  }
+  t.n = (int)list.items.size();
+  t.nt = list.nt;
   return IDFX_OK;
 }
 
-// cell: for the cell sweeps of blocks of nt threads, else for the march
-std::vector<int4> sweep_items(const EnsEngine& e, int dir, const std::vector<int>& boxes, bool cell, int nt) {
-  std::vector<int4> v;
-  if (cell) {  // one entry per tile of nt cells
+// nt > 0: for the cell sweeps of blocks of nt threads, else for the march
+EnsList sweep_items(const EnsEngine& e, int dir, const std::vector<int>& boxes, int nt) {
+  EnsList list;
+  list.nt = nt;
+  std::vector<int4>& v = list.items;
+  if (nt > 0) {  // one entry per tile of nt cells
     for (int b : boxes) {
       const long long n = cell_tiles(e.boxes[b].g, dir, nt, e.precision == IDFX_FP64 ? 8 : 4);
       for (long long x = 0; x < n; x++) v.push_back(make_int4(b, (int)x, 0, 0));
     }
-    return v;
+    return list;
   }
   for (int b : boxes) {
     const Geo& g = e.boxes[b].g;
@@ -193,7 +209,7 @@ std::vector<int4> sweep_items(const EnsEngine& e, int dir, const std::vector<int
     for (int y = 0; y < nseg; y++)
       for (long long x = 0; x < nx; x++) v.push_back(make_int4(b, (int)x, y, 0));
   }
-  return v;
+  return list;
 }
 
 // the per-box phases' work lists for blocks of bt threads
@@ -210,35 +226,40 @@ void phase_items(const EnsEngine& e, const std::vector<int>& order, int bt, std:
   }
 }
 
+// every work list of the ensemble's boxes and segments as they are now: all
+// of them replaced, or (no memory) none
 int build_tables(EnsEngine& e) {
   const std::vector<int> order = schedule(e);
-  std::vector<int4> fill, begin, edges, active, fill64, begin64, edges64, active64;
-  phase_items(e, order, kT, fill, begin, edges, active);
-  phase_items(e, order, kTM, fill64, begin64, edges64, active64);
-  int rc = upload_table(e, e.fill, fill);
-  if (!rc) rc = upload_table(e, e.begin, begin);
-  if (!rc) rc = upload_table(e, e.edges, edges);
-  if (!rc) rc = upload_table(e, e.active, active);
-  if (!rc) rc = upload_table(e, e.fill64, fill64);
-  if (!rc) rc = upload_table(e, e.begin64, begin64);
-  if (!rc) rc = upload_table(e, e.edges64, edges64);
-  if (!rc) rc = upload_table(e, e.active64, active64);
+  const bool fp64 = e.precision == IDFX_FP64;
+  const std::vector<EnsTable*> tables = e.tables();
+  std::vector<EnsList> lists(tables.size());
+  auto list_of = [&](const EnsTable& t) -> EnsList& {
+    return lists[std::find(tables.begin(), tables.end(), &t) - tables.begin()];
+  };
+  phase_items(e, order, kT, list_of(e.fill).items, list_of(e.begin).items, list_of(e.edges).items,
+              list_of(e.active).items);
+  phase_items(e, order, kTM, list_of(e.fill64).items, list_of(e.begin64).items, list_of(e.edges64).items,
+              list_of(e.active64).items);
   int dev = 0, sms = 148;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   long long cells = 0;
   for (int b = 0; b < e.nbox; b++) cells += active_cells(e.boxes[b].g);
-  for (int d = 0; d < e.D && !rc; d++) {
-    e.cell32[d] = e.precision != IDFX_FP64 && cell_sweep_wins(e.D, d, cells);
-    e.cell_nt[d] = cell_threads(sms, [&](int t) {
+  for (int d = 0; d < e.D; d++) {
+    const int nt = cell_threads(sms, [&](int t) {
       long long n = 0;
-      for (int b = 0; b < e.nbox; b++) n += cell_tiles(e.boxes[b].g, d, t, e.precision == IDFX_FP64 ? 8 : 4);
+      for (int b = 0; b < e.nbox; b++) n += cell_tiles(e.boxes[b].g, d, t, fp64 ? 8 : 4);
       return n;
     });
-    const bool fp64 = e.precision == IDFX_FP64;
-    rc = upload_table(e, e.sweep[d], sweep_items(e, d, order, fp64 || e.cell32[d], e.cell_nt[d]));
-    if (!rc) rc = upload_table(e, e.sweep64[d], sweep_items(e, d, order, fp64, kTM));
+    list_of(e.sweep[d]) = sweep_items(e, d, order, fp64 || cell_sweep_wins(e.D, d, cells) ? nt : 0);
+    list_of(e.sweep64[d]) = sweep_items(e, d, order, fp64 ? kTM : 0);
   }
+  std::vector<EnsTable> fresh(tables.size());
+  int rc = IDFX_OK;
+  for (size_t i = 0; i < tables.size() && !rc; i++) rc = upload_table(fresh[i], lists[i]);
+  if (!rc)
+    for (size_t i = 0; i < tables.size(); i++) std::swap(fresh[i], *tables[i]);
+  for (EnsTable& t : fresh) free_table(t);
   return rc;
 }
 
@@ -447,18 +468,19 @@ int autotune(EnsEngine& e, int reps) {
   cudaEventCreate(&ea);
   cudaEventCreate(&eb);
   EnsTable trial;
+  std::vector<int> before;  // the segments that the work lists are made for
+  for (const EnsBox& B : e.boxes) before.insert(before.end(), B.seg, B.seg + 3);
   for (auto& kv : classes) {
     if (rc) break;
     const std::vector<int>& members = kv.second;
     for (int d = 0; d < e.D && !rc; d++) {
-      e.cell32[d] = false;  // (build_tables below decides again)
       int best_seg = e.boxes[members[0]].seg[d];
       float best_ms = 1e30f;
       for (int s = 2; s <= 64; s *= 2) {
         if (s > kv.first[d]) break;
         for (int b : members) e.boxes[b].seg[d] = s;
         rc = upload_boxes(e);
-        if (!rc) rc = upload_table(e, trial, sweep_items(e, d, members, false, 0));
+        if (!rc) rc = upload_table(trial, sweep_items(e, d, members, 0));
         if (rc) break;
         const float ms = time_sweep(e, d, trial, reps, ea, eb);
         if (ms < best_ms) {
@@ -469,7 +491,7 @@ int autotune(EnsEngine& e, int reps) {
       for (int b : members) e.boxes[b].seg[d] = best_seg;
     }
   }
-  if (trial.items) cudaFree(trial.items);
+  free_table(trial);
   cudaEventDestroy(ea);
   cudaEventDestroy(eb);
   if (cudaGetLastError() != cudaSuccess && !rc) rc = IDFX_ERR_CUDA;
@@ -481,7 +503,12 @@ int autotune(EnsEngine& e, int reps) {
   cudaFree(backup);
   if (!rc) rc = upload_boxes(e);
   if (!rc) rc = build_tables(e);
-  if (!rc) rc = capture_graph(e);
+  if (rc) {  // the segments that the lists, which are the old ones, are made for
+    for (int b = 0; b < e.nbox; b++) std::copy_n(before.begin() + 3 * b, 3, e.boxes[b].seg);
+    upload_boxes(e);
+  } else {
+    rc = capture_graph(e);
+  }
   if (rc && e.err.empty()) e.err = "autotune: CUDA failure";
   return rc;
 }
@@ -502,8 +529,7 @@ void release(EnsEngine& e) {
   if (e.exec_checks) cudaGraphExecDestroy(e.exec_checks);
   if (e.exec_persist) cudaGraphExecDestroy(e.exec_persist);
   if (e.d_bar) cudaFree(e.d_bar);
-  for (EnsTable* t : e.tables())
-    if (t->items) cudaFree(t->items);
+  for (EnsTable* t : e.tables()) free_table(*t);
   if (e.d_boxes) cudaFree(e.d_boxes);
   if (e.d_ctl) cudaFree(e.d_ctl);
   if (e.h_ctl) cudaFreeHost(e.h_ctl);

@@ -22,10 +22,14 @@ struct EnsBox {
   int seg[3];  // march segment length per direction (autotuned)
 };
 
-// one entry per CUDA block of a phase: {box, block.x, block.y, block.z}
+// one entry per CUDA block of a phase: {box, block.x, block.y, block.z}; of a
+// sweep {box, tile, 0, 0} for the cell sweep with nt threads a block where
+// nt > 0, else {box, block.x, segment, 0} for the march.  The list says which
+// kernel it is for, so that the two cannot come apart.
 struct EnsTable {
   int4* items = nullptr;
   int n = 0;
+  int nt = 0;
 };
 
 // grid-wide barrier of the persistent ensemble kernel (device memory)
@@ -62,8 +66,6 @@ struct EnsEngine {
   bool own_stream = false;
   EnsTable fill, begin, sweep[3], edges, active;
   EnsTable sweep64[3];                          // the persistent kernel's sweeps: tiles of 64 cells (FP64), marches
-  bool cell32[3] = {false, false, false};       // FP32 batched sweeps with a thread per cell
-  int cell_nt[3] = {128, 128, 128};             // threads of the cell sweeps' blocks (batched launches)
   EnsTable fill64, begin64, edges64, active64;  // the same phases at 64 threads per item (persistent kernel)
   std::vector<EnsTable*> tables() {
     return {&fill, &begin, &sweep[0], &sweep[1], &sweep[2], &edges, &active, &sweep64[0], &sweep64[1],

@@ -121,8 +121,8 @@ __global__ void __launch_bounds__(kCellThreads, cell_resident(sizeof(T)))
 template <int D, int ORDER, int SOLVER, typename T>
 void launch_ens_dir(EnsEngine& e, int dir, const EnsTable& t, int invdt, int last) {
   if (t.n == 0) return;
-  if (sizeof(T) == 8 || e.cell32[dir]) {
-    const int nt = e.cell_nt[dir];
+  if (t.nt > 0) {
+    const int nt = t.nt;
     const size_t sm = cell_smem_bytes(D, nt, sizeof(T));
     if (dir == 0) ke_sweep_cell<D, 0, ORDER, SOLVER, T><<<t.n, nt, sm, e.stream>>>(e.d_boxes, t.items, invdt, last);
     if (dir == 1) ke_sweep_cell<D, 1, ORDER, SOLVER, T><<<t.n, nt, sm, e.stream>>>(e.d_boxes, t.items, invdt, last);
