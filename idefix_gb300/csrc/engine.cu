@@ -825,7 +825,8 @@ int idfx_gpu_create(const idfx_gpu_config* cfg, void* stream, idfx_gpu** out) {
   const size_t nc = (size_t)g.ncell, nf = (size_t)g.nface;
   const bool hll_emf = (g.emf == kEmfUctHll || g.emf == kEmfUctHlld);
   // the mixed path's sweeps and the learned correction read the primitives in FP32
-  const bool vc32 = cfg->precision == IDFX_MIXED || cfg->order == IDFX_LEARNED;
+  // (the learned correction rounds them itself where they do not fit)
+  bool vc32 = cfg->precision == IDFX_MIXED || cfg->order == IDFX_LEARNED;
   size_t len = 3 * NV * nc + 2 * g.D * nf + nc  // Vc, Uc, Uc0, Vs, Vs0, InvDt
                + 6 * nc + 3 * nc + 3 * nc + 3 * nc  // face EMFs, sv, cell EMFs, corner EMFs
                + (hll_emf ? 12 * nc : 0)
@@ -838,7 +839,16 @@ int idfx_gpu_create(const idfx_gpu_config* cfg, void* stream, idfx_gpu** out) {
     rc = cuda_check(e, cudaStreamCreateWithFlags(&e.stream, cudaStreamNonBlocking), "cudaStreamCreate");
     e.own_stream = (rc == IDFX_OK);
   }
-  if (rc == IDFX_OK) rc = cuda_check(e, cudaMalloc(&e.pool, len * sizeof(double)), "cudaMalloc(fields)");
+  if (rc == IDFX_OK) {
+    cudaError_t got = cudaMalloc(&e.pool, len * sizeof(double));
+    if (got != cudaSuccess && cfg->order == IDFX_LEARNED) {
+      cudaGetLastError();
+      vc32 = false;
+      len -= (NV * nc + 1) / 2;
+      got = cudaMalloc(&e.pool, len * sizeof(double));
+    }
+    rc = cuda_check(e, got, "cudaMalloc(fields)");
+  }
   if (rc == IDFX_OK) rc = cuda_check(e, cudaMemsetAsync(e.pool, 0, len * sizeof(double), e.stream), "cudaMemset");
   if (rc == IDFX_OK) rc = cuda_check(e, cudaMalloc(&e.ctl, sizeof(Ctl)), "cudaMalloc(ctl)");
   if (rc == IDFX_OK) rc = cuda_check(e, cudaMallocHost(&e.ctl_host, sizeof(Ctl)), "cudaMallocHost(ctl)");
@@ -862,7 +872,7 @@ int idfx_gpu_create(const idfx_gpu_config* cfg, void* stream, idfx_gpu** out) {
   f.ezi = take(nc); f.ezj = take(nc); f.exj = take(nc); f.exk = take(nc); f.eyi = take(nc); f.eyk = take(nc);
   f.svx = take(nc); f.svy = take(nc); f.svz = take(nc);
   f.Ex1 = take(nc); f.Ex2 = take(nc); f.Ex3 = take(nc);
-  f.ex = take(nc); f.ey = take(nc); f.ez = take(nc);
+  f.ex = take(nc); f.ey = take(nc); f.ez = take(nc);  // in a row: learned corrections (launch_learned)
   for (int d = 0; d < 3; d++) {
     f.aL[d] = hll_emf ? take(nc) : nullptr;
     f.aR[d] = hll_emf ? take(nc) : nullptr;

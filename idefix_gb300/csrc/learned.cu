@@ -16,6 +16,7 @@
 #include "../../include/idefix_gb300.h"
 #include "engine.hpp"
 #include "learned.cuh"
+#include "learned_window.cuh"
 #include "sweep_cell.cuh"
 #include "train_tile.cuh"
 #include "umma.cuh"
@@ -203,8 +204,12 @@ constexpr StencilTable stencil_table() {
 __constant__ StencilTable kStencil = stencil_table();
 static_assert(NIN <= 256, "stencil element in a byte");
 
-__global__ void __launch_bounds__(LN, 1) k_learned_correct(Geo g, const float* __restrict__ Vc, LearnedDev L,
-                                                           Ctl* ctl, LBox box, float* __restrict__ Y) {
+// LEAN: the cells of a window (learned_window.cuh) in its direction, the
+// primitives rounded from FP64 here, the corrections at Y [16][room]
+template <bool LEAN>
+__global__ void __launch_bounds__(LN, 1)
+    k_learned_correct(Geo g, const float* __restrict__ Vc, const double* __restrict__ Vc64, LearnedDev L, Ctl* ctl,
+                      LBox box, LearnedWindow win, float* __restrict__ Y, long long room) {
   if (ctl->done) return;
   extern __shared__ __align__(128) unsigned char sm[];
   unsigned char* Xs = sm + LS_X;
@@ -270,30 +275,48 @@ __global__ void __launch_bounds__(LN, 1) k_learned_correct(Geo g, const float* _
     }
   };
   bool ok = __syncthreads_and(mbar_wait(bar + 1, 0u)) != 0;  // the weights
-  const int tiles = (int)((box.cells + LT - 1) / LT);
+  constexpr int ND = LEAN ? 1 : 3;  // directions of a tile
+  const long long cells = LEAN ? (long long)win.lines * win.per : box.cells;
+  const int tiles = (int)((cells + LT - 1) / LT);
   // this block's share of all tiles' directions, in a row
-  int item = (int)(3LL * tiles * blockIdx.x / gridDim.x);
-  const int end = (int)(3LL * tiles * (blockIdx.x + 1) / gridDim.x);
+  int item = (int)((long long)ND * tiles * blockIdx.x / gridDim.x);
+  const int end = (int)((long long)ND * tiles * (blockIdx.x + 1) / gridDim.x);
+  auto prim = [&](int v, long long c) -> float {
+    if constexpr (LEAN) return d2f_rn(Vc64[v * g.ncell + c]);
+    else return Vc[v * g.ncell + c];
+  };
   while (item < end && ok) {
-    const long long q = (long long)(item / 3) * LT + row;
-    const bool valid = q < box.cells;
+    const long long q = (long long)(item / ND) * LT + row;
+    const bool valid = q < cells;
     const unsigned p = valid ? (unsigned)q : 0u;  // cells of a box fit 31 bits
-    const int ix[3] = {box.lo[0] + (int)(p % (unsigned)box.m[0]),
-                       box.lo[1] + (int)(p / (unsigned)box.m[0] % (unsigned)box.m[1]),
-                       box.lo[2] + (int)(p / (unsigned)box.m[0] / (unsigned)box.m[1])};
+    int ix[3];
+    if constexpr (LEAN) {
+      const int d = win.dir, a = d == 0 ? 1 : 0, b = d == 2 ? 1 : 2;
+      unsigned line, pos;
+      window_cell(win, p, line, pos);
+      const unsigned na = (unsigned)(g.n[a] + 2 * g.ext);
+      const int at[3] = {g.beg[d] - 1 + (int)pos, g.beg[a] - g.ext + (int)(line % na),
+                         g.beg[b] - g.ext + (int)(line / na)};  // along d, a, b
+      ix[0] = d == 0 ? at[0] : at[1];
+      ix[1] = d == 0 ? at[1] : d == 1 ? at[0] : at[2];
+      ix[2] = d == 2 ? at[0] : at[2];
+    } else {
+      ix[0] = box.lo[0] + (int)(p % (unsigned)box.m[0]);
+      ix[1] = box.lo[1] + (int)(p / (unsigned)box.m[0] % (unsigned)box.m[1]);
+      ix[2] = box.lo[2] + (int)(p / (unsigned)box.m[0] / (unsigned)box.m[1]);
+    }
     const long long cc = cidx(g, ix[2], ix[1], ix[0]);
     for (int e = tid; e < 3 * LT; e += LN) out[e] = 0;
     __syncthreads();
     // ---- the scaled stencil, two variables per thread ------------------
     {
-      const float rho = Vc[cc], prs = Vc[4 * g.ncell + cc];
+      const float rho = prim(0, cc), prs = prim(4, cc);
       const float cs = sqrtf((float)g.gamma * prs / rho), sb = sqrtf(rho) * cs;
       int bad = 0;
 #pragma unroll
       for (int k = 0; k < 2; k++) {
         const int v = 2 * quarter + k;
-        const float* base = Vc + v * g.ncell;
-        const float cen = base[cc];
+        const float cen = prim(v, cc);
 #pragma unroll
         for (int oz = -1; oz <= 1; oz++)
 #pragma unroll
@@ -304,7 +327,7 @@ __global__ void __launch_bounds__(LN, 1) k_learned_correct(Geo g, const float* _
               // column more than the stencil has around it)
               const int nx = min(max(ix[0] + ox, 0), g.nt[0] - 1), ny = min(max(ix[1] + oy, 0), g.nt[1] - 1),
                         nz = min(max(ix[2] + oz, 0), g.nt[2] - 1);
-              const float s = base[cidx(g, nz, ny, nx)];
+              const float s = prim(v, cidx(g, nz, ny, nx));
               float x;
               if (v == 0 || v == 4) x = s / cen - 1.f;
               else if (v < 4) x = zdiv(s - cen, cs);
@@ -325,7 +348,8 @@ __global__ void __launch_bounds__(LN, 1) k_learned_correct(Geo g, const float* _
         if (bad & (1 << d)) out[d * LT + row] = 1;  // (any of the cell's threads)
     }
     __syncthreads();
-    for (int d = item % 3; d < 3 && item < end && ok; d++, item++) {
+    const int d0 = LEAN ? win.dir : item % 3;
+    for (int d = d0; d < (LEAN ? d0 + 1 : 3) && item < end && ok; d++, item++) {
       for (int c = 8 * quarter; c < K1; c += 32) {  // this direction's input, eight columns at a time
         alignas(16) __nv_bfloat16 t[8];
 #pragma unroll
@@ -349,7 +373,8 @@ __global__ void __launch_bounds__(LN, 1) k_learned_correct(Geo g, const float* _
           if (o / 4 != quarter) continue;
           float z = y[o] + bs[2 * NH + o];
           if (o == 0 && out[d * LT + row]) z = __int_as_float(0x7fffffff);
-          Y[((long long)d * NOUT + o) * g.ncell + cc] = z;
+          if constexpr (LEAN) Y[o * room + q] = z;
+          else Y[((long long)d * NOUT + o) * g.ncell + cc] = z;
         }
       }
     }
@@ -365,9 +390,9 @@ __global__ void __launch_bounds__(LN, 1) k_learned_correct(Geo g, const float* _
 }
 
 // the cell sweep with PLM plus the correction (sweep_cell.cuh, ORDER 5)
-template <int DIR>
+template <int DIR, bool WINDOW>
 __global__ void __launch_bounds__(kCellThreads, cell_resident(8))
-    k_sweep_learned(Geo g, Fields f, const Ctl* ctl, int invdt, int last_dir, LearnedRecon lr) {
+    k_sweep_learned(Geo g, Fields f, const Ctl* ctl, int invdt, int last_dir, LearnedRecon<WINDOW> lr) {
   extern __shared__ double learned_cell_sm[];
   d_sweep_cell<3, DIR, IDFX_LEARNED, kHLLD, double>(g, f, ctl, invdt, last_dir, blockIdx.x, learned_cell_sm, lr);
 }
@@ -437,39 +462,67 @@ struct LearnedModel {
   __nv_bfloat16* Wp = nullptr;
   float* w = nullptr;
   float *fmin = nullptr, *fmax = nullptr;
-  float* Y = nullptr;  // corrections [3][NOUT][ncell]
+  float* Y = nullptr;  // corrections [3][NOUT][ncell]; null: window by window where the corner EMFs lie
   unsigned long long* counters = nullptr;
   bool ranged = false;
 };
 
 namespace idfx {
 
+// the network over every cell of the box, or over a window's
+template <bool WINDOW>
+static void launch_correct(Engine& e, const LearnedModel& m, const LearnedWindow& win, float* Y, long long room) {
+  const LearnedDev L{m.Wp, m.w, m.ranged ? m.fmin : nullptr, m.ranged ? m.fmax : nullptr};
+  const LBox box = learned_box(e.g);
+  const long long cells = WINDOW ? (long long)win.lines * win.per : box.cells;
+  const long long items = (cells + LT - 1) / LT * (WINDOW ? 1 : 3);
+  mark_begin(e, kKLearned);
+  k_learned_correct<WINDOW><<<(unsigned)(items < e.sms ? items : e.sms), LN, SM_LEARN, e.stream>>>(
+      e.g, e.f.Vc32, e.f.Vc, L, e.ctl, box, win, Y, room);
+  mark_end(e);
+}
+
+// the cell sweep along d over `lines` lines
+template <bool WINDOW>
+static void launch_sweep_learned(Engine& e, int d, int invdt, int last, long long lines,
+                                 const LearnedRecon<WINDOW>& lr) {
+  const Geo& g = e.g;
+  const int nt = cell_threads(e.sms, [&](int t) { return cell_tiles(g, d, t, 8, lines); });
+  const unsigned grid = (unsigned)cell_tiles(g, d, nt, 8, lines);
+  const size_t sm = cell_smem_bytes(3, nt, 8);
+  mark_begin(e, kKSweepX + d);
+  if (d == 0) k_sweep_learned<0, WINDOW><<<grid, nt, sm, e.stream>>>(g, e.f, e.ctl, invdt, last, lr);
+  if (d == 1) k_sweep_learned<1, WINDOW><<<grid, nt, sm, e.stream>>>(g, e.f, e.ctl, invdt, last, lr);
+  if (d == 2) k_sweep_learned<2, WINDOW><<<grid, nt, sm, e.stream>>>(g, e.f, e.ctl, invdt, last, lr);
+  mark_end(e);
+}
+
 // the learned sweeps of one stage: the corrections of the three directions,
 // then direction after direction (the same InvDt modes as the plain sweeps: 1
 // first contribution, 2 accumulate; the last direction folds the CFL
-// maximum); states: face states instead
+// maximum); states: face states instead.  Without room for the corrections
+// of a box, each direction in windows, whose corrections the sweep takes
+// before the next window's replace them.
 static void launch_learned(Engine& e, int invdt, int fold_max, double* states) {
-  LearnedModel* m = static_cast<LearnedModel*>(e.learned);
-  LearnedDev L{m->Wp, m->w, m->ranged ? m->fmin : nullptr, m->ranged ? m->fmax : nullptr};
-  const LBox box = learned_box(e.g);
-  const long long tiles = (box.cells + LT - 1) / LT;
-  mark_begin(e, kKLearned);
-  k_learned_correct<<<(unsigned)(3 * tiles < e.sms ? 3 * tiles : e.sms), LN, SM_LEARN, e.stream>>>(e.g, e.f.Vc32, L, e.ctl,
-                                                                                          box, m->Y);
-  mark_end(e);
+  const LearnedModel& m = *static_cast<LearnedModel*>(e.learned);
+  const Geo& g = e.g;
+  if (m.Y) launch_correct<false>(e, m, LearnedWindow{}, m.Y, 0);
   for (int d = 0; d < 3; d++) {
-    if (e.only_dir >= 0 && e.only_dir != d) continue;
-    const int nt = cell_threads(e.sms, [&](int t) { return cell_tiles(e.g, d, t, 8); });
-    const unsigned grid = (unsigned)cell_tiles(e.g, d, nt, 8);
-    const size_t sm = cell_smem_bytes(3, nt, 8);
     const int inv = (invdt == 0) ? 0 : (d == 0 ? invdt : 2);
     const int last = fold_max && d == 2;
-    const LearnedRecon lr{m->Y, states, m->counters};
-    mark_begin(e, kKSweepX + d);
-    if (d == 0) k_sweep_learned<0><<<grid, nt, sm, e.stream>>>(e.g, e.f, e.ctl, inv, last, lr);
-    if (d == 1) k_sweep_learned<1><<<grid, nt, sm, e.stream>>>(e.g, e.f, e.ctl, inv, last, lr);
-    if (d == 2) k_sweep_learned<2><<<grid, nt, sm, e.stream>>>(e.g, e.f, e.ctl, inv, last, lr);
-    mark_end(e);
+    const unsigned lines = (unsigned)cell_lines(g, d), per = (unsigned)(g.n[d] + 2);
+    if (m.Y) {
+      launch_sweep_learned(e, d, inv, last, lines, LearnedRecon<false>{m.Y, 0, LearnedWindow{}, states, m.counters});
+      continue;
+    }
+    float* Y = reinterpret_cast<float*>(e.f.ex);  // ex, ey and ez, one after the other
+    const long long room = 6 * g.ncell / NOUT;
+    for (unsigned l = 0; l < lines;) {
+      const LearnedWindow win = window_from(d, l, lines, per, (unsigned)room);
+      launch_correct<true>(e, m, win, Y, room);
+      launch_sweep_learned(e, d, inv, last, win.lines, LearnedRecon<true>{Y, room, win, states, m.counters});
+      l += win.lines;
+    }
   }
 }
 
@@ -586,9 +639,15 @@ int idfx_gpu_set_learned(idfx_gpu* hg, const float* params, const float* fmin, c
     ok = ok && cudaMalloc(&m->fmin, sizeof(float) * NIN) == cudaSuccess;
     ok = ok && cudaMalloc(&m->fmax, sizeof(float) * NIN) == cudaSuccess;
     ok = ok && cudaMalloc(&m->counters, sizeof(unsigned long long) * 2) == cudaSuccess;
-    ok = ok && cudaMalloc(&m->Y, sizeof(float) * 3 * NOUT * e.g.ncell) == cudaSuccess;
-    ok = ok && cudaFuncSetAttribute(k_learned_correct, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)SM_LEARN) ==
-                   cudaSuccess;
+    ok = ok && cudaFuncSetAttribute(k_learned_correct<false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)SM_LEARN) == cudaSuccess;
+    ok = ok && cudaFuncSetAttribute(k_learned_correct<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                    (int)SM_LEARN) == cudaSuccess;
+    // no room for the whole box's corrections: window by window (launch_learned)
+    if (ok && e.f.Vc32 && cudaMalloc(&m->Y, sizeof(float) * 3 * NOUT * e.g.ncell) != cudaSuccess) {
+      m->Y = nullptr;
+      cudaGetLastError();
+    }
     if (!ok) {
       free_learned(e);
       e.err = "set_learned: CUDA allocation failed";

@@ -1,6 +1,7 @@
 // Flux sweeps with one thread per cell (every direction, 2-D and 3-D): the
 // FP64 sweeps, and the FP32 sweeps of the mixed path up to a size.
 #pragma once
+#include "learned_window.cuh"
 #include "mhd_kernels.cuh"
 
 namespace idfx {
@@ -78,14 +79,20 @@ inline int cell_threads(int sms, Tiles tiles) {
   return nt;
 }
 
-// tiles of nt cells of the lines along dir
-__host__ inline long long cell_tiles(const Geo& g, int dir, int nt, size_t size) {
-  const int a = (dir == 0) ? 1 : 0, b = (dir == 2) ? 1 : 2, cols = cell_cols(dir, size, nt);
+// lines along dir, and the tiles of nt cells of `lines` of them (all)
+__host__ inline long long cell_lines(const Geo& g, int dir) {
+  const int a = (dir == 0) ? 1 : 0, b = (dir == 2) ? 1 : 2;
+  return (long long)(g.n[a] + 2 * g.ext) * (g.D == 3 ? g.n[b] + 2 * g.ext : 1);
+}
+__host__ inline long long cell_tiles(const Geo& g, int dir, int nt, size_t size, long long lines) {
+  const int cols = cell_cols(dir, size, nt);
   const int lead = (g.order == 4) ? 1 : 0;  // PPM's extra position
   const int step = nt / cols - 2 - lead;
-  const long long lines = (long long)(g.n[a] + 2 * g.ext) * (g.D == 3 ? g.n[b] + 2 * g.ext : 1);
   const long long total = (lines + cols - 1) / cols * (g.n[dir] + 2 + lead);
   return (total - 2 - lead + step - 1) / step;
+}
+__host__ inline long long cell_tiles(const Geo& g, int dir, int nt, size_t size) {
+  return cell_tiles(g, dir, nt, size, cell_lines(g, dir));
 }
 
 // shared memory of a block of nt threads: right-face states (PPM: before
@@ -94,18 +101,23 @@ __host__ __device__ constexpr size_t cell_smem_bytes(int D, int nt, size_t size)
   return size * (size_t)((2 * D + 1) + (D + 2) + 1) * (size_t)nt;
 }
 
-// the learned order (5, 3-D): corrections Y [3][16][ncell] of the PLM states
-// (learned.cu), where the face states go instead of the sweep (or null), and
-// the counts of evaluated and fallen-back cells
+// the learned order (5, 3-D): corrections Y of the PLM states (learned.cu) -
+// [3][16][ncell], or those of a window's cells [16][room] -, where the face
+// states go instead of the sweep (or null), and the counts of evaluated and
+// fallen-back cells
+template <bool WINDOW>
 struct LearnedRecon {
+  static constexpr bool window = WINDOW;
   const float* Y;
+  long long room;
+  LearnedWindow win;
   double* states;
   unsigned long long* counters;
 };
 
-template <int D, int DIR, int ORDER, int SOLVER, typename T>
+template <int D, int DIR, int ORDER, int SOLVER, typename T, typename LR = LearnedRecon<false>>
 __device__ __forceinline__ void d_sweep_cell(const Geo& g, const Fields& f, const Ctl* ctl, int invdt, int last_dir,
-                                             unsigned tile, T* sm, const LearnedRecon& lr = LearnedRecon{}) {
+                                             unsigned tile, T* sm, const LR& lr = LR{}) {
   if (ctl->done) return;
   using v = Var<D>;
   using dd = Dir<D, DIR>;
@@ -132,8 +144,10 @@ __device__ __forceinline__ void d_sweep_cell(const Geo& g, const Fields& f, cons
   const unsigned q = tile * (unsigned)(npos - 2 - E) + (unsigned)t;
   const unsigned bundle = q / P;
   const int p = (int)(q - bundle * P);
-  const unsigned line = bundle * cols + (unsigned)(tid - t * cols);
-  const bool valid = line < nA * nB;
+  unsigned line = bundle * cols + (unsigned)(tid - t * cols);
+  const unsigned lines = LR::window ? lr.win.lines : nA * nB;
+  const bool valid = line < lines;
+  if constexpr (LR::window) line += lr.win.line0;
   int idx[3];
   idx[DIR] = g.beg[DIR] - 1 - E + p;
   idx[A] = g.beg[A] - g.ext + (int)(valid ? line % nA : 0);
@@ -208,15 +222,18 @@ __device__ __forceinline__ void d_sweep_cell(const Geo& g, const Fields& f, cons
         Recon<2>::plm(w1, w1 - w0, w2 - w1, false, vl[n], vr[n]);
       }
       const T cs = root(quot(g.gamma * cen[v::PRS], cen[v::RHO])), sb = root(cen[v::RHO]) * cs;
-      const float* Y = lr.Y + (long long)DIR * 16 * g.ncell + cc;
+      const float* Y = lr.Y;
+      if constexpr (LR::window) Y += window_index(lr.win, line, (unsigned)p);
+      else Y += (long long)DIR * 16 * g.ncell + cc;
+      const long long out = LR::window ? lr.room : g.ncell;  // from one output to the next
       T cl[NV], cr[NV];
 #pragma unroll
       for (int rv = 0; rv < 8; rv++) {
         if (rv == 5) continue;  // normal field: the face value is used
         const int n = rv == 0 || rv == 4 ? rv : (rv < 4 ? 1 : 5) + (DIR + rv - (rv < 4 ? 1 : 5)) % 3;
         const T sc = rv == 0 ? cen[v::RHO] : rv == 4 ? cen[v::PRS] : rv < 4 ? cs : sb;
-        cl[n] = vl[n] + f2d_exact(Y[rv * g.ncell]) * sc;
-        cr[n] = vr[n] + f2d_exact(Y[(8 + rv) * g.ncell]) * sc;
+        cl[n] = vl[n] + f2d_exact(Y[rv * out]) * sc;
+        cr[n] = vr[n] + f2d_exact(Y[(8 + rv) * out]) * sc;
       }
       // plain PLM where the stencil is outside the trained range (a NaN) or a
       // corrected density or pressure is not positive
@@ -242,7 +259,7 @@ __device__ __forceinline__ void d_sweep_cell(const Geo& g, const Fields& f, cons
     const bool owner = valid && (t < npos - 2 || blockIdx.x == gridDim.x - 1);
     const unsigned fell = __ballot_sync(0xffffffffu, owner && fall);
     if ((tid & 31) == 0 && fell) atomicAdd(lr.counters + 1, (unsigned long long)__popc(fell));
-    if (tile == 0 && tid == 0) atomicAdd(lr.counters, (unsigned long long)nA * nB * P);
+    if (tile == 0 && tid == 0) atomicAdd(lr.counters, (unsigned long long)lines * P);
     if (lr.states) return;
   } else if (valid) {
     const Recip l3{g.l3b[DIR], g.l3y[DIR]};
