@@ -111,10 +111,13 @@ __global__ void k_uc_field_all(Geo g, Fields f, int to_prim) {
 }
 
 // the cell-centred field of Uc from the faces over the active cells, as the
-// stage end forms it (mixed path, whose stage ends do not store it)
+// stage end forms it (mixed path, whose stage ends do not store it); ctl: only
+// where a stage end left this Uc (a run may have had nothing to do)
 template <int D>
-__global__ void k_uc_field_active(Geo g, Fields f) {
+__global__ void k_uc_field_active(Geo g, Fields f, const Ctl* ctl) {
   using v = Var<D>;
+  chain_wait();
+  if (ctl && !ctl->uc_fresh) return;
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long tot = (long long)g.n[0] * g.n[1] * (D == 3 ? g.n[2] : 1);
   if (tid >= tot) return;
@@ -1093,13 +1096,24 @@ int idfx_gpu_sizes(const idfx_gpu* h, int* nvar, int* nghost, long long* vc_len,
   return IDFX_OK;
 }
 
+// the field part of Uc that the mixed path's stage ends left out, before
+// anything writes Uc or the faces it comes from.  A periodic block's arrays may be
+// uploaded without (its Uc is then rebuilt from the new faces); with walls Uc
+// stays the run's.
+static void complete_uc(Engine& e) {
+  if (!e.uc_field_stale) return;
+  IDFX_CHAIN_D(k_uc_field_active, nblocks(n_active(e.g)), kThreads, e.g, e.f, e.g.nonper ? e.ctl : nullptr);
+  e.uc_field_stale = false;
+}
+
 static int copy_state(idfx_gpu* h, const double* Vc, const double* Vs, cudaMemcpyKind kind, bool up) {
   if (!h) return IDFX_ERR_STATE;
   Engine& e = h->e;
   const size_t bc = sizeof(double) * (2 * e.g.D + 2) * e.g.ncell;
   const size_t bs = sizeof(double) * e.g.D * e.g.nface;
-  const bool d2d = (kind == cudaMemcpyDeviceToDevice);  // by a kernel (see k_copy_f64)
+  const bool d2d = (kind == cudaMemcpyDeviceToDevice);  // by a kernel (k_copy_state)
   if (up) {
+    if (e.g.nonper) complete_uc(e);
     if (d2d) {
       copy_device(e, e.f.Vc, Vc, e.f.Vs, Vs, e.ctl);
     } else {
@@ -1133,10 +1147,7 @@ int idfx_gpu_download_prim_device(idfx_gpu* h, double* Vc, double* Vs) {
 int idfx_gpu_download_cons(idfx_gpu* h, double* Uc) {
   if (!h || !Uc) return IDFX_ERR_STATE;
   Engine& e = h->e;
-  if (e.uc_field_stale) {  // mixed path: the field part of Uc from the faces
-    IDFX_DISPATCH_D(k_uc_field_active, nblocks(n_active(e.g)), kThreads, e.g, e.f);
-    e.uc_field_stale = false;
-  }
+  complete_uc(e);
   IDFX_CK(cudaMemcpyAsync(Uc, e.f.Uc, sizeof(double) * (2 * e.g.D + 2) * e.g.ncell, cudaMemcpyDeviceToHost,
                           e.stream));
   IDFX_CK(cudaStreamSynchronize(e.stream));
@@ -1207,7 +1218,10 @@ int idfx_gpu_run(idfx_gpu* h, double tstop, long long max_cycles) {
 // ---------------------------------------------------------------------------
 // the building blocks run whatever the time-integrator control says; after
 // any of them the next cycle rebuilds the conserved state from Vc
-static void clear_done(Engine& e) { ctl_clear(e, kClrUcFresh | kClrDone); }
+static void clear_done(Engine& e) {
+  complete_uc(e);
+  ctl_clear(e, kClrUcFresh | kClrDone);
+}
 
 static int sync_status(Engine& e) {
   IDFX_CK(cudaGetLastError());
