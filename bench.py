@@ -442,8 +442,7 @@ def run_ours(args, world, rank, local):
                          "frac": (achieved_gbs / hbm_peak) if achieved_gbs else None,
                          "traffic": traffic, "kernel": dom, "peak_kind": peak_kind,
                          "bytes_per_cell": sweep_bytes_per_cell,
-                         "traffic_note": "ncu dram read+write per active cell of the 128^3 sweep (segments 64), "
-                                         "scaled to 256^3 by the processed columns, x 256^3 cells",
+                         "traffic_note": "ncu dram read+write per active cell of the 128^3 sweep, x 256^3 cells",
                          "note": "FP64-issue bound (GB300 FP64 ~1.2 TFLOP/s): see fp64_roofline"},
             "fp64_roofline": fp64_roof,
             "fp64_flop": fp64_flop_roof(value / world, fp64_peak) if args.precision == "fp64" else None,

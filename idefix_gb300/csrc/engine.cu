@@ -436,8 +436,7 @@ void launch_find_shock(Engine& e) {
 void ctl_clear(Engine& e, int what) { k_ctl_clear<<<1, 1, 0, e.stream>>>(e.ctl, what); }
 void ctl_push(Engine& e) { k_ctl_put<<<1, 1, 0, e.stream>>>(e.ctl, *e.ctl_host); }
 
-// device -> device copy of n doubles on the engine's stream (SMs, not a copy engine)
-// Vc and Vs (null: not that part) on the device
+// Vc and Vs (null: not that part) from device arrays on the engine's stream (SMs, not a copy engine)
 void copy_device(Engine& e, double* vc, const double* vc0, double* vs, const double* vs0, Ctl* ctl) {
   const CopyF64 a{vc, vc0, vc && vc0 ? (2LL * e.g.D + 2) * e.g.ncell : 0LL};
   const CopyF64 b{vs, vs0, vs && vs0 ? (long long)e.g.D * e.g.nface : 0LL};
@@ -673,9 +672,8 @@ bool tile_sweep_eligible(Engine& e, int dir) {
 
 // Validation of a block configuration and the block's grid and geometry:
 // ghost zones (grid.cpp:60-65), cell widths (gridHost.cpp:80-86), face
-// areas (makeGeometry.cpp:146-147,178-179,201-202), the correctly rounded
-// reciprocals of the exact quotient forms, and the CT extension of the
-// sweeps.  Shared by the handle (idfx_gpu_create) and the allocation-free
+// areas (makeGeometry.cpp:146-147,178-179,201-202), LimO3's squared widths,
+// and the CT extension of the sweeps.  Shared by the handle (idfx_gpu_create) and the allocation-free
 // stage, so that both set up a block identically.
 int block_geometry(const idfx_gpu_config* cfg, Geo& g) {
   if (!cfg) return IDFX_ERR_STATE;
@@ -729,12 +727,9 @@ int block_geometry(const idfx_gpu_config* cfg, Geo& g) {
   }
   g.gamma = cfg->gamma;
   g.gm1 = cfg->gamma - 1.0;
-  g.rgm1 = 1.0 / g.gm1;  // correctly rounded reciprocals (Markstein quotients)
   for (int d = 0; d < 3; d++) {
-    g.rdx[d] = 1.0 / g.dx[d];
     const double e = 0.1 * g.dx[d];  // LimO3's r dx, squared as the limiter does
     g.l3b[d] = e * e;
-    g.l3y[d] = 1.0 / g.l3b[d];
   }
   g.ext = 1;  // hlldMHD.hpp:30-49: uct_hll(d) with HLLD/HLL needs nghost cells
   if ((g.emf == kEmfUctHll || g.emf == kEmfUctHlld) && (g.solver == kHLLD || g.solver == kHLL)) g.ext = g.ng;

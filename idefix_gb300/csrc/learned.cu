@@ -1,8 +1,7 @@
 // Learned interface-state correction (see learned.cuh): the trainer around
-// the training kernels (train_tile.cuh), the coarsening of fine snapshots and
-// the learned sweep of the ORDER 5 solver (network inference fused with the
-// reconstruction, the Riemann solve and the flux difference), with their C
-// ABI.
+// the training kernels (train_tile.cuh), the coarsening of fine snapshots, the
+// network's corrections of a stage of the ORDER 5 solver and its sweeps (the
+// cell sweep on the corrected PLM states), with their C ABI.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -121,7 +120,7 @@ __global__ void k_coarsen(const double* __restrict__ Vc, const double* __restric
 // ---------------------------------------------------------------------------
 // Learned correction (ORDER 5): the network over every cell whose face states
 // a sweep reconstructs, for the three directions in one launch; the sweeps
-// (k_sweep_learned: the cell sweep of the FP64 path) then add the correction
+// (k_sweep_learned: the cell sweep of the FP64 path) add the correction
 // to the PLM states.  Together in one kernel per direction, 128 of its 256
 // threads solved FP64 Riemann problems while the tensor core and the other
 // half waited, features were gathered from FP64 three times over, and a 32^3
@@ -434,7 +433,8 @@ __global__ void __launch_bounds__(128, 1) k_umma_check(int N, int K, const __nv_
   umma::fence_after_sync();
   const uint32_t taddr = *slot;
   if (tid == 0) {
-    umma::mma_tile(taddr, umma::smem_addr(As), umma::smem_addr(Bs), K, umma::idesc_bf16_f32(128, N), false);
+    umma::mma_run(taddr, umma::along_columns(umma::smem_addr(As), K), umma::along_columns(umma::smem_addr(Bs), K), 128,
+                  N, K);
     umma::mma_commit(bar);
   }
   const bool ok = umma::mbar_wait_bounded(bar, 0, umma::kMmaSpin);

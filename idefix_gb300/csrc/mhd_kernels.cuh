@@ -43,9 +43,7 @@ struct Geo {
   double gamma, gm1;
   int ext;  // perpendicular extension of the flux sweeps for CT
   double shock_smoothing;  // [Hydro] shockFlattening value (flags in Fields::shock)
-  double rgm1;    // RN(1 / gm1), for the FP64 Riemann solvers
-  double rdx[3];  // RN(1 / dx[d]), for the InvDt quotient
-  double l3b[3], l3y[3];  // LimO3: (0.1 dx[d])^2 and RN(1 / that)
+  double l3b[3];  // LimO3: (0.1 dx[d])^2
   int bc[3][2];  // boundary type per direction and side (IDFX_BC_*: 0 periodic)
   int nonper;    // some direction is not periodic: ghosts filled by k_bc_* first
 };
@@ -718,7 +716,7 @@ __device__ __forceinline__ void d_sweep_march(const Geo& g, const Fields& f, con
   const long long f0 = fidx(g, idx[2], idx[1], idx[0]);
   const double* vs = f.Vs + DIR * g.nface;
   const T dxd = (T)g.dx[DIR];
-  const Recip l3{g.l3b[DIR], g.l3y[DIR]};
+  const double l3 = g.l3b[DIR];
   const T gam = (T)g.gamma;
   T w[NV][W];
   T vrp[NV];            // right-face state of the previous cell
@@ -798,7 +796,7 @@ __device__ __forceinline__ void d_sweep_march(const Geo& g, const Fields& f, con
       vL[dd::BXn] = bn;
       vR[dd::BXn] = bn;
       RiemannOut<D, T> r;
-      riemann<D, DIR, SOLVER>(gam, (T)g.rgm1, vL, vR, r);
+      riemann<D, DIR, SOLVER>(gam, vL, vR, r);
       store_emf<D, DIR>(g, f, cc, r, vL, vR);
       if (active_col) {
         // flux x area and the flux difference in FP32; the conserved state
@@ -889,7 +887,7 @@ __device__ __forceinline__ void d_sweep_xwarp(const Geo& g, const Fields& f, con
   const int base = beg - 1;  // first cell reconstructed (left state of face beg)
   const T gam = (T)g.gamma;
   const T dxd = (T)g.dx[0];
-  const Recip l3{g.l3b[0], g.l3y[0]};
+  const double l3 = g.l3b[0];
   const T dtdVT = (T)ctl->dtdV;
   const T areaT = (T)g.A[0];
   const T invdxT = T(1) / (T)g.dx[0];
@@ -972,7 +970,7 @@ __device__ __forceinline__ void d_sweep_xwarp(const Geo& g, const Fields& f, con
       vL[dd::BXn] = bn;
       vR[dd::BXn] = bn;
       RiemannOut<D, T> r;
-      riemann<D, 0, SOLVER>(gam, (T)g.rgm1, vL, vR, r);
+      riemann<D, 0, SOLVER>(gam, vL, vR, r);
       store_emf<D, 0>(g, f, cc, r, vL, vR);
 #pragma unroll
       for (int n = 0; n < v::BX1; n++) FA[n] = r.F[n] * areaT;
@@ -1125,7 +1123,7 @@ __device__ __forceinline__ void d_sweep_xbulk(const Geo& g, const Fields& f, con
   const int beg = g.beg[0], end = g.end[0];
   const T gam = (T)g.gamma;
   const T dxd = (T)g.dx[0];
-  const Recip l3{g.l3b[0], g.l3y[0]};
+  const double l3 = g.l3b[0];
   const T dtdVT = (T)ctl->dtdV;
   const T areaT = (T)g.A[0];
   const T invdxT = T(1) / (T)g.dx[0];
@@ -1209,7 +1207,7 @@ __device__ __forceinline__ void d_sweep_xbulk(const Geo& g, const Fields& f, con
       vL[dd::BXn] = bn;
       vR[dd::BXn] = bn;
       RiemannOut<D, T> r;
-      riemann<D, 0, SOLVER>(gam, (T)g.rgm1, vL, vR, r);
+      riemann<D, 0, SOLVER>(gam, vL, vR, r);
       store_emf<D, 0>(g, f, cc, r, vL, vR);
 #pragma unroll
       for (int n = 0; n < NU; n++) FA[n] = r.F[n] * areaT;

@@ -17,7 +17,6 @@
 
 #include "exact_ops.cuh"
 #include "intdiv.cuh"
-#include "rdiv.cuh"
 #include "seeddiv.cuh"
 
 namespace idfx {
@@ -66,9 +65,8 @@ __device__ __forceinline__ float fdiv_corrected(float a, float b) {
 }
 
 // division: FP64 IEEE correctly rounded (the bit-identical path; from FP32
-// seeds, three FP64-pipe operations instead of the hardware sequence's
-// seven, seeddiv.cuh); FP32 (the mixed path, FP32-accurate rather than
-// bit-matched) fdiv_corrected
+// seeds and integers, off the FP64 pipe, seeddiv.cuh); FP32 (the mixed path,
+// FP32-accurate rather than bit-matched) fdiv_corrected
 template <typename T>
 __device__ __forceinline__ T dv(T a, T b) {
   if constexpr (sizeof(T) == 4) {
@@ -135,12 +133,10 @@ __device__ __forceinline__ T sumsq(T a, T b, T c) {
 // cons <-> prim (convertConsToPrim.hpp:15-100; eos_adiabatic.hpp:38-45)
 // gm1 = gamma - 1.0, evaluated once on the host
 // ---------------------------------------------------------------------------
-// QUOT: how p / gm1 is formed - 0 the hardware division, 1 on the integer
-// pipe (whole-array kernels), 2 from rgm1 = RN(1 / gm1) formed once on the
-// host (Riemann solvers, FP64: Markstein's correction, rdiv.cuh); all three
-// give the correctly rounded quotient.  bb = B^2 where the caller has it (HAVE_B2)
-template <int D, int QUOT = 0, bool HAVE_B2 = false, typename T>
-__device__ __forceinline__ void prim_to_cons(T gm1, T* U, const T* V, T rgm1 = T(0), T bb = T(0)) {
+// IPIPE: p / gm1 with the whole-array kernels' quotient (dvi), else with the
+// sweeps' (dv); both correctly rounded.  bb = B^2 where the caller has it (HAVE_B2)
+template <int D, bool IPIPE = false, bool HAVE_B2 = false, typename T>
+__device__ __forceinline__ void prim_to_cons(T gm1, T* U, const T* V, T bb = T(0)) {
   using v = Var<D>;
   U[v::RHO] = V[v::RHO];
   U[v::MX1] = V[v::MX1] * V[v::RHO];
@@ -159,12 +155,9 @@ __device__ __forceinline__ void prim_to_cons(T gm1, T* U, const T* V, T rgm1 = T
     if constexpr (!HAVE_B2) mag = sumsq<2>(U[v::BX1], U[v::BX2], z);
   }
   T pq;
-  if constexpr (QUOT == 1) {
+  if constexpr (IPIPE) {
     pq = dvi(V[v::PRS], gm1);
-  } else if constexpr (QUOT == 2 && sizeof(T) == 8) {
-    pq = quot(V[v::PRS], gm1);
   } else {
-    (void)rgm1;
     pq = dv(V[v::PRS], gm1);
   }
   if constexpr (sizeof(T) == 8) {  // the halves exact on the integer pipe
@@ -323,7 +316,7 @@ __device__ __forceinline__ T lim_mc(T dvp, T dvm) {  // :68-76
 // FP64 path divides by it and by 3 with Markstein's correction (rdiv.cuh),
 // bit-identical to the divisions
 template <typename T>
-__device__ __forceinline__ T lim_limo3(T dvp, T dvm, T dx, const Recip& e2) {  // :25-52
+__device__ __forceinline__ T lim_limo3(T dvp, T dvm, T dx, double e2) {  // :25-52
   const T r = T(0.1), eps = T(1.e-12);
   T th = dv(dvm, dvp + T(1.e-16));
   T q;
@@ -339,7 +332,7 @@ __device__ __forceinline__ T lim_limo3(T dvp, T dvm, T dx, const Recip& e2) {  /
   T psi = fmax(T(0), c);
   T eta = r * dx;
   if constexpr (sizeof(T) == 8) {
-    eta = quot(dvm * dvm + dvp * dvp, e2.b);
+    eta = quot(dvm * dvm + dvp * dvp, e2);
   } else {
     (void)e2;
     eta = dv(dvm * dvm + dvp * dvp, eta * eta);
@@ -471,9 +464,9 @@ struct Recon {
   // shock: the cell is flagged by shock flattening (minmod slope, PLM and
   // LimO3 only, extrapolateToFaces.hpp:96-218)
   template <typename T>
-  // e2: (0.1 dx)^2 and its reciprocal (LimO3, FP64 path; Geo::l3b, l3y)
+  // e2: (0.1 dx)^2 (LimO3, FP64 path; Geo::l3b)
   __device__ __forceinline__ static void cell(const T* w, T dx, bool pos, T& vl, T& vr, bool shock = false,
-                                              const Recip& e2 = Recip{0.0, 0.0}) {
+                                              double e2 = 0.0) {
     if constexpr (ORDER == 1) {
       vl = w[0];
       vr = w[0];
@@ -591,7 +584,7 @@ __device__ __forceinline__ T half_b2(const T* v) {
 // sweep, the 256^3 x / y / z sweeps of a cycle 19.1 / 19.3 / 19.2 -> 17.9 / 18.3 /
 // 18.0 ms).
 template <int D, int DIR, typename T>
-__device__ __forceinline__ void riemann_hlld(T gamma, T rgm1, const T* vL, const T* vR, RiemannOut<D, T>& r) {
+__device__ __forceinline__ void riemann_hlld(T gamma, const T* vL, const T* vR, RiemannOut<D, T>& r) {
   using v = Var<D>;
   using d = Dir<D, DIR>;
   constexpr int NV = v::NV;
@@ -699,7 +692,7 @@ __device__ __forceinline__ void riemann_hlld(T gamma, T rgm1, const T* vL, const
   T vS[NV], uS[NV];
 #pragma unroll
   for (int n = 0; n < NV; n++) vS[n] = sideL ? vL[n] : vR[n];
-  prim_to_cons<D, 2, true>(gm1, uS, vS, rgm1, sideL ? bbL : bbR);
+  prim_to_cons<D, false, true>(gm1, uS, vS, sideL ? bbL : bbR);
   uS[Xn] = sideL ? uL[Xn] : uR[Xn];
   T* F = r.F;
   const T pt = sideL ? ptL : ptR;
@@ -782,7 +775,7 @@ __device__ __forceinline__ void riemann_hlld(T gamma, T rgm1, const T* vL, const
 
 // HLL (hllMHD.hpp:154-453; the Hall whistler term is not part of ideal MHD)
 template <int D, int DIR, typename T>
-__device__ __forceinline__ void riemann_hll(T gamma, T rgm1, const T* vL, const T* vR, RiemannOut<D, T>& r) {
+__device__ __forceinline__ void riemann_hll(T gamma, const T* vL, const T* vR, RiemannOut<D, T>& r) {
   using v = Var<D>;
   using d = Dir<D, DIR>;
   constexpr int NV = v::NV;
@@ -799,8 +792,8 @@ __device__ __forceinline__ void riemann_hll(T gamma, T rgm1, const T* vL, const 
   r.sr = sr;
   r.cmax = fmax(fabs(sl), fabs(sr));
   const T gm1 = gamma - T(1);
-  prim_to_cons<D, 2>(gm1, uL, vL, rgm1);
-  prim_to_cons<D, 2>(gm1, uR, vR, rgm1);
+  prim_to_cons<D>(gm1, uL, vL);
+  prim_to_cons<D>(gm1, uR, vR);
   phys_flux<D, DIR>(fluxL, vL, uL);
   phys_flux<D, DIR>(fluxR, vR, uR);
   T* F = r.F;
@@ -836,7 +829,7 @@ __device__ __forceinline__ void riemann_hll(T gamma, T rgm1, const T* vL, const 
 
 // TVDLF / Rusanov (tvdlfMHD.hpp:140-232)
 template <int D, int DIR, typename T>
-__device__ __forceinline__ void riemann_tvdlf(T gamma, T rgm1, const T* vL, const T* vR, RiemannOut<D, T>& r) {
+__device__ __forceinline__ void riemann_tvdlf(T gamma, const T* vL, const T* vR, RiemannOut<D, T>& r) {
   using v = Var<D>;
   using d = Dir<D, DIR>;
   constexpr int NV = v::NV;
@@ -856,8 +849,8 @@ __device__ __forceinline__ void riemann_tvdlf(T gamma, T rgm1, const T* vL, cons
   r.cmax = cmax;
   T fluxL[NV], fluxR[NV];
   const T gm1 = gamma - T(1);
-  prim_to_cons<D, 2>(gm1, r.uL, vL, rgm1);
-  prim_to_cons<D, 2>(gm1, r.uR, vR, rgm1);
+  prim_to_cons<D>(gm1, r.uL, vL);
+  prim_to_cons<D>(gm1, r.uR, vR);
   phys_flux<D, DIR>(fluxL, vL, r.uL);
   phys_flux<D, DIR>(fluxR, vR, r.uR);
 #pragma unroll
@@ -866,7 +859,7 @@ __device__ __forceinline__ void riemann_tvdlf(T gamma, T rgm1, const T* vL, cons
 
 // Roe with the entropy fix (roeMHD.hpp:175-650, energy equation branch)
 template <int D, int DIR, typename T>
-__device__ __forceinline__ void riemann_roe(T gamma, T rgm1, const T* vL, const T* vR, RiemannOut<D, T>& r) {
+__device__ __forceinline__ void riemann_roe(T gamma, const T* vL, const T* vR, RiemannOut<D, T>& r) {
   using v = Var<D>;
   using d = Dir<D, DIR>;
   constexpr int NV = v::NV;
@@ -882,8 +875,8 @@ __device__ __forceinline__ void riemann_roe(T gamma, T rgm1, const T* vL, const 
 #pragma unroll
   for (int n = 0; n < NV; n++) dV[n] = vR[n] - vL[n];
   const T gm1 = gamma - T(1);
-  prim_to_cons<D, 2>(gm1, uL, vL, rgm1);
-  prim_to_cons<D, 2>(gm1, uR, vR, rgm1);
+  prim_to_cons<D>(gm1, uL, vL);
+  prim_to_cons<D>(gm1, uR, vR);
 #pragma unroll
   for (int n = 0; n < NV; n++) dU[n] = uR[n] - uL[n];
   phys_flux<D, DIR>(fluxL, vL, uL);
@@ -1094,13 +1087,12 @@ __device__ __forceinline__ void riemann_roe(T gamma, T rgm1, const T* vL, const 
   }
 }
 
-// rgm1 = RN(1 / (gamma - 1)), used by the FP64 path
 template <int D, int DIR, int SOLVER, typename T>
-__device__ __forceinline__ void riemann(T gamma, T rgm1, const T* vL, const T* vR, RiemannOut<D, T>& r) {
-  if constexpr (SOLVER == kHLLD) riemann_hlld<D, DIR>(gamma, rgm1, vL, vR, r);
-  if constexpr (SOLVER == kHLL) riemann_hll<D, DIR>(gamma, rgm1, vL, vR, r);
-  if constexpr (SOLVER == kROE) riemann_roe<D, DIR>(gamma, rgm1, vL, vR, r);
-  if constexpr (SOLVER == kTVDLF) riemann_tvdlf<D, DIR>(gamma, rgm1, vL, vR, r);
+__device__ __forceinline__ void riemann(T gamma, const T* vL, const T* vR, RiemannOut<D, T>& r) {
+  if constexpr (SOLVER == kHLLD) riemann_hlld<D, DIR>(gamma, vL, vR, r);
+  if constexpr (SOLVER == kHLL) riemann_hll<D, DIR>(gamma, vL, vR, r);
+  if constexpr (SOLVER == kROE) riemann_roe<D, DIR>(gamma, vL, vR, r);
+  if constexpr (SOLVER == kTVDLF) riemann_tvdlf<D, DIR>(gamma, vL, vR, r);
 }
 
 }  // namespace idfx

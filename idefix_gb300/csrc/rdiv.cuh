@@ -1,10 +1,10 @@
 // FP64 division by a divisor whose correctly rounded reciprocal is known.
 //
-// The FP64 pipe of this GPU is narrow and the flux sweeps are bound by it;
-// a hardware-sequence division costs several of its instructions.  Where a
-// divisor is a constant of the run (LimO3's cell width and its three), its
-// reciprocal is formed once and each quotient takes three FP64 operations,
-// bit-identical to a / b:
+// Three FP64 operations per quotient where a hardware-sequence division takes
+// seven, bit-identical to a / b.  The flux sweeps took it for divisors that are
+// constants of the run or shared; their quotients are formed off the FP64 pipe now
+// (seeddiv.cuh), and this form stands with the others in the division self-check
+// (idfx_check_division) and its host test alone:
 //   y = RN(1/b)            (host division, or the device's correctly rounded
 //                           reciprocal __drcp_rn)
 //   q = RN(a y)            (within one ulp of a / b)

@@ -35,7 +35,7 @@
 #include <stdint.h>
 
 #include "fpconv.cuh"  // fbits / ffrom
-#include "rdiv.cuh"
+#include "intdiv.cuh"  // rcp_seed
 
 namespace idfx {
 

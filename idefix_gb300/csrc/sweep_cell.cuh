@@ -262,7 +262,7 @@ __device__ __forceinline__ void d_sweep_cell(const Geo& g, const Fields& f, cons
     if (tile == 0 && tid == 0) atomicAdd(lr.counters, (unsigned long long)lines * P);
     if (lr.states) return;
   } else if (valid) {
-    const Recip l3{g.l3b[DIR], g.l3y[DIR]};
+    const double l3 = g.l3b[DIR];
     const T dxd = from_f64<T>(g.dx[DIR]);
     const bool shk = f.shock && f.shock[cc];
 #pragma unroll
@@ -290,7 +290,7 @@ __device__ __forceinline__ void d_sweep_cell(const Geo& g, const Fields& f, cons
     vL[dd::BXn] = bn;
     vl[dd::BXn] = bn;
     RiemannOut<D, T> r;
-    riemann<D, DIR, SOLVER>(from_f64<T>(g.gamma), from_f64<T>(g.rgm1), vL, vl, r);
+    riemann<D, DIR, SOLVER>(from_f64<T>(g.gamma), vL, vl, r);
     store_emf<D, DIR>(g, f, cc, r, vL, vl);
     if (active_col) {
       const Scale<T> area = scale_by(from_f64<T>(g.A[DIR]));

@@ -151,7 +151,7 @@ __global__ void __launch_bounds__(32 * kTW) k_sweep_tile(Geo g, Fields f, const 
   const double* vs = f.Vs + DIR * g.nface;
   const T gam = (T)g.gamma;
   const T dxd = (T)g.dx[DIR];
-  const Recip l3{g.l3b[DIR], g.l3y[DIR]};
+  const double l3 = g.l3b[DIR];
   const T dtdVT = (T)ctl->dtdV;
   const T areaT = (T)g.A[DIR];
   const T invdxT = T(1) / (T)g.dx[DIR];
@@ -202,7 +202,7 @@ __global__ void __launch_bounds__(32 * kTW) k_sweep_tile(Geo g, Fields f, const 
         vL[dd::BXn] = bn;
         vR[dd::BXn] = bn;
         RiemannOut<D, T> r;
-        riemann<D, DIR, SOLVER>(gam, (T)g.rgm1, vL, vR, r);
+        riemann<D, DIR, SOLVER>(gam, vL, vR, r);
         store_emf<D, DIR>(g, f, cc, r, vL, vR);
         if (active) {
           T FA[NU];

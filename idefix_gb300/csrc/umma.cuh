@@ -134,19 +134,6 @@ __device__ __forceinline__ bool mbar_wait_bounded(uint64_t* bar, uint32_t parity
 }
 constexpr long long kMmaSpin = 1ll << 22;
 
-// A run of MMAs over K (multiple of 16): D (M x N, TMEM) (+)= A (M x K) . B
-// (N x K)^T, both K-major no-swizzle tiles at a_base / b_base (shared
-// addresses) with K columns; issued by one thread
-__device__ __forceinline__ void mma_tile(uint32_t d_tmem, uint32_t a_base, uint32_t b_base, int K, uint32_t idesc,
-                                         bool accumulate) {
-  const uint32_t sbo = (uint32_t)K * 16u;
-  for (int k = 0; k < K; k += 16) {
-    const uint64_t ad = smem_desc(a_base + (uint32_t)k * 16u, 128u, sbo);
-    const uint64_t bd = smem_desc(b_base + (uint32_t)k * 16u, 128u, sbo);
-    mma_bf16(d_tmem, ad, bd, idesc, (accumulate || k > 0) ? 1u : 0u);
-  }
-}
-
 // an operand over a tile of C columns at shared address `base`: as it lies
 // (K-major, the MMA's K along the columns) or transposed (MN-major, K along
 // the rows)
