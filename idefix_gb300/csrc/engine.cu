@@ -111,13 +111,13 @@ __global__ void k_uc_field_all(Geo g, Fields f, int to_prim) {
 }
 
 // the cell-centred field of Uc from the faces over the active cells, as the
-// stage end forms it (mixed path, whose stage ends do not store it); ctl: only
-// where a stage end left this Uc (a run may have had nothing to do)
+// stage end forms it (mixed path, whose stage ends do not store it), where one
+// has left it out (a run may have had nothing to do)
 template <int D>
-__global__ void k_uc_field_active(Geo g, Fields f, const Ctl* ctl) {
+__global__ void k_uc_field_active(Geo g, Fields f, const double* faces, const Ctl* ctl) {
   using v = Var<D>;
   chain_wait();
-  if (ctl && !ctl->uc_fresh) return;
+  if (!ctl->uc_stale) return;
   const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
   const long long tot = (long long)g.n[0] * g.n[1] * (D == 3 ? g.n[2] : 1);
   if (tid >= tot) return;
@@ -127,7 +127,7 @@ __global__ void k_uc_field_active(Geo g, Fields f, const Ctl* ctl) {
   const int k = (D == 3) ? g.beg[2] + (int)(r / g.n[1]) : 0;
   const long long c = cidx(g, k, j, i), fc = fidx(g, k, j, i);
   for (int d = 0; d < D; d++) {
-    const double* vs = f.Vs + d * g.nface;
+    const double* vs = faces + d * g.nface;
     f.Uc[(v::BX1 + d) * g.ncell + c] = 0.5 * (vs[fc] + vs[fc + g.fs[d]]);
   }
 }
@@ -181,9 +181,10 @@ __global__ void k_ctl_get(const Ctl* ctl, Ctl* host) {
   chain_wait();
   *host = *ctl;
 }
-enum { kClrUcFresh = 1, kClrDone = 2, kClrNan = 4, kClrDivB = 8, kClrInvDt = 16 };
+enum { kClrUcFresh = 1, kClrDone = 2, kClrNan = 4, kClrDivB = 8, kClrInvDt = 16, kClrUcStale = 32 };
 __global__ void k_ctl_clear(Ctl* ctl, int what) {
   if (what & kClrUcFresh) ctl->uc_fresh = 0;
+  if (what & kClrUcStale) ctl->uc_stale = 0;
   if (what & kClrDone) ctl->done = 0;
   if (what & kClrNan) ctl->nan_count = 0ull;
   if (what & kClrDivB) ctl->divb_bits = 0ull;
@@ -1092,12 +1093,14 @@ int idfx_gpu_sizes(const idfx_gpu* h, int* nvar, int* nghost, long long* vc_len,
 }
 
 // the field part of Uc that the mixed path's stage ends left out, before
-// anything writes Uc or the faces it comes from.  A periodic block's arrays may be
-// uploaded without (its Uc is then rebuilt from the new faces); with walls Uc
-// stays the run's.
+// anything else writes Uc.  Its faces are the next cycle's Runge-Kutta begin copy,
+// which the last face update wrote and an upload leaves alone; without that copy
+// (one stage, NaN checks) the faces themselves, before an upload replaces them.
+static bool faces_copied(const Engine& e) { return e.nstages > 1 && e.check_nan_period <= 0; }
 static void complete_uc(Engine& e) {
   if (!e.uc_field_stale) return;
-  IDFX_CHAIN_D(k_uc_field_active, nblocks(n_active(e.g)), kThreads, e.g, e.f, e.g.nonper ? e.ctl : nullptr);
+  IDFX_CHAIN_D(k_uc_field_active, nblocks(n_active(e.g)), kThreads, e.g, e.f, faces_copied(e) ? e.f.Vs0 : e.f.Vs, e.ctl);
+  ctl_clear(e, kClrUcStale);
   e.uc_field_stale = false;
 }
 
@@ -1108,7 +1111,7 @@ static int copy_state(idfx_gpu* h, const double* Vc, const double* Vs, cudaMemcp
   const size_t bs = sizeof(double) * e.g.D * e.g.nface;
   const bool d2d = (kind == cudaMemcpyDeviceToDevice);  // by a kernel (k_copy_state)
   if (up) {
-    if (e.g.nonper) complete_uc(e);
+    if (!faces_copied(e)) complete_uc(e);
     if (d2d) {
       copy_device(e, e.f.Vc, Vc, e.f.Vs, Vs, e.ctl);
     } else {

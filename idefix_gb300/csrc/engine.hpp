@@ -33,7 +33,7 @@ struct Engine {
   int only_dir = -1;         // >= 0: sweeps launch that direction alone (autotuner)
   bool stage_outputs = false;  // mixed path: a stage end queued in this run wrote the next stage's inputs
   bool faces_saved = false;    // the last face update queued wrote the next cycle's Vs0
-  bool uc_field_stale = false; // mixed path: stage ends queued without the field part of Uc
+  bool uc_field_stale = false; // mixed path: stage ends queued without the field part of Uc (Ctl::uc_stale where one ran)
   std::string err;
   double* pool = nullptr;    // one allocation for every field
   size_t pool_len = 0;

@@ -62,6 +62,7 @@ struct Ctl {
   int status;  // Status
   int uc_fresh;  // 1: Uc (active cells) is the state the last stage end left
                  // and Vc was derived from it; 0 after any write from outside
+  int uc_stale;  // 1: the last stage end left out Uc's field part (kSeNoUcField)
 };
 
 // The EMF buffers (face EMFs ezi..eyk, upwind weights sv*, cell EMFs Ex*,
@@ -1840,7 +1841,10 @@ __device__ __forceinline__ void d_stage_end(const Geo& g, const Fields& f, const
   const int k = (D == 3) ? g.beg[2] + (int)(r / g.n[1]) : 0;
   const long long c = cidx(g, k, j, i);
   const long long fc = fidx(g, k, j, i);
-  if (tid == 0) ((Ctl*)ctl)->uc_fresh = 1;  // read by the next stage begin
+  if (tid == 0) {
+    ((Ctl*)ctl)->uc_fresh = 1;  // read by the next stage begin
+    if (out & kSeNoUcField) ((Ctl*)ctl)->uc_stale = 1;
+  }
   if (!combine) stage_end_cell<D, E, 0>(g, f, wc, w0, c, fc, out);
   else if (dbits(wc) == dbits(0.5) && dbits(w0) == dbits(0.5)) stage_end_cell<D, E, 1>(g, f, wc, w0, c, fc, out);
   else stage_end_cell<D, E, 2>(g, f, wc, w0, c, fc, out);
