@@ -141,7 +141,7 @@ __global__ void k_coarsen(const double* __restrict__ Vc, const double* __restric
 // Measured (32^3, both stages of a cycle): the three fused sweeps 434 / 469 /
 // 472 us; this launch 185 us (241 with whole tiles to a block and the range
 // looked up by column) and the three sweeps 91 / 93 / 95 us.  Two cycles with
-// their copies 3356 -> 1196 us, one cycle of 64^3 13978 -> 2792 us.
+// their copies 3356 -> 1085 us, one cycle of 64^3 13978 -> 2650 us.
 // ---------------------------------------------------------------------------
 constexpr int LT = 128;   // cells of a tile
 constexpr int LN = 512;   // threads

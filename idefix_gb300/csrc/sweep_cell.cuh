@@ -52,7 +52,10 @@ __host__ __device__ constexpr int cell_resident(size_t size) { return size == 8 
 //            1024^2 57 / 58 (78), 2048^2 204 / 159
 //   3-D x    32^3 10 / 11, 64^3 20 / 25, 128^3 105 / 113, 192^3 328 / 315
 //   3-D y,z  48^3 16, 17 / 15, 22 (17, 33), 64^3 24, 25 / 25, 29 (25, 63), 91 x 62 x 45
-//            PPM 40, 42 / 48, 53, 96^3 65, 67 / 42, 53
+//            PPM 40, 42 / 48, 53, 96^3 65, 67 / 42, 53; against the segment
+//            chosen untimed 80^3 37, 39 / 34, 67, 96^3 60, 60 / 42, 68, 128^3 132,
+//            136 / 96, 117, 160^3 249, 260 / 169, 168 (an untuned z sweep between
+//            74^3 and 96^3 would be faster in this form)
 // (across x a tile's overlap is 2 of its 16 positions.)  Ensembles the same by
 // the cells of all boxes: 20 boxes of 64^2 .. 384^2, 3 cycles 2423 -> 1911 us.
 inline bool cell_sweep_wins(int D, int dir, long long cells) {
